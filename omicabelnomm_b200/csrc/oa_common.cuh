@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "omicabel_b200.h"
 
@@ -111,6 +112,62 @@ __device__ __forceinline__ float warp_sumf(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// Power-of-two scale of a column for its FP16 hi / lo split, from (an upper
+// bound of) its sum of squares: sqrt(ss) * scale lies in [2^13, 2^14), so no
+// element overflows FP16 (65504), and elements down to 2^-16 of that (the
+// root mean square of 2^30 rows) keep hi + lo to 2^-22 of themselves; smaller
+// ones to 2^-25 absolute.  *inv = 1 / scale.
+__device__ __forceinline__ float half_scale(double ss, float* inv) {
+    int e = 14;                                      // scale 1 where the sum is not usable
+    const int hx = __double2hiint(ss);
+    if (hx >= 0 && hx < 0x7ff00000) {
+        const int ex = (hx >> 20) - 1022;            // ss < 2^ex
+        e = ex < -200 ? -100 : (ex > 280 ? 140 : (ex + 1) >> 1);   // sqrt(ss) < 2^e
+    }
+    *inv = __int_as_float((127 + e - 14) << 23);
+    return __int_as_float((127 + 14 - e) << 23);
+}
+// Scale of the orthonormal covariate basis' columns (their sums of squares are at most 1).
+constexpr float HALF_SCALE_Q = 16384.f;
+
+// x * scale = hi + lo in FP16
+__device__ __forceinline__ void split_half(float xs, __half& hi, __half& lo) {
+    hi = __float2half_rn(xs);
+    lo = __float2half_rn(xs - __half2float(hi));
+}
+
+// BF16 hi/lo of 8 floats (x = hi + lo to ~2^-17 relative), packed
+__device__ __forceinline__ void split8(const float4 p0, const float4 p1, uint4& hi, uint4& lo) {
+    const float e[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    uint32_t h[4], o[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const __nv_bfloat162 hb = __floats2bfloat162_rn(e[2 * u], e[2 * u + 1]);
+        const float2 hf = __bfloat1622float2(hb);
+        const __nv_bfloat162 lb = __floats2bfloat162_rn(e[2 * u] - hf.x, e[2 * u + 1] - hf.y);
+        h[u] = *reinterpret_cast<const uint32_t*>(&hb);
+        o[u] = *reinterpret_cast<const uint32_t*>(&lb);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// FP16 hi/lo of 8 floats times sc (a power of two), packed
+__device__ __forceinline__ void split8h(const float4 p0, const float4 p1, float sc, uint4& hi, uint4& lo) {
+    const float e[8] = {p0.x * sc, p0.y * sc, p0.z * sc, p0.w * sc, p1.x * sc, p1.y * sc, p1.z * sc, p1.w * sc};
+    uint32_t h[4], o[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const __half2 hb = __floats2half2_rn(e[2 * u], e[2 * u + 1]);
+        const float2 hf = __half22float2(hb);
+        const __half2 lb = __floats2half2_rn(e[2 * u] - hf.x, e[2 * u + 1] - hf.y);
+        h[u] = *reinterpret_cast<const uint32_t*>(&hb);
+        o[u] = *reinterpret_cast<const uint32_t*>(&lb);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // In-place inverse of a small SPD matrix (row-major k x k, k <= OA_MAX_R or

@@ -302,7 +302,11 @@ struct oa_engine {
     // traits
     int t = 0;
     DBuf<float> Yraw, Yt;
+    // 16-bit hi / lo of the GEMMs' column operand, n_pad values per column: the traits' residuals Y~
+    // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  BF16 in the mixed form; FP16
+    // of scaled columns in the plain form, with cscale = 1 / scale of each column
     DBuf<__nv_bfloat16> Yhi, Ylo;
+    DBuf<float> cscale;
     DBuf<double> tsums, rss0, b0, W, zQ;
     DBuf<int> tcounts, pat, zset, nobs, set_off, set_rows, set_rep, set_kind, set_slot, tperm, tinv;
     DBuf<float> a_r2, inv_ncorr, vf;
@@ -332,9 +336,10 @@ struct oa_engine {
         size_t smem = 0;
     } lp;
     long long tune_gen = 0;
-    DBuf<float> B2;
-    DBuf<__nv_bfloat16> B2hi, B2lo;
     std::vector<int> h_nobs;
+    // the chunk's GEMM stores z = X'Y~ (and the pre-GEMM's columns beside it, from one read of X) and
+    // k_test_stats evaluates it: the plain form, and narrow mixed blocks (combined_columns)
+    bool stored_z = false;
     // SNP chunk buffers
     int chunk = 0;
     DBuf<float> Xstage[2];
@@ -349,8 +354,8 @@ struct oa_engine {
     int n_inter = 0, inter_keep = 0;
     DBuf<__nv_bfloat16> Xhi, Xlo;
     DBuf<float> mean, varx, aobs, afull, zA, zD;
-    DBuf<float> D, Dset, C2T;   // pre-GEMM path: X'X, per-set X'X, pre-GEMM output
-    DBuf<float> C2part;         // plain pre-GEMM: partial product of the second K half
+    DBuf<float> D, Dset, C2T;   // X'X, per-set X'X; stored products (pre-GEMM columns and / or z)
+    DBuf<float> xscale;         // plain form: 1 / scale of each SNP column's FP16 split
     DBuf<int> has_nan;
     DBuf<double> sinv, sfinv;
     DBuf<float> qdel;           // quirk mode: per (pattern, SNP) terms of the reference's r >= 2 downdate
@@ -428,15 +433,14 @@ int live_engines(int device, int delta) {
 template <class F>
 void for_each_buf(oa_engine* e, F&& f) {
     f(e->Q64); f(e->Rinv); f(e->Qr); f(e->Qb); f(e->qsum); f(e->Afull_lean);
-    f(e->Yraw); f(e->Yt); f(e->Yhi); f(e->Ylo);
+    f(e->Yraw); f(e->Yt); f(e->Yhi); f(e->Ylo); f(e->cscale);
     f(e->tsums); f(e->rss0); f(e->b0); f(e->W); f(e->zQ);
     f(e->tcounts); f(e->pat); f(e->zset); f(e->nobs); f(e->set_off); f(e->set_rows); f(e->set_rep);
     f(e->set_kind); f(e->set_slot); f(e->tperm); f(e->tinv);
     f(e->a_r2); f(e->inv_ncorr); f(e->vf); f(e->thash); f(e->tcheck); f(e->sst); f(e->qrows); f(e->pat_bad);
-    f(e->B2); f(e->B2hi); f(e->B2lo);
     f(e->Xstage[0]); f(e->Xstage[1]); f(e->Xmodel); f(e->inter); f(e->Xhi); f(e->Xlo);
     f(e->mean); f(e->varx); f(e->aobs); f(e->afull); f(e->zA); f(e->zD); f(e->D); f(e->Dset); f(e->C2T);
-    f(e->C2part);
+    f(e->xscale);
     f(e->has_nan); f(e->sinv); f(e->sfinv); f(e->sing); f(e->qdel); f(e->qK);
     f(e->rec); f(e->rec2); f(e->cov); f(e->cov2); f(e->counters); f(e->keys); f(e->keys2); f(e->perm);
     f(e->perm2); f(e->cub_tmp);
@@ -512,12 +516,10 @@ bool padded(const oa_engine* e) { return e->ru != e->r; }
 // A chunk passes through k_column_model (a dosage model, interactions or zero padding).
 bool column_pass(const oa_engine* e) { return e->in_cols > 0 || padded(e); }
 
-// Mixed form with the pre-GEMM statistics path: nothing after the column
-// statistics reads the FP32 chunk (the GEMMs read its BF16 split), so a row
-// subset is gathered by the statistics kernel as it stages the columns.
-bool lean_gathers(const oa_engine* e) {
-    return e->subset && e->use_pre && e->cfg.precision == OA_MIXED_BF16X3;
-}
+// With the pre-GEMM statistics path nothing after the column statistics reads
+// the FP32 chunk (the GEMMs read its split), so a row subset is gathered by
+// the statistics kernel as it stages the columns.
+bool lean_gathers(const oa_engine* e) { return e->subset && e->use_pre; }
 
 template <int R>
 oa_status chunk_input(oa_engine* e, const float* xr, int c0, int mbc, const float** X) {
@@ -619,6 +621,13 @@ oa_status exact_trait_sets(oa_engine* e, const float* Y, int t, const std::vecto
         }
     }
     return OA_OK;
+}
+
+// The per-SNP covariate sums of the current trait block come from the pre-GEMM (else from row gathers,
+// which handle neither the quirk, nor padding columns, nor 8 columns per SNP).
+bool use_pre_for(const oa_engine* e) {
+    return quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1 ||
+           (e->req.stats_path != 2 && e->c2 <= std::max(e->t, 256));
 }
 
 oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_ptr) {
@@ -766,10 +775,10 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     e->b2_ready = false;
     e->lp = oa_engine::LeanPlan{};
     OA_CHECK(e->Yt.ensure((size_t)t * e->n_pad));
-    if (e->cfg.precision == OA_MIXED_BF16X3) {
-        OA_CHECK(e->Yhi.ensure((size_t)t * e->n_pad));
-        OA_CHECK(e->Ylo.ensure((size_t)t * e->n_pad));
-    }
+    const size_t ycols = (size_t)t + (use_pre_for(e) ? e->c2 : 0);   // B2 follows Y~
+    OA_CHECK(e->Yhi.ensure(ycols * e->n_pad));
+    OA_CHECK(e->Ylo.ensure(ycols * e->n_pad));
+    OA_CHECK(e->cscale.ensure(ycols));
     OA_CHECK(e->rss0.ensure(t));
     OA_CHECK(e->sst.ensure(t));
     OA_CHECK(e->nobs.ensure(t));
@@ -779,9 +788,9 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->vf.ensure(t));
     const bool mixed = e->cfg.precision == OA_MIXED_BF16X3;
     k_trait_resid<<<t, OA_NTHREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
-                                               e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, e->Yt.p,
-                                               mixed ? e->Yhi.p : nullptr, mixed ? e->Ylo.p : nullptr, e->rss0.p,
-                                               e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p, e->inv_ncorr.p, e->vf.p);
+                                               e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, e->Yt.p, e->Yhi.p,
+                                               e->Ylo.p, e->rss0.p, e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p,
+                                               e->inv_ncorr.p, e->vf.p, mixed ? nullptr : e->cscale.p);
     ++e->launches;
     OA_CU(cudaGetLastError());
     OA_CU(cudaStreamSynchronize(e->st));
@@ -812,37 +821,58 @@ int wave_chunk(const oa_engine* e, int t) {
     return mt * 128 / r;
 }
 
+// A buffer of at least `want` elements that keeps its first `keep`.
+template <class T>
+oa_status grow_keep(oa_engine* e, DBuf<T>& b, size_t keep, size_t want) {
+    if (b.n >= want) return OA_OK;
+    DBuf<T> big;
+    OA_CHECK(big.ensure(want));
+    if (cudaMemcpyAsync(big.p, b.p, keep * sizeof(T), cudaMemcpyDeviceToDevice, e->st) != cudaSuccess) {
+        big.release();
+        OA_CU(cudaGetLastError());
+    }
+    b.release();
+    b = big;
+    return OA_OK;
+}
+
+// Mixed blocks whose traits and pre-GEMM columns fit one 256-column tile: both products come from one
+// launch that reads the split columns once (reading them is what bounds such a block).
+bool combined_columns(const oa_engine* e) {
+    return e->cfg.precision == OA_MIXED_BF16X3 && e->use_pre && !e->fuse_split && e->t + e->c2 <= 256;
+}
+
 oa_status prepare_tuning(oa_engine* e) {
-    const int t = e->t, l = e->l, n = e->n;
+    const int l = e->l, n = e->n;
     e->chunk = std::min(e->cfg.max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : wave_chunk(e, e->t));
     // default pipeline: CTA pairs with 64-wide K-blocks (the fastest at wide trait blocks; blocks of
     // at most 128 traits take the 1-SM narrow tiles whatever the variant)
     e->variant = (e->req.gemm_variant >= 1 && e->req.gemm_variant <= 4) ? e->req.gemm_variant : 4;
     e->raster = e->req.gemm_raster == 2 ? 2 : 1;
     e->lean_spb = e->req.lean_spb > 0 ? std::min(e->req.lean_spb, 8 / e->r) : 0;
-    // the row-gather form handles neither the quirk, nor padding columns, nor 8 columns per SNP
-    e->use_pre = quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1 ||
-                 (e->req.stats_path != 2 && e->c2 <= std::max(t, 256));
+    e->use_pre = use_pre_for(e);
     if (e->use_pre && !e->b2_ready) {
-        const size_t nb2 = (size_t)e->c2 * e->n_pad;
-        OA_CHECK(e->B2.ensure(nb2));
-        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, e->B2.p);
+        const size_t ny = (size_t)e->t * e->n_pad, nb2 = (size_t)e->c2 * e->n_pad;
+        const bool half = e->cfg.precision == OA_PLAIN_FP32;
+        OA_CHECK(grow_keep(e, e->Yhi, ny, ny + nb2));   // the tuning may have changed since the traits were set
+        OA_CHECK(grow_keep(e, e->Ylo, ny, ny + nb2));
+        OA_CHECK(grow_keep(e, e->cscale, e->t, (size_t)e->t + e->c2));
+        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, half,
+                                                                   e->Yhi.p + ny, e->Ylo.p + ny);
         ++e->launches;
         if (e->nsets > 0) {
-            k_b2_scatter<<<e->nsets, 256, 0, e->st>>>(e->Qr.p, e->LP, e->n_pad, l, e->set_off.p, e->set_rows.p,
-                                                      e->B2.p);
+            k_b2_scatter<<<e->nsets, 256, 0, e->st>>>(e->Qr.p, e->LP, e->n_pad, l, e->set_off.p, e->set_rows.p, half,
+                                                      e->Yhi.p + ny, e->Ylo.p + ny);
             ++e->launches;
         }
-        if (e->cfg.precision == OA_MIXED_BF16X3) {
-            OA_CHECK(e->B2hi.ensure(nb2));
-            OA_CHECK(e->B2lo.ensure(nb2));
-            k_split_bf16<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->B2.p, (long long)nb2, e->B2hi.p,
-                                                                          e->B2lo.p);
+        if (half) {
+            k_fill<<<(e->c2 + 255) / 256, 256, 0, e->st>>>(e->cscale.p + e->t, e->c2, 1.f / HALF_SCALE_Q);
             ++e->launches;
         }
         OA_CU(cudaGetLastError());
         e->b2_ready = true;
     }
+    e->stored_z = e->cfg.precision == OA_PLAIN_FP32 || combined_columns(e);
     if (e->use_pre) OA_CHECK(lean_plan(e));
     return OA_OK;
 }
@@ -878,7 +908,8 @@ StatsArgs stats_args(oa_engine* e, const float* X, int mbc, int LP, int spb, int
     A.sfinv = e->cfg.disp_cov ? e->sfinv.p : nullptr;
     A.zA = e->zA.p;
     A.zD = e->zD.p;
-    A.write_split = e->cfg.precision == OA_MIXED_BF16X3;
+    A.write_split = 1;
+    A.xscale = e->cfg.precision == OA_PLAIN_FP32 ? e->xscale.p : nullptr;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
@@ -1019,6 +1050,9 @@ bool fused_chunk(const oa_engine* e, const float* X, size_t ldx, const int* xrow
 }
 
 template <int R>
+oa_status schur(oa_engine* e, const float* C2, int mbc);
+
+template <int R>
 oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, int mbc, bool fused) {
     const int spb = e->lp.spb;
     const size_t smem = e->lp.smem;
@@ -1041,8 +1075,8 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     A.has_nan = e->has_nan.p;
     A.D = e->D.p;
     A.Dset = e->Dset.p;
-    const bool mixed = e->cfg.precision == OA_MIXED_BF16X3;
-    A.write_split = mixed && !fused ? 1 : 0;
+    A.write_split = fused ? 0 : 1;
+    A.xscale = e->cfg.precision == OA_PLAIN_FP32 ? e->xscale.p : nullptr;
     A.use_xi = e->lp.xi ? 1 : 0;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
@@ -1062,25 +1096,30 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     const int grid = std::min(groups, e->sm_count * per_sm);
     OA_CU(oa_launch_snp_lean(R, spb, A, grid, threads, smem, e->st));
     ++e->launches;
+    if (e->stored_z) return OA_OK;   // the pre-GEMM's columns come with the main product
     const int ldc = e->chunk * R;
+    const size_t ny = (size_t)e->t * e->n_pad;   // B2 follows Y~
+    int* err = reinterpret_cast<int*>(e->counters.p + 3);
     if (fused)
-        OA_CU(oa_launch_pre_tcf(X, ldx, e->n, mbc * R, e->mean.p, e->has_nan.p, e->center ? 1 : 0, e->B2hi.p,
-                                e->B2lo.p, e->c2,
-                                e->n_pad, e->C2T.p, ldc, reinterpret_cast<int*>(e->counters.p + 3), e->st));
-    else if (mixed)
-        OA_CU(oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, e->B2hi.p, e->B2lo.p, e->c2, e->n_pad, e->C2T.p, ldc,
-                               reinterpret_cast<int*>(e->counters.p + 3), e->st));
+        OA_CU(oa_launch_pre_tcf(X, ldx, e->n, mbc * R, e->mean.p, e->has_nan.p, e->center ? 1 : 0, e->Yhi.p + ny,
+                                e->Ylo.p + ny, e->c2, e->n_pad, e->C2T.p, ldc, err, e->st));
     else
-        OA_CU(oa_launch_pre_simt(X, (size_t)e->n, mbc * R, e->B2.p, (size_t)e->n_pad, e->c2, e->n, e->mean.p,
-                                 e->has_nan.p, e->center ? 1 : 0, e->C2T.p, ldc, e->C2part.p, e->st));
+        OA_CU(oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, e->Yhi.p + ny, e->Ylo.p + ny, e->c2, e->n_pad, e->C2T.p,
+                               ldc, err, e->st));
     ++e->launches;
+    return schur<R>(e, e->C2T.p, mbc);
+}
+
+// Schur complements of the chunk's (SNP, pattern) systems from the pre-GEMM columns C2.
+template <int R>
+oa_status schur(oa_engine* e, const float* C2, int mbc) {
     SchurArgs S{};
     S.l = e->l;
     S.mb = mbc;
     S.G = e->G;
     S.Z = e->Z;
-    S.ldc = ldc;
-    S.C2 = e->C2T.p;
+    S.ldc = e->chunk * R;
+    S.C2 = C2;
     S.D = e->D.p;
     S.Dset = e->Dset.p;
     S.W = e->W.p;
@@ -1097,7 +1136,7 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     S.rr = e->ru;
     S.qdel = quirk_on(e) ? e->qdel.p : nullptr;
     S.qK = quirk_on(e) ? e->qK.p : nullptr;
-    S.Afull_lean = qx ? e->Afull_lean.p : nullptr;
+    S.Afull_lean = want_lean_qx(e) && oa_lean_has_qx(R, e->lp.spb) ? e->Afull_lean.p : nullptr;
     OA_CU(oa_launch_schur(R, S, e->st));
     ++e->launches;
     return OA_OK;
@@ -1187,21 +1226,60 @@ CovArgs cov_args(oa_engine* e, int mbc) {
     return C;
 }
 
+constexpr int Z_TRAITS = 8192;   // traits per stored product
+
+// Name of the kernel that forms the stored product.
+const char* stored_name(const oa_engine* e) {
+    if (e->cfg.precision != OA_PLAIN_FP32) return "k_gemm_tc";
+    return std::min(e->t, Z_TRAITS) + (e->use_pre && e->t <= Z_TRAITS ? e->c2 : 0) > 128 ? "k_gemm_tcp2"
+                                                                                          : "k_gemm_tcp";
+}
+
 template <int R>
 oa_status gemm_dispatch(oa_engine* e, const float* X, int mbc, int snp_base, bool fused) {
     EpiArgs E = epi_args(e, mbc, snp_base);
+    if (e->stored_z) {
+        const bool plain = e->cfg.precision == OA_PLAIN_FP32;
+        const int ldc = e->chunk * R, c2 = e->use_pre ? e->c2 : 0;
+        int* err = reinterpret_cast<int*>(e->counters.p + 3);
+        auto product = [&](int col0, int cols) -> oa_status {   // columns [col0, col0 + cols) of [Y~ | B2] to C2T
+            const __nv_bfloat16 *bh = e->Yhi.p + (size_t)col0 * e->n_pad, *bl = e->Ylo.p + (size_t)col0 * e->n_pad;
+            OA_CU(plain ? oa_launch_gemm_tcp(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->xscale.p,
+                                             e->cscale.p + col0, e->C2T.p, ldc, err, e->st)
+                        : oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->C2T.p, ldc, err,
+                                           e->st));
+            ++e->launches;
+            return OA_OK;
+        };
+        auto tests = [&](int j0, int nt) -> oa_status {
+            OA_CU(oa_launch_test_stats(R, E, e->C2T.p, ldc, j0, nt, e->st));
+            ++e->launches;
+            return OA_OK;
+        };
+        if (e->t <= Z_TRAITS) {
+            OA_CHECK(product(0, e->t + c2));
+            if (c2) OA_CHECK(schur<R>(e, e->C2T.p + (size_t)e->t * ldc, mbc));
+            OA_CHECK(tests(0, e->t));
+        } else {   // wide trait blocks: z in segments, so that it stays within a few hundred MB
+            if (c2) {
+                OA_CHECK(product(e->t, c2));
+                OA_CHECK(schur<R>(e, e->C2T.p, mbc));
+            }
+            for (int j0 = 0; j0 < e->t; j0 += Z_TRAITS) {
+                const int nt = std::min(Z_TRAITS, e->t - j0);
+                OA_CHECK(product(j0, nt));
+                OA_CHECK(tests(j0, nt));
+            }
+        }
+        e->last_name = stored_name(e);
+        return OA_OK;
+    }
     if (fused) {
         OA_CU(oa_launch_gemm_tcf(R, e->raster, X, (size_t)e->n, e->n, mbc * R, e->mean.p, e->has_nan.p,
                                  e->center ? 1 : 0,
                                  e->Yhi.p, e->Ylo.p, e->t, e->n_pad, E, reinterpret_cast<int*>(e->counters.p + 3),
                                  e->st));
         e->last_name = e->t > 128 ? "k_gemm_tc2f" : "k_gemm_tcf";
-    } else if (e->cfg.precision == OA_PLAIN_FP32) {
-        // X'y~ does not change when a column is shifted (y~ is orthogonal to the intercept on the
-        // observed rows): the main GEMM reads the dosages as they are, imputing NaN only
-        OA_CU(oa_launch_gemm_simt(R, X, (size_t)e->n, mbc * R, e->Yt.p, (size_t)e->n_pad, e->t, e->n, e->mean.p,
-                                  e->has_nan.p, 0, E, e->st));
-        e->last_name = "k_gemm_simt";
     } else {
         OA_CU(oa_launch_gemm_tc(R, e->variant, e->raster, e->Xhi.p, e->Xlo.p, mbc * R, e->Yhi.p, e->Ylo.p, e->t,
                                 e->n_pad, E, reinterpret_cast<int*>(e->counters.p + 3), e->st));
@@ -1231,16 +1309,15 @@ oa_status ensure_chunk_buffers(oa_engine* e) {
         OA_CHECK(e->afull.ensure(mb * l * r));
         OA_CHECK(e->sfinv.ensure(mb * r * r));
     }
-    if (e->cfg.precision == OA_MIXED_BF16X3) {
-        OA_CHECK(e->Xhi.ensure(mb * r * e->n_pad));
-        OA_CHECK(e->Xlo.ensure(mb * r * e->n_pad));
-    }
+    OA_CHECK(e->Xhi.ensure(mb * r * e->n_pad));
+    OA_CHECK(e->Xlo.ensure(mb * r * e->n_pad));
+    if (e->cfg.precision == OA_PLAIN_FP32) OA_CHECK(e->xscale.ensure(mb * r));
     if (e->use_pre) {
         OA_CHECK(e->D.ensure(mb * r * r));
         OA_CHECK(e->Dset.ensure((size_t)std::max(e->nsets, 1) * mb * r * r));
-        OA_CHECK(e->C2T.ensure((size_t)e->c2 * mb * r));
-        if (e->cfg.precision == OA_PLAIN_FP32) OA_CHECK(e->C2part.ensure((size_t)e->c2 * mb * r));
     }
+    const size_t zcols = e->stored_z ? std::min(e->t, Z_TRAITS) : 0;
+    OA_CHECK(e->C2T.ensure((zcols + (e->use_pre ? e->c2 : 0)) * mb * r));
     return OA_OK;
 }
 
@@ -1436,7 +1513,7 @@ oa_status run_block(oa_engine* e, const float* xr, int mb, bool host_input) {
         float bms = 0.f;
         e->block_ms = cudaEventElapsedTime(&bms, e->k0, e->k1) == cudaSuccess ? bms : 0.f;
         cudaGetLastError();
-        e->last_name = e->cfg.precision == OA_PLAIN_FP32                ? "k_gemm_simt"
+        e->last_name = e->stored_z                                      ? stored_name(e)
                        : e->fused_last                                  ? (e->t > 128 ? "k_gemm_tc2f" : "k_gemm_tcf")
                        : (e->t > 128 && e->variant >= 3) ? "k_gemm_tc2"
                                                           : "k_gemm_tc";
@@ -1451,12 +1528,17 @@ oa_status run_block(oa_engine* e, const float* xr, int mb, bool host_input) {
 // threshold, with headroom; every test with store_all) + the unused tails
 // of the epilogue warps' reserved blocks (at most one block per warp and
 // launch).  A block that still overflows grows the buffer and runs again.
+// Slots left unused by one chunk's launches: at most one reserved block per epilogue warp.
+long long block_tails(const oa_engine* e, long long t) {
+    return (t + Z_TRAITS - 1) / Z_TRAITS * (long long)e->sm_count * EPI_WARPS_TC * EMIT_BLOCK;
+}
+
 long long slots_needed(const oa_engine* e, long long mb, long long t, long long chunk) {
     const long long tests = mb * t;
     const double tail = std::erfc((double)e->cfg.min_t_store / std::sqrt(2.0));
     const double share = std::min(1.0, 1.5 * tail + 1e-3);
     const long long nch = (mb + chunk - 1) / chunk;
-    const long long slack = nch * (long long)e->sm_count * EPI_WARPS_TC * EMIT_BLOCK;
+    const long long slack = nch * block_tails(e, t);
     const long long rows = e->cfg.store_all ? tests : (long long)(tests * share);
     return std::max<long long>(1 << 16, rows + slack);
 }
@@ -2256,10 +2338,8 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         OA_CHECK(e->thash.ensure(t * 4));
         for (auto* b : {&e->pat, &e->zset, &e->tperm, &e->tinv}) OA_CHECK(b->ensure(t));
         OA_CHECK(e->Yt.ensure(t * e->n_pad));
-        if (e->cfg.precision == OA_MIXED_BF16X3) {
-            OA_CHECK(e->Yhi.ensure(t * e->n_pad));
-            OA_CHECK(e->Ylo.ensure(t * e->n_pad));
-        }
+        OA_CHECK(e->Yhi.ensure(t * e->n_pad));
+        OA_CHECK(e->Ylo.ensure(t * e->n_pad));
         OA_CHECK(e->rss0.ensure(t));
         for (auto* b : {&e->sst, &e->a_r2, &e->inv_ncorr, &e->vf}) OA_CHECK(b->ensure(t));
         OA_CHECK(e->nobs.ensure(t));
@@ -2278,7 +2358,7 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         OA_CHECK(ensure_cap(e, slots));
         const size_t cap = (size_t)e->cap;   // slots, with the headroom ensure_cap adds
         // rows written: all slots but the block tails
-        const long long tails = ((snps + chunk - 1) / chunk) * (long long)e->sm_count * EPI_WARPS_TC * EMIT_BLOCK;
+        const long long tails = ((snps + chunk - 1) / chunk) * block_tails(e, traits);
         const size_t R = (size_t)std::max<long long>(1, slots - tails);
         OA_CHECK(e->keys.ensure(cap));
         OA_CHECK(e->keys2.ensure(cap));

@@ -358,9 +358,11 @@ __device__ __forceinline__ void epi_retire(const EpiArgs& E, Emitter& em) {
 }
 
 // Block-reserved row emission for records built only by the lanes that
-// store: `write` receives the slot of the calling lane's row.
+// store: `write` receives the slot of the calling lane's row.  `block` slots
+// (at least 32) are reserved at a time.
 template <int R, class W>
-__device__ __forceinline__ void epi_emit_lazy(const EpiArgs& E, bool st, Emitter& em, W&& write) {
+__device__ __forceinline__ void epi_emit_lazy(const EpiArgs& E, bool st, Emitter& em, W&& write,
+                                              int block = EMIT_BLOCK) {
     if (!E.rec) return;
     const unsigned m = __ballot_sync(0xffffffffu, st);
     if (!m) return;
@@ -369,10 +371,10 @@ __device__ __forceinline__ void epi_emit_lazy(const EpiArgs& E, bool st, Emitter
     if (em.used + k > em.cap) {   // warp-uniform
         epi_retire<R>(E, em);
         unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(E.rec_count, (unsigned long long)EMIT_BLOCK);
+        if (lane == 0) b = atomicAdd(E.rec_count, (unsigned long long)block);
         em.base = __shfl_sync(0xffffffffu, b, 0);
         em.used = 0;
-        em.cap = EMIT_BLOCK;
+        em.cap = block;
     }
     if (st) {
         const unsigned long long idx = em.base + (unsigned long long)(em.used + __popc(m & ((1u << lane) - 1u)));

@@ -31,6 +31,7 @@
 
 #include "oa_epilogue.cuh"
 #include "oa_launch.h"
+#include "oa_test_stats.cuh"
 
 namespace oa {
 namespace tc {
@@ -1503,6 +1504,8 @@ k_gemm_tc2f(const __grid_constant__ CUtensorMap mAf, const __grid_constant__ CUt
     if (threadIdx.x == 0 && abort_sh) atomicExch(err, 1);
 }
 
+#include "oa_gemm_tcp.cuh"
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1600,6 +1603,64 @@ static cudaError_t go2(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int x
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_gemm_tc2<R, SH>, a_hi, a_lo, b_hi, b_lo, xrows, t, n_pad / SH::BK, E, raster,
                               err);
+}
+
+// Launch of the promoted kernels (oa_gemm_tcp.cuh).
+template <class SH>
+static cudaError_t go_p(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows, const __nv_bfloat16* Bhi,
+                        const __nv_bfloat16* Blo, int t, int n_pad, const float* rscale, const float* cscale,
+                        float* cout, int ldc, int* err, cudaStream_t st) {
+    CUtensorMap a_hi, a_lo, b_hi, b_lo;
+    if (!make_map(&a_hi, Xhi, xrows, n_pad, BM, SH::BK) || !make_map(&a_lo, Xlo, xrows, n_pad, BM, SH::BK) ||
+        !make_map(&b_hi, Bhi, t, n_pad, SH::BN, SH::BK) || !make_map(&b_lo, Blo, t, n_pad, SH::BN, SH::BK))
+        return cudaErrorInvalidValue;
+    static int attr_done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_done[dev & 63]) {   // once per device, never during a stream capture
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tcp<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)SH::SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        attr_done[dev & 63] = 1;
+    }
+    const int ntiles = ((xrows + BM - 1) / BM) * ((t + SH::BN - 1) / SH::BN);
+    k_gemm_tcp<SH><<<std::min(ntiles, sm_count()), NUM_THREADS, SH::SMEM_BYTES, st>>>(
+        a_hi, a_lo, b_hi, b_lo, xrows, t, n_pad / SH::BK, rscale, cscale, cout, ldc, err);
+    return cudaGetLastError();
+}
+
+template <class SH>
+static cudaError_t go_p2(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows, const __nv_bfloat16* Bhi,
+                         const __nv_bfloat16* Blo, int t, int n_pad, const float* rscale, const float* cscale,
+                         float* cout, int ldc, int* err, cudaStream_t st) {
+    CUtensorMap a_hi, a_lo, b_hi, b_lo;
+    if (!make_map(&a_hi, Xhi, xrows, n_pad, BM, SH::BK) || !make_map(&a_lo, Xlo, xrows, n_pad, BM, SH::BK) ||
+        !make_map(&b_hi, Bhi, t, n_pad, SH::BN / 2, SH::BK) || !make_map(&b_lo, Blo, t, n_pad, SH::BN / 2, SH::BK))
+        return cudaErrorInvalidValue;
+    static int attr_done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_done[dev & 63]) {   // once per device, never during a stream capture
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_tcp2<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)SH::SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        attr_done[dev & 63] = 1;
+    }
+    const int ntiles = ((xrows + 2 * BM - 1) / (2 * BM)) * ((t + SH::BN - 1) / SH::BN);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * std::min(ntiles, sm_count() / 2), 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SH::SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_gemm_tcp2<SH>, a_hi, a_lo, b_hi, b_lo, xrows, t, n_pad / SH::BK, rscale,
+                              cscale, cout, ldc, err);
 }
 
 // Pipeline variant: 1 = BK 32 x 4 stages, 2 = BK 64 x 2 stages, 3 = CTA pairs (2-SM MMA), BK 32 x 6 stages,
@@ -1752,6 +1813,38 @@ cudaError_t oa_launch_pre_tc(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo,
     return tc::go<1, tc::Shape<64, 2, 256>, true>(Xhi, Xlo, xrows, Bhi, Blo, c2, n_pad, none, C, ldc, 1, err, st);
 }
 
+
+cudaError_t oa_launch_gemm_tcp(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows,
+                               const __nv_bfloat16* Bhi, const __nv_bfloat16* Blo, int cols, int n_pad,
+                               const float* rscale, const float* cscale, float* C, int ldc, int* err,
+                               cudaStream_t st) {
+    if (cols <= 64)
+        return tc::go_p<tc::ShapeP<4, 64, false>>(Xhi, Xlo, xrows, Bhi, Blo, cols, n_pad, rscale, cscale, C, ldc, err,
+                                                  st);
+    if (cols <= 128)
+        return tc::go_p<tc::ShapeP<3, 128, false>>(Xhi, Xlo, xrows, Bhi, Blo, cols, n_pad, rscale, cscale, C, ldc,
+                                                   err, st);
+    return tc::go_p2<tc::ShapeP<3, 256, true>>(Xhi, Xlo, xrows, Bhi, Blo, cols, n_pad, rscale, cscale, C, ldc, err,
+                                               st);
+}
+
+template <int R>
+static cudaError_t go_ts(const EpiArgs& E, const float* z, int ldz, int j0, int nt, cudaStream_t st) {
+    const long long items = (long long)((E.mb + TS_THREADS - 1) / TS_THREADS) * ((nt + TS_TRAITS - 1) / TS_TRAITS);
+    const int grid = (int)std::min<long long>(items, (long long)TS_CTAS_PER_SM * tc::sm_count());
+    k_test_stats<R><<<grid, TS_THREADS, 0, st>>>(E, z, ldz, j0, nt);
+    return cudaGetLastError();
+}
+
+cudaError_t oa_launch_test_stats(int R, const EpiArgs& E, const float* z, int ldz, int j0, int nt, cudaStream_t st) {
+    switch (R) {
+        case 1: return go_ts<1>(E, z, ldz, j0, nt, st);
+        case 2: return go_ts<2>(E, z, ldz, j0, nt, st);
+        case 4: return go_ts<4>(E, z, ldz, j0, nt, st);
+        case 8: return go_ts<8>(E, z, ldz, j0, nt, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
 
 bool oa_gemm_tc_fusable(int variant, int t) { return t <= 128 || variant >= 3; }
 

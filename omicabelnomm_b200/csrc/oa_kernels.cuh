@@ -223,6 +223,8 @@ k_set_gram(const double* __restrict__ Q64, int n, int l, const int* __restrict__
 // kept sorted by missingness pattern inside the engine).  Writes Y~ (FP32,
 // and BF16 hi/lo for the tensor-core form), RSS0, SST and the constants the
 // epilogue folds: a_r2 = (n-1)/((n_corr-1) SST), 1/n_corr, (n-miss)/n.
+// With yscale (the FP32-accurate tensor-core form) the split is FP16 of the
+// scaled residuals, written once RSS0 is known, and yscale[jj] = 1 / scale.
 static __global__ void __launch_bounds__(OA_NTHREADS)
 k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, int p,
               const double* __restrict__ Q64, const double* __restrict__ sums,
@@ -231,7 +233,8 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
               __nv_bfloat16* __restrict__ Yhi, __nv_bfloat16* __restrict__ Ylo,
               double* __restrict__ rss0, float* __restrict__ sst, int* __restrict__ nobs,
               double* __restrict__ b0out, float* __restrict__ a_r2, float* __restrict__ inv_ncorr,
-              float* __restrict__ vf) {
+              float* __restrict__ vf, float* __restrict__ yscale = nullptr) {
+    __shared__ float half_s;
     __shared__ double b0[OA_MAX_L];
     __shared__ double red[8];
     const int jj = blockIdx.x;
@@ -261,7 +264,7 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
             }
         }
         out[k] = e;
-        if (Yhi) {
+        if (Yhi && !yscale) {
             const __nv_bfloat16 hi = __float2bfloat16_rn(e);
             Yhi[(size_t)jj * n_pad + k] = hi;
             Ylo[(size_t)jj * n_pad + k] = __float2bfloat16_rn(e - __bfloat162float(hi));
@@ -283,6 +286,18 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
         a_r2[jj] = (float)((double)(n - 1) / ((double)(ncorr - 1) * (double)sstf));
         inv_ncorr[jj] = (float)(1.0 / (double)ncorr);
         vf[jj] = (float)((double)no / (double)n);
+        if (yscale) {
+            float inv;
+            half_s = half_scale(s, &inv);
+            yscale[jj] = inv;
+        }
+    }
+    if (yscale) {
+        __syncthreads();
+        const float sc = half_s;
+        __half* yh = reinterpret_cast<__half*>(Yhi) + (size_t)jj * n_pad;
+        __half* yl = reinterpret_cast<__half*>(Ylo) + (size_t)jj * n_pad;
+        for (int k = threadIdx.x; k < n_pad; k += blockDim.x) split_half(out[k] * sc, yh[k], yl[k]);   // own writes
     }
 }
 

@@ -16,18 +16,20 @@ cudaError_t oa_launch_snp_lean(int R, int spb, const LeanArgs& A, int grid, int 
 int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads);
 bool oa_lean_has_qx(int R, int spb);
 cudaError_t oa_launch_schur(int R, const SchurArgs& S, cudaStream_t st);
-// pre-GEMM C[col * ldc + row] = sum_k X[row][k] B[col][k], col < c2 (tensor-core and SIMT forms)
+// pre-GEMM C[col * ldc + row] = sum_k X[row][k] B[col][k], col < c2 (BF16 hi / lo operands)
 cudaError_t oa_launch_pre_tc(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows,
                              const __nv_bfloat16* Bhi, const __nv_bfloat16* Blo, int c2, int n_pad, float* C, int ldc,
                              int* err, cudaStream_t st);
-// cpart (c2 * ldc floats, or null): scratch for the second K half of a split product
-cudaError_t oa_launch_pre_simt(const float* X, size_t ldx, int xrows, const float* B, size_t ldb, int c2, int K,
-                               const float* colmean, const int* has_nan, int center, float* C, int ldc, float* cpart,
-                               cudaStream_t st);
-// center: dosages taken relative to colmean (NaN -> 0); else NaN -> colmean
+// FP32-accurate product C[col * ldc + row] = rscale[row] * cscale[col] * sum_k X[row][k] B[col][k], col < cols,
+// of FP16 hi / lo operands (held in 16-bit buffers): each K-block's tensor-core sum is added in FP32 registers
+cudaError_t oa_launch_gemm_tcp(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows,
+                               const __nv_bfloat16* Bhi, const __nv_bfloat16* Blo, int cols, int n_pad,
+                               const float* rscale, const float* cscale, float* C, int ldc, int* err, cudaStream_t st);
+// statistics of traits [j0, j0 + nt) from the stored product z (column 0 = trait j0)
+cudaError_t oa_launch_test_stats(int R, const EpiArgs& E, const float* z, int ldz, int j0, int nt, cudaStream_t st);
+// FP32 SIMT product with fused statistics, r = 1, 2 or 4 (zero-allocation entry point); NaN dosages -> colmean
 cudaError_t oa_launch_gemm_simt(int R, const float* X, size_t ldx, int xrows, const float* Yt, size_t ldy, int t,
-                                int K, const float* colmean, const int* has_nan, int center, const EpiArgs& E,
-                                cudaStream_t st);
+                                int K, const float* colmean, const int* has_nan, const EpiArgs& E, cudaStream_t st);
 // variant: 1 = BK 32 x 4 stages, 2 = BK 64 x 2 stages, 3 = CTA pairs (2-SM MMA) BK 32 x 6, 4 = pairs BK 64 x 3;
 // raster: 1 = trait tiles inner, 2 = SNP tiles inner
 // Bound (ns of %globaltimer) of the pipeline waits of the tensor-core GEMMs and of the staging waits of the

@@ -37,6 +37,7 @@ struct LeanArgs {
     __nv_bfloat16* Xhi;   // [mb*r][n_pad] (tensor-core form) or null
     __nv_bfloat16* Xlo;
     int write_split;
+    float* xscale;        // FP16 split of the columns times a power of two, 1 / scale here ([mb*r]); null: BF16 split
     int use_xi;           // with several columns per group: keep the row-interleaved copy for the set pass
     int center;           // take each column relative to its mean (valid when XL holds an intercept)
     int* err;
@@ -97,22 +98,6 @@ __device__ __forceinline__ void block_sum_fd(float (&v)[NV], double (&out)[NB], 
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NB; ++q) out[q] = bc[q];
-}
-
-// BF16 hi/lo of 8 floats (x = hi + lo to ~2^-17 relative), packed
-__device__ __forceinline__ void split8(const float4 p0, const float4 p1, uint4& hi, uint4& lo) {
-    const float e[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-    uint32_t h[4], o[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const __nv_bfloat162 hb = __floats2bfloat162_rn(e[2 * u], e[2 * u + 1]);
-        const float2 hf = __bfloat1622float2(hb);
-        const __nv_bfloat162 lb = __floats2bfloat162_rn(e[2 * u] - hf.x, e[2 * u + 1] - hf.y);
-        h[u] = *reinterpret_cast<const uint32_t*>(&hb);
-        o[u] = *reinterpret_cast<const uint32_t*>(&lb);
-    }
-    hi = make_uint4(h[0], h[1], h[2], h[3]);
-    lo = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // One CTA handles SPB SNPs (SPB*R columns) per group; a persistent loop over
@@ -261,6 +246,7 @@ k_snp_lean(LeanArgs A) {
         // NaN is counted and mean-imputed in place (src/Utility.cpp:302-326)
         // and the sweep is repeated - rare, dosage files seldom hold NaN
         float sh[NC];                          // subtracted from every value (centring), 0 without
+        float hs[NC];                          // scale of the FP16 split
         bool cnan[NC];
         {
             constexpr int NQX = QX ? NC * LEAN_QX_L : 0;
@@ -354,6 +340,20 @@ k_snp_lean(LeanArgs A) {
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c) sh[c] = A.center ? cmean[c] : 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) hs[c] = 1.f;
+            if (A.xscale) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    // sum of squares of the shifted column; the second term keeps it an upper bound
+                    // where the FP32 sums cancel (a column that is constant but for its last digits)
+                    const double raw = tot[NC + c * R + c % R], s0 = sh[c];
+                    const double d = raw - 2.0 * s0 * tot[c] + (double)n * s0 * s0;
+                    float inv = 1.f;
+                    hs[c] = half_scale(fmax(d, 0.0) + raw * 0x1p-18, &inv);
+                    if (threadIdx.x == 0 && c < ncol) A.xscale[i0 * R + c] = inv;
+                }
+            }
             if constexpr (QX) {
                 // A = Q'(x - shift) = Q'x - shift * (column sums of Q), in FP64; thread u writes entry u
                 // (compile-time register indices)
@@ -416,8 +416,12 @@ k_snp_lean(LeanArgs A) {
                     e[c][7] = p1.w - s0;
                     if (A.write_split && c < ncol) {
                         uint4 h, o;
-                        split8(make_float4(e[c][0], e[c][1], e[c][2], e[c][3]),
-                               make_float4(e[c][4], e[c][5], e[c][6], e[c][7]), h, o);
+                        const float4 lo4 = make_float4(e[c][0], e[c][1], e[c][2], e[c][3]);
+                        const float4 hi4 = make_float4(e[c][4], e[c][5], e[c][6], e[c][7]);
+                        if (A.xscale)
+                            split8h(lo4, hi4, hs[c], h, o);
+                        else
+                            split8(lo4, hi4, h, o);
                         reinterpret_cast<uint4*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k8] = h;
                         reinterpret_cast<uint4*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k8] = o;
                     }
@@ -522,36 +526,46 @@ k_snp_lean(LeanArgs A) {
 }
 
 // The pre-GEMM's column matrix B2 = [Q | Q o m_1 | ... | Q o m_S] (K-major:
-// column c of B2 is row c of the c2 x n_pad array), FP32 and, for the
-// tensor-core form, BF16 hi/lo.  Step 1 writes Q and zeros; step 2 scatters
-// Q's rows into the columns of every row set that contains them.
-static __global__ void k_b2_init(const float* __restrict__ Qr, int LP, int n, int n_pad, int l, int c2,
-                          float* __restrict__ B2) {
-    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q >= (long long)c2 * n_pad) return;
-    const int c = (int)(q / n_pad), k = (int)(q % n_pad);
-    B2[q] = (c < l && k < n) ? Qr[(size_t)k * LP + c] : 0.f;
-}
-
-static __global__ void k_b2_scatter(const float* __restrict__ Qr, int LP, int n_pad, int l, const int* __restrict__ set_off,
-                             const int* __restrict__ rows, float* __restrict__ B2) {
-    const int s = blockIdx.x;
-    const int r0 = set_off[s], r1 = set_off[s + 1];
-    float* dst = B2 + (size_t)(l + s * l) * n_pad;
-    for (int kk = r0 + threadIdx.x; kk < r1; kk += blockDim.x) {
-        const int k = rows[kk];
-        for (int a = 0; a < l; ++a) dst[(size_t)a * n_pad + k] = Qr[(size_t)k * LP + a];
+// column c of B2 is row c of the c2 x n_pad array), split into 16-bit hi / lo:
+// BF16, or FP16 of HALF_SCALE_Q times the value (`half`).  Step 1 writes Q and
+// zeros; step 2 scatters Q's rows into the columns of every row set that
+// contains them.
+__device__ __forceinline__ void b2_store(float v, int half, __nv_bfloat16* hi, __nv_bfloat16* lo) {
+    if (half) {
+        split_half(v * HALF_SCALE_Q, *reinterpret_cast<__half*>(hi), *reinterpret_cast<__half*>(lo));
+    } else {
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        *hi = h;
+        *lo = __float2bfloat16_rn(v - __bfloat162float(h));
     }
 }
 
-static __global__ void k_split_bf16(const float* __restrict__ src, long long count, __nv_bfloat16* __restrict__ hi,
-                             __nv_bfloat16* __restrict__ lo) {
+static __global__ void k_b2_init(const float* __restrict__ Qr, int LP, int n, int n_pad, int l, int c2, int half,
+                          __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (q >= count) return;
-    const float v = src[q];
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    hi[q] = h;
-    lo[q] = __float2bfloat16_rn(v - __bfloat162float(h));
+    if (q >= (long long)c2 * n_pad) return;
+    const int c = (int)(q / n_pad), k = (int)(q % n_pad);
+    b2_store((c < l && k < n) ? Qr[(size_t)k * LP + c] : 0.f, half, hi + q, lo + q);
+}
+
+static __global__ void k_b2_scatter(const float* __restrict__ Qr, int LP, int n_pad, int l, const int* __restrict__ set_off,
+                             const int* __restrict__ rows, int half, __nv_bfloat16* __restrict__ hi,
+                             __nv_bfloat16* __restrict__ lo) {
+    const int s = blockIdx.x;
+    const int r0 = set_off[s], r1 = set_off[s + 1];
+    const size_t base = (size_t)(l + s * l) * n_pad;
+    for (int kk = r0 + threadIdx.x; kk < r1; kk += blockDim.x) {
+        const int k = rows[kk];
+        for (int a = 0; a < l; ++a) {
+            const size_t q = base + (size_t)a * n_pad + k;
+            b2_store(Qr[(size_t)k * LP + a], half, hi + q, lo + q);
+        }
+    }
+}
+
+static __global__ void k_fill(float* __restrict__ p, int n, float v) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n) p[q] = v;
 }
 
 struct SchurArgs {

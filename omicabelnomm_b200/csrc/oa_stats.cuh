@@ -60,6 +60,7 @@ struct StatsArgs {
     __nv_bfloat16* Xhi;  // [mb*r][n_pad] or null (tensor-core form)
     __nv_bfloat16* Xlo;
     int write_split;
+    float* xscale;       // FP16 split of the columns times a power of two, 1 / scale here ([mb*r]); null: BF16 split
     int center;          // take each column relative to its mean (valid when XL holds an intercept)
     int nbuf;            // column buffers (2: the next group streams in during this one)
     int* err;            // set if a staging copy did not complete in time
@@ -237,32 +238,6 @@ k_snp_stats(StatsArgs A) {
             }
         }
         __syncthreads();
-        if (A.write_split) {
-            // BF16 hi/lo of each column, 8 elements (two 16-byte stores) per thread and step
-            const int np8 = A.n_pad / 8;
-            for (int c = 0; c < ncol; ++c) {
-                const float* col = xs + (size_t)c * nS;
-                const float s0 = cshift[c];
-                uint4* hi = reinterpret_cast<uint4*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad);
-                uint4* lo = reinterpret_cast<uint4*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad);
-                for (int k8 = threadIdx.x; k8 < np8; k8 += blockDim.x) {
-                    uint32_t h[4], o[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int k = k8 * 8 + 2 * u;
-                        const float v0 = k < n ? col[k] - s0 : 0.f, v1 = k + 1 < n ? col[k + 1] - s0 : 0.f;
-                        const __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
-                        const __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
-                        const __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
-                        h[u] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-                        o[u] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-                    }
-                    hi[k8] = make_uint4(h[0], h[1], h[2], h[3]);
-                    lo[k8] = make_uint4(o[0], o[1], o[2], o[3]);
-                }
-            }
-        }
-
         // 3. all-rows sums: D = X'X (R x R) and A = Q'X (LP x R, zero-padded Q) per SNP
         float acc[ACC];
 #pragma unroll
@@ -305,6 +280,36 @@ k_snp_stats(StatsArgs A) {
                 full[u] = s;
             }
             __syncthreads();
+        }
+
+        if (A.write_split) {
+            // BF16 or scaled FP16 hi/lo of each column, 8 elements (two 16-byte stores) per thread and step
+            const int np8 = A.n_pad / 8;
+            for (int c = 0; c < ncol; ++c) {
+                const float* col = xs + (size_t)c * nS;
+                const float s0 = cshift[c];
+                float sc = 1.f, inv = 1.f;
+                if (A.xscale) {
+                    const double d = full[(c / R) * NA + (c % R) * R + c % R];
+                    sc = half_scale(d, &inv);
+                    if (threadIdx.x == 0) A.xscale[i0 * R + c] = inv;
+                }
+                uint4* hi = reinterpret_cast<uint4*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad);
+                uint4* lo = reinterpret_cast<uint4*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad);
+                for (int k8 = threadIdx.x; k8 < np8; k8 += blockDim.x) {
+                    float e[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) e[u] = k8 * 8 + u < n ? col[k8 * 8 + u] - s0 : 0.f;
+                    const float4 p0 = make_float4(e[0], e[1], e[2], e[3]), p1 = make_float4(e[4], e[5], e[6], e[7]);
+                    uint4 h, o;
+                    if (A.xscale)
+                        split8h(p0, p1, sc, h, o);
+                    else
+                        split8(p0, p1, h, o);
+                    hi[k8] = h;
+                    lo[k8] = o;
+                }
+            }
         }
 
         // 4. all-rows Schur complement per SNP: var_x of the SNP terms (src/Algorithm.cpp:665-670)
