@@ -284,9 +284,8 @@ struct oa_engine {
     cudaStream_t st = nullptr, cp = nullptr;
     cudaEvent_t ev_copied[2]{}, ev_used[2]{}, k0 = nullptr, k1 = nullptr;
     long long launches = 0;
-    float last_ms = 0.f;
-    float stats_ms = 0.f;
-    float block_ms = 0.f;   // device time of the last SNP block on the engine's stream (events k0, k1)
+    int timed_chunks = 0;       // chunks of the last SNP block, whose events hold its kernel times
+    bool block_timed = false;   // the last SNP block ran (events k0, k1 bracket it on the engine's stream)
     cudaEvent_t s0 = nullptr, s1 = nullptr;
     const char* last_name = "";
     // covariates
@@ -1490,7 +1489,7 @@ oa_status run_block(oa_engine* e, const float* xr, int mb, bool host_input) {
         if (!launched) OA_CHECK(enqueue_block<R>(e, xr, mb, host_input, false));
         OA_CU(cudaEventRecord(e->k1, e->st));
         const unsigned long long* cnt = e->h_cnt;
-        OA_CU(cudaMemcpyAsync(e->h_cnt, e->counters.p, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->st));
+        OA_CU(cudaMemcpyAsync(e->h_cnt, e->counters.p, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->st));
         OA_CU(cudaStreamSynchronize(e->st));
         if (cnt[3]) {
             set_err("a device pipeline wait timed out (the kernel stopped cleanly)");
@@ -1501,18 +1500,8 @@ oa_status run_block(oa_engine* e, const float* xr, int mb, bool host_input) {
             drop_graph(e);
             continue;
         }
-        float total = 0.f, stotal = 0.f;
-        for (int c = 0; c < nch; ++c) {
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, e->cev0[c], e->cev1[c]) == cudaSuccess) total += ms;
-            if (cudaEventElapsedTime(&ms, e->sev0[c], e->sev1[c]) == cudaSuccess) stotal += ms;
-        }
-        cudaGetLastError();
-        e->last_ms = total;
-        e->stats_ms = stotal;
-        float bms = 0.f;
-        e->block_ms = cudaEventElapsedTime(&bms, e->k0, e->k1) == cudaSuccess ? bms : 0.f;
-        cudaGetLastError();
+        e->timed_chunks = nch;   // their events are read when a time is asked for (block_times)
+        e->block_timed = true;
         e->last_name = e->stored_z                                      ? stored_name(e)
                        : e->fused_last                                  ? (e->t > 128 ? "k_gemm_tc2f" : "k_gemm_tcf")
                        : (e->t > 128 && e->variant >= 3) ? "k_gemm_tc2"
@@ -1565,7 +1554,6 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
     OA_CHECK(ensure_chunk_buffers(e));
     const long long tests = (long long)mb * e->t;
     OA_CHECK(ensure_cap(e, slots_needed(e, mb, e->t, e->chunk)));
-    OA_CU(cudaMemsetAsync(e->counters.p, 0, 8 * sizeof(unsigned long long), e->st));
     if (e->dense_on || e->cfg.disp_cov) {
         const size_t nd = (size_t)e->t * mb;
         OA_CHECK(e->d_beta.ensure(nd * e->r));
@@ -1576,8 +1564,8 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         OA_CHECK(e->d_flags.ensure(nd));
         e->dense_ld = mb;
     }
-    e->last_ms = 0.f;
-    e->stats_ms = 0.f;
+    e->timed_chunks = 0;
+    e->block_timed = false;
     e->last_mb = mb;
     if (e->subset) {
         if (host_input) {
@@ -1600,9 +1588,7 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         OA_CHECK(run_block<R>(e, xr, mb, host_input));
     }
     OA_TRACE("stored rows: sort, copy back, convert");
-    unsigned long long cnt[5];
-    OA_CU(cudaMemcpyAsync(e->h_cnt, e->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, e->st));
-    OA_CU(cudaStreamSynchronize(e->st));
+    unsigned long long cnt[5];   // read back by run_block
     std::memcpy(cnt, e->h_cnt, sizeof cnt);
     std::memset(out, 0, sizeof *out);
     out->count = (int64_t)cnt[4];
@@ -1615,6 +1601,11 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
     // slots of the warps' reserved blocks sort last and are dropped
     const long long NS = (long long)cnt[0];   // slots handed out
     const long long N = (long long)cnt[4];    // rows written
+    // few rows: one copy of all fields (they are contiguous), converted by this thread; many: in pieces,
+    // each converted by all host threads while the next copies.  With the pieces' 7 copies each a block
+    // with 1,000 stored rows took 58 copies and 180 us of the stream
+    const bool few = N <= (1 << 18);
+    const int pieces = few ? 1 : RESULT_PIECES;
     const int l = e->l, p = e->p;
     // the packed fields of N rows (16 + 12 R bytes each) fit in N Rec-sized slots per rec_slots(R)
     OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, (size_t)N * rec_slots(R), e->retired_pinned));
@@ -1649,7 +1640,11 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         OA_CU(cudaGetLastError());
         // the rows come back in pieces, each converted on the host while the next is in flight
         const RowsSoA hsoa = rows_soa(e->h_rec, N, R);
-        for (int k = 0; k < RESULT_PIECES; ++k) {
+        if (few) {
+            OA_CU(cudaMemcpyAsync(e->h_rec, e->rec2.p, rows_soa_bytes(N, R), cudaMemcpyDeviceToHost, e->st));
+            OA_CU(cudaEventRecord(e->ev_piece[0], e->st));
+        }
+        for (int k = 0; k < RESULT_PIECES && !few; ++k) {
             const long long q0 = N * k / RESULT_PIECES, q1 = N * (k + 1) / RESULT_PIECES, nq = q1 - q0;
             if (nq > 0) {
                 auto d2h = [&](void* dst, const void* src, size_t bytes) {
@@ -1709,15 +1704,15 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
             e->o_mask[q] = m;
         }
     };
-    const int nthr = N > (1 << 18) ? (int)std::min<unsigned>(32u, std::max(1u, std::thread::hardware_concurrency())) : 1;
+    const int nthr = !few ? (int)std::min<unsigned>(32u, std::max(1u, std::thread::hardware_concurrency())) : 1;
     std::atomic<int> piece_err{0};
     auto convert_pieces = [&](int k0, int nk) {   // thread k0 of nk: its share of every piece, in piece order
-        for (int k = 0; k < RESULT_PIECES; ++k) {
+        for (int k = 0; k < pieces; ++k) {
             if (N > 0 && cudaEventSynchronize(e->ev_piece[k]) != cudaSuccess) {
                 piece_err = 1;
                 return;
             }
-            const long long q0 = N * k / RESULT_PIECES, q1 = N * (k + 1) / RESULT_PIECES;
+            const long long q0 = N * k / pieces, q1 = N * (k + 1) / pieces;
             convert(q0 + (q1 - q0) * k0 / nk, q0 + (q1 - q0) * (k0 + 1) / nk);
         }
     };
@@ -1785,7 +1780,8 @@ oa_status autotune_impl(oa_engine* e, const float* xr, int mb, oa_tuning* best_o
         for (int rep = 0; rep < 3; ++rep) {   // first run: allocations and kernel attributes
             const oa_status s = run_snps_any(e, xr, mb, false, false, &rows);
             if (s != OA_OK) return s;
-            if (rep > 0) sum += e->block_ms;   // the whole block on the device
+            float ms = 0.f;   // the whole block on the device
+            if (rep > 0 && cudaEventElapsedTime(&ms, e->k0, e->k1) == cudaSuccess) sum += ms;
         }
         *ms = sum / 2.f;
         return OA_OK;
@@ -2446,13 +2442,32 @@ oa_status oa_dense_flags(oa_engine* e, uint8_t* flags) {
 
 int64_t oa_kernel_launches(const oa_engine* e) { return e ? e->launches : 0; }
 
+// Sum of the elapsed times between the chunks' events of the last SNP block.  The events are read here
+// and not after every block: cudaEventElapsedTime takes about 4 us a pair, 0.24 ms for the 27 chunks of
+// 500,000 SNPs.
+static float chunk_ms(const oa_engine* e, const std::vector<cudaEvent_t>& a, const std::vector<cudaEvent_t>& b) {
+    float total = 0.f;
+    for (int c = 0; c < e->timed_chunks; ++c) {
+        float ms = 0.f;
+        if (cudaEventElapsedTime(&ms, a[c], b[c]) == cudaSuccess) total += ms;
+    }
+    cudaGetLastError();
+    return total;
+}
+
 float oa_last_kernel_ms(const oa_engine* e, const char** name) {
     if (!e) return 0.f;
     if (name) *name = e->last_name;
-    return e->last_ms;
+    return chunk_ms(e, e->cev0, e->cev1);
 }
 
-float oa_last_stats_ms(const oa_engine* e) { return e ? e->stats_ms : 0.f; }
-float oa_last_block_ms(const oa_engine* e) { return e ? e->block_ms : 0.f; }
+float oa_last_stats_ms(const oa_engine* e) { return e ? chunk_ms(e, e->sev0, e->sev1) : 0.f; }
+float oa_last_block_ms(const oa_engine* e) {
+    float ms = 0.f;
+    if (!e || !e->block_timed) return 0.f;
+    const bool ok = cudaEventElapsedTime(&ms, e->k0, e->k1) == cudaSuccess;
+    cudaGetLastError();
+    return ok ? ms : 0.f;
+}
 
 }  // extern "C"
