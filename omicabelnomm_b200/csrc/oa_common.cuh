@@ -138,36 +138,24 @@ __device__ __forceinline__ void split_half(float xs, __half& hi, __half& lo) {
     lo = __float2half_rn(xs - __half2float(hi));
 }
 
-// BF16 hi/lo of 8 floats (x = hi + lo to ~2^-17 relative), packed
-__device__ __forceinline__ void split8(const float4 p0, const float4 p1, uint4& hi, uint4& lo) {
-    const float e[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-    uint32_t h[4], o[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const __nv_bfloat162 hb = __floats2bfloat162_rn(e[2 * u], e[2 * u + 1]);
-        const float2 hf = __bfloat1622float2(hb);
-        const __nv_bfloat162 lb = __floats2bfloat162_rn(e[2 * u] - hf.x, e[2 * u + 1] - hf.y);
-        h[u] = *reinterpret_cast<const uint32_t*>(&hb);
-        o[u] = *reinterpret_cast<const uint32_t*>(&lb);
-    }
-    hi = make_uint4(h[0], h[1], h[2], h[3]);
-    lo = make_uint4(o[0], o[1], o[2], o[3]);
+// BF16 hi/lo of 4 floats (x = hi + lo to ~2^-17 relative), packed
+__device__ __forceinline__ void split4(const float4 p, uint2& hi, uint2& lo) {
+    const __nv_bfloat162 h0 = __floats2bfloat162_rn(p.x, p.y), h1 = __floats2bfloat162_rn(p.z, p.w);
+    const float2 f0 = __bfloat1622float2(h0), f1 = __bfloat1622float2(h1);
+    const __nv_bfloat162 l0 = __floats2bfloat162_rn(p.x - f0.x, p.y - f0.y);
+    const __nv_bfloat162 l1 = __floats2bfloat162_rn(p.z - f1.x, p.w - f1.y);
+    hi = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+    lo = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
 }
 
-// FP16 hi/lo of 8 floats times sc (a power of two), packed
-__device__ __forceinline__ void split8h(const float4 p0, const float4 p1, float sc, uint4& hi, uint4& lo) {
-    const float e[8] = {p0.x * sc, p0.y * sc, p0.z * sc, p0.w * sc, p1.x * sc, p1.y * sc, p1.z * sc, p1.w * sc};
-    uint32_t h[4], o[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const __half2 hb = __floats2half2_rn(e[2 * u], e[2 * u + 1]);
-        const float2 hf = __half22float2(hb);
-        const __half2 lb = __floats2half2_rn(e[2 * u] - hf.x, e[2 * u + 1] - hf.y);
-        h[u] = *reinterpret_cast<const uint32_t*>(&hb);
-        o[u] = *reinterpret_cast<const uint32_t*>(&lb);
-    }
-    hi = make_uint4(h[0], h[1], h[2], h[3]);
-    lo = make_uint4(o[0], o[1], o[2], o[3]);
+// FP16 hi/lo of 4 floats times sc (a power of two), packed
+__device__ __forceinline__ void split4h(const float4 p, float sc, uint2& hi, uint2& lo) {
+    const float x = p.x * sc, y = p.y * sc, z = p.z * sc, w = p.w * sc;
+    const __half2 h0 = __floats2half2_rn(x, y), h1 = __floats2half2_rn(z, w);
+    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+    const __half2 l0 = __floats2half2_rn(x - f0.x, y - f0.y), l1 = __floats2half2_rn(z - f1.x, w - f1.y);
+    hi = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+    lo = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
 }
 
 // In-place inverse of a small SPD matrix (row-major k x k, k <= OA_MAX_R or

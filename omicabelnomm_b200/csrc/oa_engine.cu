@@ -322,16 +322,13 @@ struct oa_engine {
     // tuning: requested (0 = automatic) and in effect
     oa_tuning req{};
     int variant = 1, raster = 1, lean_spb = 0;
-    // statistics-kernel layout requests (environment; 0 / -1 = the plan's choice): column buffers (1, 2)
-    // and the row-interleaved column copy of the set pass (0, 1)
-    int lean_nbuf = 0, lean_xi = -1;
     int lean_threads_req = 0;   // 256 or 512 threads per column-statistics CTA (OA_LEAN_THREADS), 0: by n
     // work items of the lean kernel's set pass (per trait block) and its launch plan
-    DBuf<int> item_start, set_item_off, pass_off;
+    DBuf<int> items, set_item_off, set_blk_off, pass_off;   // items: {first index block, rows} pairs
+    DBuf<uint16_t> item_rows;   // the sets' rows in the order the set pass reads them
     std::vector<int> h_set_item_off;
     struct LeanPlan {
-        int spb = 0, nbuf = 0, items_cap = 0, npass = 0;
-        bool xi = true;   // row-interleaved column copy for the set pass
+        int spb = 0, items_cap = 0, npass = 0;
         size_t smem = 0;
     } lp;
     long long tune_gen = 0;
@@ -444,7 +441,7 @@ void for_each_buf(oa_engine* e, F&& f) {
     f(e->rec); f(e->rec2); f(e->cov); f(e->cov2); f(e->counters); f(e->keys); f(e->keys2); f(e->perm);
     f(e->perm2); f(e->cub_tmp);
     f(e->d_beta); f(e->d_se); f(e->d_t); f(e->d_r2); f(e->d_sig); f(e->d_flags); f(e->xrows);
-    f(e->item_start); f(e->set_item_off); f(e->pass_off); f(e->marks);
+    f(e->items); f(e->item_rows); f(e->set_item_off); f(e->set_blk_off); f(e->pass_off); f(e->marks);
 }
 
 // Columns [c0, c0 + ncol) of a strided block gathered to the engine's rows.
@@ -733,16 +730,22 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->W.ensure((size_t)std::max(e->G, 1) * l * l));
     OA_CHECK(e->zQ.ensure((size_t)std::max(e->Z, 1) * l * l));
     OA_CHECK(e->pat_bad.ensure(std::max(e->G, 1)));
-    // work items of at most LEAN_ITEM_ROWS rows of one set, tiling the flattened row lists
-    std::vector<int> istart;
+    // index blocks of LEAN_BLOCK_ROWS rows of one set, and work items of some of a set's blocks
+    std::vector<int> blk_off(e->nsets + 1, 0), items;
+    for (int s2 = 0; s2 < e->nsets; ++s2)
+        blk_off[s2 + 1] = blk_off[s2] + (off[s2 + 1] - off[s2] + LEAN_BLOCK_ROWS - 1) / LEAN_BLOCK_ROWS;
+    const int item_rows = lean_item_rows(blk_off[e->nsets]);
     e->h_set_item_off.assign(e->nsets + 1, 0);
     for (int s2 = 0; s2 < e->nsets; ++s2) {
-        e->h_set_item_off[s2] = (int)istart.size();
-        for (int r0 = off[s2]; r0 < off[s2 + 1]; r0 += LEAN_ITEM_ROWS) istart.push_back(r0);
+        e->h_set_item_off[s2] = (int)items.size() / 2;
+        for (int r0 = off[s2]; r0 < off[s2 + 1]; r0 += item_rows) {
+            items.push_back(blk_off[s2] + (r0 - off[s2]) / LEAN_BLOCK_ROWS);
+            items.push_back(std::min(item_rows, off[s2 + 1] - r0));
+        }
     }
-    e->h_set_item_off[e->nsets] = (int)istart.size();
-    istart.push_back(off[e->nsets]);
-    OA_CHECK(e->item_start.ensure(istart.size()));
+    e->h_set_item_off[e->nsets] = (int)items.size() / 2;
+    OA_CHECK(e->items.ensure(items.size()));
+    OA_CHECK(e->set_blk_off.ensure(blk_off.size()));
     OA_CHECK(e->set_item_off.ensure(e->h_set_item_off.size()));
     H2DBatch h2d;
     h2d.add(e->pat.p, ipat);
@@ -753,13 +756,20 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     h2d.add(e->set_rep.p, rep);
     h2d.add(e->set_kind.p, kind);
     h2d.add(e->set_slot.p, slot);
-    h2d.add(e->item_start.p, istart);
+    h2d.add(e->items.p, items);
+    h2d.add(e->set_blk_off.p, blk_off);
     h2d.add(e->set_item_off.p, e->h_set_item_off);
     OA_CHECK(flush_h2d(e, h2d));
     k_set_rows<<<e->nsets, OA_NTHREADS, 0, e->st>>>(Y, (size_t)n, n, e->set_rep.p, e->set_kind.p, e->set_off.p,
                                                    e->set_rows.p);
     k_set_gram<<<e->nsets, OA_NTHREADS, 0, e->st>>>(e->Q64.p, n, l, e->set_kind.p, e->set_off.p, e->set_rows.p,
                                                    e->W.p, e->zQ.p, e->set_slot.p, e->pat_bad.p);
+    if (e->n_pad < 65536) {   // longer columns do not fit the statistics kernel's shared memory
+        OA_CHECK(e->item_rows.ensure((size_t)std::max(blk_off[e->nsets], 1) * LEAN_BLOCK_ROWS));
+        k_item_rows<<<e->nsets, 1024, 0, e->st>>>(e->set_rows.p, e->set_off.p, e->set_blk_off.p, e->n_pad,
+                                                  e->item_rows.p);
+        ++e->launches;
+    }
     const int total_rows = off[e->nsets];
     OA_CHECK(e->qrows.ensure((size_t)std::max(total_rows, 1) * e->LP));
     if (total_rows > 0) {
@@ -950,10 +960,10 @@ oa_status stats_gather(oa_engine* e, const float* X, int mbc) {
     return pick(std::integral_constant<int, 16>{});
 }
 
-// Lean path: k_snp_lean (imputation, BF16 split, X'X over all rows and over
+// Lean path: k_snp_lean (imputation, 16-bit split, X'X over all rows and over
 // each row set) -> pre-GEMM C2 = [Q | Q o m_1 | ...]'X -> k_schur.
-// SNPs per CTA group of k_snp_lean: requested, else two CTAs per SM where a
-// double-buffered group fits in half the shared memory (a power of two <= 8 / r)
+// SNPs per CTA group of k_snp_lean: requested, else as many (a power of two <= 8 / r) as
+// LEAN_GROUP_BYTES of shared memory hold
 // With two or more columns per SNP and at most LEAN_QX_L covariates, k_snp_lean also sums the
 // all-rows covariate projection A = Q'X of every column (short FP32 partial sums, FP64 across
 // warps) for k_schur: the pre-GEMM's A (FP32 sums over all n rows; BF16 hi/lo products in the mixed
@@ -972,6 +982,9 @@ int lean_threads(const oa_engine* e) {
     return long_col ? LEAN_MAX_THREADS : 256;
 }
 
+// Shared memory of a group that takes several SNPs by itself: at least four CTAs per SM.
+constexpr size_t LEAN_GROUP_BYTES = 50 * 1024;
+
 int lean_group(const oa_engine* e) {
     if (lean_threads(e) == LEAN_MAX_THREADS) return 1;   // the 512-thread kernel takes one SNP per group
     const int cap = want_lean_qx(e) ? LEAN_QX_NC / e->r : 8 / e->r;
@@ -981,30 +994,21 @@ int lean_group(const oa_engine* e) {
         return std::min(s, cap);
     }
     int s = 1;
-    while (s * 2 <= cap && lean_smem_bytes(e->r, e->n_pad, s * 2, 2, 0, true, want_lean_qx(e)) <= 100 * 1024)
-        s *= 2;
+    while (s * 2 <= cap && lean_smem_bytes(e->r, e->n_pad, s * 2, 0, want_lean_qx(e)) <= LEAN_GROUP_BYTES) s *= 2;
     return s;
 }
 
 // Launch plan of k_snp_lean for the current trait block and tuning: SNPs per
-// group, column buffers, shared memory, and passes over the row sets whose
+// group, shared memory, and passes over the row sets whose
 // work items fit in shared memory.  Host-only (runs before any capture).
 oa_status lean_plan(oa_engine* e) {
     const int R = e->r;
     const size_t limit = 227 * 1024 - 1024;
     int spb = lean_group(e);
-    // A set pass heavier than the column passes (more rows in the row sets than in a column) is
-    // latency-bound: it runs faster with more CTAs per SM (one column buffer, no interleaved copy)
-    // than with a prefetched second buffer.
-    const long long set_rows = e->h_set_item_off.empty() ? 0 : (long long)e->h_set_item_off.back() * LEAN_ITEM_ROWS;
-    const bool heavy_sets = set_rows > e->n;
-    int nbuf = e->lean_nbuf ? e->lean_nbuf : (heavy_sets ? 1 : 2);
-    const bool xi = e->lean_xi >= 0 ? e->lean_xi == 1 : !heavy_sets;
     const bool qx = want_lean_qx(e);
-    while (spb > 1 && lean_smem_bytes(R, e->n_pad, spb, nbuf, 0, xi, qx) > 200 * 1024) spb /= 2;
-    if (lean_smem_bytes(R, e->n_pad, spb, nbuf, 0, xi, qx) > 200 * 1024) nbuf = 1;
-    const size_t base = lean_smem_bytes(R, e->n_pad, spb, nbuf, 0, xi, qx);
-    const size_t per_item = (size_t)spb * R * R * 4;
+    while (spb > 1 && lean_smem_bytes(R, e->n_pad, spb, 0, qx) > 200 * 1024) spb /= 2;
+    const size_t base = lean_smem_bytes(R, e->n_pad, spb, 0, qx);
+    const size_t per_item = (size_t)spb * (R * (R + 1) / 2) * 4;
     int max_items = 1;
     for (int s2 = 0; s2 < e->nsets; ++s2)
         max_items = std::max(max_items, e->h_set_item_off[s2 + 1] - e->h_set_item_off[s2]);
@@ -1014,7 +1018,7 @@ oa_status lean_plan(oa_engine* e) {
     }
     const int total_items = std::max(1, e->h_set_item_off.empty() ? 1 : e->h_set_item_off.back());
     const int cap = (int)std::min<size_t>((size_t)total_items, (limit - base) / per_item);
-    if (e->lp.spb == spb && e->lp.nbuf == nbuf && e->lp.items_cap == cap && e->lp.xi == xi) return OA_OK;
+    if (e->lp.spb == spb && e->lp.items_cap == cap) return OA_OK;
     std::vector<int> passes{0};
     for (int s0 = 0; s0 < e->nsets;) {
         int s1 = s0 + 1;
@@ -1028,11 +1032,9 @@ oa_status lean_plan(oa_engine* e) {
     OA_CHECK(flush_h2d(e, h2d));
     OA_CU(cudaStreamSynchronize(e->st));
     e->lp.spb = spb;
-    e->lp.nbuf = nbuf;
     e->lp.items_cap = cap;
     e->lp.npass = e->nsets > 0 ? (int)passes.size() - 1 : 0;
-    e->lp.xi = xi;
-    e->lp.smem = lean_smem_bytes(R, e->n_pad, spb, nbuf, cap, xi, qx);
+    e->lp.smem = lean_smem_bytes(R, e->n_pad, spb, cap, qx);
     return OA_OK;
 }
 
@@ -1062,10 +1064,9 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     A.n = e->n;
     A.n_pad = e->n_pad;
     A.mb = mbc;
-    A.nbuf = e->lp.nbuf;
     A.nsets = e->nsets;
-    A.rows = e->set_rows.p;
-    A.item_start = e->item_start.p;
+    A.item_rows = reinterpret_cast<const uint4*>(e->item_rows.p);
+    A.items = reinterpret_cast<const int2*>(e->items.p);
     A.set_item_off = e->set_item_off.p;
     A.pass_off = e->pass_off.p;
     A.npass = e->lp.npass;
@@ -1076,7 +1077,6 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     A.Dset = e->Dset.p;
     A.write_split = fused ? 0 : 1;
     A.xscale = e->cfg.precision == OA_PLAIN_FP32 ? e->xscale.p : nullptr;
-    A.use_xi = e->lp.xi ? 1 : 0;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
@@ -1953,8 +1953,6 @@ oa_status oa_engine_create(const oa_config* cfg, oa_engine** out) {
     if (const char* v = getenv("OA_STATS_PATH")) e->req.stats_path = std::string(v) == "pre" ? 1 : (std::string(v) == "gather" ? 2 : 0);
     if (const char* v = getenv("OA_TC_VARIANT")) e->req.gemm_variant = std::min(4, std::max(0, atoi(v)));
     if (const char* v = getenv("OA_LEAN_SPB")) e->req.lean_spb = std::max(0, atoi(v));
-    if (const char* v = getenv("OA_LEAN_NBUF")) e->lean_nbuf = atoi(v) == 1 ? 1 : (atoi(v) == 2 ? 2 : 0);
-    if (const char* v = getenv("OA_LEAN_XI")) e->lean_xi = atoi(v) == 0 ? 0 : (atoi(v) == 1 ? 1 : -1);
     if (const char* v = getenv("OA_LEAN_THREADS")) e->lean_threads_req = atoi(v) == 512 ? 512 : (atoi(v) == 256 ? 256 : 0);
     e->chunk = std::min(cfg->max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : 16384 / e->r);
     if (const char* v = getenv("OA_FUSED_SPLIT")) e->fuse_split = v[0] != '0';
@@ -2340,7 +2338,7 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         for (auto* b : {&e->sst, &e->a_r2, &e->inv_ncorr, &e->vf}) OA_CHECK(b->ensure(t));
         OA_CHECK(e->nobs.ensure(t));
         OA_CHECK(e->b0.ensure(t * l));
-        OA_CHECK(stage_reserve(e, 48 * t + 65536 + 16 * n / LEAN_ITEM_ROWS));
+        OA_CHECK(stage_reserve(e, 48 * t + 65536 + 16 * n / LEAN_BLOCK_ROWS));
     }
     const auto t_traits = std::chrono::steady_clock::now();
     {

@@ -14,6 +14,8 @@
 //     (D - D_g) - (A - A_g)' W_g (A - A_g)
 // and its inverse, plus var_x from the all-rows complement D - A'A.
 #pragma once
+#include <type_traits>
+
 #include "oa_stats.cuh"
 
 namespace oa {
@@ -22,10 +24,10 @@ struct LeanArgs {
     const float* X;       // SNP block, column c at X + c*ldx
     size_t ldx;
     const int* xrows;     // row k of a column is X[c*ldx + xrows[k]] (a row subset), or null: X[c*ldx + k]
-    int n, n_pad, mb, nbuf;
+    int n, n_pad, mb;
     int nsets;
-    const int* rows;          // flattened row lists of the row sets
-    const int* item_start;    // work items: rows [item_start[i], item_start[i+1]) of one set
+    const uint4* item_rows;   // rows of the sets in blocks of LEAN_BLOCK_ROWS 16-bit values (k_item_rows)
+    const int2* items;        // work items, each within one set: {first block, rows}
     const int* set_item_off;  // items of set s: [set_item_off[s], set_item_off[s+1])
     const int* pass_off;      // passes over sets [pass_off[p], pass_off[p+1]) whose items fit in shared memory
     int npass;
@@ -38,7 +40,6 @@ struct LeanArgs {
     __nv_bfloat16* Xlo;
     int write_split;
     float* xscale;        // FP16 split of the columns times a power of two, 1 / scale here ([mb*r]); null: BF16 split
-    int use_xi;           // with several columns per group: keep the row-interleaved copy for the set pass
     int center;           // take each column relative to its mean (valid when XL holds an intercept)
     int* err;
     // all-rows covariate projection A = Q'(x - shift) of every column, summed here (short FP32
@@ -58,53 +59,132 @@ struct LeanArgs {
 // for 512.
 constexpr int LEAN_MAX_THREADS = 512;
 constexpr int LEAN_MAX_WARPS = LEAN_MAX_THREADS / 32;
-constexpr int LEAN_ITEM_ROWS = 256;     // rows per work item of the set pass
+constexpr int LEAN_BLOCK_ROWS = 256;    // rows of a set per index block (one 16-byte load of eight rows per lane)
 constexpr int LEAN_STAGE_U = 8;         // elements per thread and step of the element-wise staging
 constexpr int LEAN_QX_L = 8;            // covariates of the in-kernel projection (l <= 8)
 constexpr int LEAN_QX_NC = 4;           // columns per group of the qx kernels
+constexpr int LEAN_COL_PAD = 8;         // floats after a staged column: its offset (0..3) and the pad row
 
-// Shared memory of k_snp_lean: nbuf column buffers (stride n_pad floats, the
-// tail [n, n_pad) kept zero) | with several columns per group, the centred
-// columns interleaved by row ([n_pad][spb*R], one vector load per row in the
-// set pass) | per-item partial sums | reduction scratch.
-__host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int nbuf, int items_cap,
-                                                  bool use_xi = true, bool qx = false) {
-    const int NC = spb * R;
-    const int NQ = 2 * NC + spb * R * R + (qx ? NC * LEAN_QX_L : 0);
-    return (size_t)(nbuf + (NC > 1 && use_xi ? 1 : 0)) * NC * n_pad * 4 + (size_t)items_cap * spb * R * R * 4 +
+// Shared memory of k_snp_lean: the group's columns (stride n_pad + LEAN_COL_PAD floats) | per-item
+// partial sums | reduction scratch.
+__host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int items_cap, bool qx = false) {
+    const int NC = spb * R, NU = spb * R * (R + 1) / 2;
+    const int NQ = NC + NU + (qx ? NC * LEAN_QX_L : 0);   // NU >= NC: also the NaN path's 2 NC sums
+    return (size_t)NC * (n_pad + LEAN_COL_PAD) * 4 + (size_t)items_cap * NU * 4 +
            (size_t)(LEAN_MAX_WARPS + 1) * NQ * 8 + 64;
 }
 
+// Rows per work item of the set pass: one block of a set where that gives the eight warps few items,
+// else up to four (each item ends in a shuffle reduction, which with 150 sets of 600 rows took more of
+// the shared-memory pipe than the rows themselves).
+constexpr int LEAN_ITEMS_ENOUGH = 128;
+inline int lean_item_rows(long long blocks) {
+    return LEAN_BLOCK_ROWS * (blocks > 2 * LEAN_ITEMS_ENOUGH ? 4 : (blocks > LEAN_ITEMS_ENOUGH ? 2 : 1));
+}
+
+// The rows of every set in the order the set pass reads them, in blocks of LEAN_BLOCK_ROWS: lane l of
+// step u of a block takes slot l * 8 + u (one 16-byte load of a lane covers its eight steps); slots past
+// the end of a set hold the pad row n_pad.  A set's rows are taken by their rank among its rows of the same
+// shared-memory bank (row % 32), then by bank, so that the 32 rows of a step fall into (nearly) as many
+// banks: in ascending order random rows of a set gave 3.4 wavefronts per load, and the statistics
+// kernel's shared-memory pipe was at 80 %.  One CTA of 32 warps per set, warp = bank.
+static __global__ void __launch_bounds__(1024)
+k_item_rows(const int* __restrict__ rows, const int* __restrict__ set_off, const int* __restrict__ set_blk_off,
+            int n_pad, uint16_t* __restrict__ item_rows) {
+    __shared__ int cnt[32];
+    const int s = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int r0 = set_off[s], r1 = set_off[s + 1];
+    uint16_t* out = item_rows + (size_t)set_blk_off[s] * LEAN_BLOCK_ROWS;
+    const int slots = (set_blk_off[s + 1] - set_blk_off[s]) * LEAN_BLOCK_ROWS;
+    for (int q = threadIdx.x; q < slots; q += blockDim.x) out[q] = (uint16_t)n_pad;
+    int c = 0;
+    for (int k0 = r0; k0 < r1; k0 += 32) {
+        const int row = k0 + lane < r1 ? rows[k0 + lane] : -1;
+        c += __popc(__ballot_sync(0xffffffffu, row >= 0 && row % 32 == w));
+    }
+    if (lane == 0) cnt[w] = c;
+    __syncthreads();   // counts, and the pad rows are in place
+    const int mine = cnt[lane];   // rows of bank `lane`
+    int rank = 0;
+    for (int k0 = r0; k0 < r1; k0 += 32) {
+        const int row = k0 + lane < r1 ? rows[k0 + lane] : -1;
+        unsigned m = __ballot_sync(0xffffffffu, row >= 0 && row % 32 == w);
+        for (; m; m &= m - 1, ++rank) {
+            const int r = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+            // rows of lower rank in every bank, then those of this rank in lower banks
+            const int pos = __reduce_add_sync(0xffffffffu, min(mine, rank)) +
+                            __popc(__ballot_sync(0xffffffffu, mine > rank) & ((1u << w) - 1u));
+            if (lane == 0)
+                out[pos / LEAN_BLOCK_ROWS * LEAN_BLOCK_ROWS + pos % 32 * 8 + pos % LEAN_BLOCK_ROWS / 32] = (uint16_t)r;
+        }
+    }
+}
+
+// Warp sums of the NV values of v: store(q, sum) is called for every q by one lane.  The lanes
+// halve the values between them while they halve the distance (31 shuffles for 32 values where
+// one butterfly per value takes 160), with the pairs, and so the bits, of a butterfly per value.
+template <int NV, class Store>
+__device__ __forceinline__ void warp_sums(const float (&v)[NV], Store&& store) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int base = 0; base < NV; base += 32) {
+        constexpr int REST = NV % 32 == 0 ? 32 : NV % 32;
+        const int cnt = NV - base >= 32 ? 32 : REST;           // values of this round (compile time)
+        constexpr int PMAX = NV >= 32 ? 32 : (NV > 16 ? 32 : (NV > 8 ? 16 : (NV > 4 ? 8 : (NV > 2 ? 4 : NV))));
+        float x[PMAX];
+#pragma unroll
+        for (int i = 0; i < PMAX; ++i) x[i] = i < cnt ? v[base + i < NV ? base + i : 0] : 0.f;
+        int m = PMAX, idx = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            if (m > 1) {
+                const bool up = (lane & o) != 0;
+                m /= 2;
+#pragma unroll
+                for (int i = 0; i < PMAX / 2; ++i)
+                    if (i < m) {
+                        const float keep = up ? x[i + m] : x[i], send = up ? x[i] : x[i + m];
+                        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                idx += up ? m : 0;
+            } else {
+                x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+            }
+        }
+        if ((lane & (32 / PMAX - 1)) == 0 && idx < cnt) store(base + idx, x[0]);
+    }
+}
+
 // Block-wide sum of NV floats per thread over NW warps: FP32 within a warp, FP64 across
-// warps (warp 0, fixed order); the first NB sums are copied to out[] on every
-// thread, all NV stay at red + LEAN_MAX_WARPS * NV until red is reused.
+// warps (in warp order; the values are spread over the warps); the first NB sums are copied to out[] on
+// every thread, all NV stay at red + LEAN_MAX_WARPS * NV until red is reused.
 template <int NW, int NV, int NB = NV>
 __device__ __forceinline__ void block_sum_fd(float (&v)[NV], double (&out)[NB], double* red /* [warps + 1][NV] */) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = warp_sumf(v[q]);
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) red[w * NV + q] = (double)v[q];
+    warp_sums<NV>(v, [&](int q, float sum) { red[w * NV + q] = (double)sum; });
     __syncthreads();
     double* bc = red + LEAN_MAX_WARPS * NV;
-    if (w == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            const double s = warp_sum(lane < NW ? red[lane * NV + q] : 0.0);
-            if (lane == 0) bc[q] = s;
-        }
+    for (int q = w; q < NV; q += NW) {
+        const double s = warp_sum(lane < NW ? red[lane * NV + q] : 0.0);
+        if (lane == 0) bc[q] = s;
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NB; ++q) out[q] = bc[q];
 }
 
-// One CTA handles SPB SNPs (SPB*R columns) per group; a persistent loop over
-// groups with the next group's columns streaming into shared memory (TMA
-// bulk copies of aligned columns; 4-byte cp.async copies otherwise, which also
-// gather a row subset of a resident genotype matrix) while this one is
-// processed:
+// Index of the pair (a, b), a <= b, among a SNP's R (R + 1) / 2 column pairs.
+template <int R>
+__host__ __device__ constexpr int lean_pair(int a, int b) {
+    return a * R - a * (a - 1) / 2 + (b - a);
+}
+
+// One CTA handles SPB SNPs (SPB*R columns) per group in a persistent loop over groups:
+//   staging the group's columns stream into shared memory by TMA bulk copies.  A column that does not
+//           start on a 16-byte boundary (any n that is no multiple of 4) is copied from the boundary
+//           below it to the one above its end and read at its offset o; the block's first and last
+//           columns, whose boundaries may lie outside the block, are then copied element by element.
+//           A row subset of a resident matrix (GATHER) is gathered by 4-byte cp.async copies.
 //   pass 1  column sums and raw cross products from float4 reads of the
 //           staged columns, one block reduction (FP64 across warps); NaN
 //           propagates, so a column whose sum is NaN is counted and
@@ -114,132 +194,173 @@ __device__ __forceinline__ void block_sum_fd(float (&v)[NV], double (&out)[NB], 
 //           (the Schur complements, X'y~ and var_x do not change; the sums
 //           lose their large common part); X'X of the shifted columns
 //           follows from the raw sums in FP64
-//   pass 2  BF16 hi/lo split of the shifted columns (tensor-core form) and,
-//           with several columns per group, their row-interleaved copy
-//   pass 3  X'X over each row set: work items of at most 256 rows of one set
-//           (fixed on the host per trait block) go round-robin to the warps;
-//           a warp's item sum (row indices prefetched, one vector load of
-//           the interleaved centred columns per row, shuffle reduction)
-//           lands in its own shared-memory slot, and a set's sum adds its
-//           items in order.  No atomics: the sums are bit-reproducible.
-template <int R, int SPB, bool BULK, bool QX = false, int NT = 256>
+//   pass 2  16-bit hi/lo split of the shifted columns
+//   pass 3  X'X over each row set: work items of up to four index blocks of one set
+//           (fixed per trait block) go round-robin to the warps; a warp's item
+//           sum (eight row indices per 16-byte load, gathers that seldom share
+//           a bank, shuffle reduction) lands in its own shared-memory slot, and
+//           a set's sum adds its items in order.  No atomics: the sums are
+//           bit-reproducible.
+// One column buffer and as many CTAs per SM as fit: the other CTAs cover a group's copy and its block
+// barriers better than a second buffer did (50,000 SNPs, statistics stage with two buffers / one:
+// n = 12,348 with 3 row sets 0.94 / 0.79 ms, n = 4,834 and two columns 2.97 / 1.42 ms).  Bound by HBM
+// where the row sets are few (n = 12,347: 5.9 TB/s of columns read and split written, 0.90 of a copy's
+// rate); with 20 sets of 500 rows the set pass takes the shared-memory pipe to 0.6 and it runs at
+// 4.8 TB/s (n = 10,000).  Unaligned columns: 0.86 ms where 4-byte copies took 1.27 (n = 12,347).
+template <int R, int SPB, bool GATHER, bool QX = false, int NT = 256>
 __global__ void __launch_bounds__(NT)
 k_snp_lean(LeanArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int NC = SPB * R;                 // columns per group
-    constexpr int K2 = SPB * R * R;             // X'X entries per group
+    constexpr int NP = R * (R + 1) / 2;         // column pairs per SNP
+    constexpr int NU = SPB * NP;                // X'X entries per group
     constexpr int NWARP = NT / 32;
-    const int n = A.n, nS = A.n_pad;
-    const size_t buf_floats = (size_t)NC * nS;
-    float* bufs = reinterpret_cast<float*>(smem_raw);                                   // [nbuf][NC][nS]
-    float* xi = bufs + (size_t)A.nbuf * buf_floats;                                     // [nS][NC] if NC > 1
-    const bool use_xi = NC > 1 && A.use_xi;
-    float* part = xi + (use_xi ? (size_t)NC * nS : 0);                                   // [items_cap][K2]
+    const int n = A.n, cs = A.n_pad + LEAN_COL_PAD;
+    float* cols = reinterpret_cast<float*>(smem_raw);                                    // [NC][cs]
+    float* part = cols + (size_t)NC * cs;                                                // [items_cap][NU]
     double* red = reinterpret_cast<double*>(
-        (reinterpret_cast<uintptr_t>(part + (size_t)A.items_cap * K2) + 7) & ~(uintptr_t)7);   // [LEAN_MAX_WARPS + 1][NQ]
-    __shared__ __align__(8) uint64_t mbar[2];
+        (reinterpret_cast<uintptr_t>(part + (size_t)A.items_cap * NU) + 7) & ~(uintptr_t)7);   // [LEAN_MAX_WARPS + 1][NQ]
+    __shared__ __align__(8) uint64_t mbar;
     __shared__ int stop;
     const int ngroups = (A.mb + SPB - 1) / SPB;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // some column starts or ends off a 16-byte boundary: copies write past column ends
+    const bool ragged = !GATHER && (((n | (int)(A.ldx & 3)) & 3) != 0 || (reinterpret_cast<uintptr_t>(A.X) & 15) != 0);
 
-    auto issue = [&](int g, int b) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier generic writes to the buffer
-        const int i0 = g * SPB;
-        const int ncol = min(SPB, A.mb - i0) * R;
-        const uint32_t bytes = (uint32_t)n * 4u;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(st_su32(&mbar[b])),
-                     "r"(bytes * (uint32_t)ncol)
+    // Offset (floats) of column c of the block below its first element, and whether the 16-byte
+    // boundaries around it may lie outside the block.
+    auto col_off = [&](int c) { return (int)((reinterpret_cast<uintptr_t>(A.X + (size_t)c * A.ldx) >> 2) & 3); };
+    auto col_edge = [&](int c) {
+        const int o = col_off(c);
+        return (c == 0 && o != 0) || (c == A.mb * R - 1 && ((o + n) & 3) != 0);
+    };
+    // thread 0: bulk copies of a group's columns
+    auto issue = [&](int g) {
+        const int c0 = g * SPB * R, ncol = min(SPB, A.mb - g * SPB) * R;
+        uint32_t total = 0;
+        for (int c = 0; c < ncol; ++c)
+            if (!col_edge(c0 + c)) total += ((uint32_t)(col_off(c0 + c) + n) * 4u + 15u) & ~15u;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(st_su32(&mbar)), "r"(total)
                      : "memory");
         for (int c = 0; c < ncol; ++c) {
-            const float* src = A.X + (size_t)(i0 * R + c) * A.ldx;
-            float* dst = bufs + (size_t)b * buf_floats + (size_t)c * nS;
+            if (col_edge(c0 + c)) continue;
+            const int o = col_off(c0 + c);
+            const float* src = A.X + (size_t)(c0 + c) * A.ldx - o;
             asm volatile(
                 "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                    st_su32(dst)),
-                "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(st_su32(&mbar[b]))
+                    st_su32(cols + (size_t)c * cs)),
+                "l"(reinterpret_cast<uint64_t>(src)), "r"(((uint32_t)(o + n) * 4u + 15u) & ~15u), "r"(st_su32(&mbar))
                 : "memory");
         }
     };
-
-    // element-wise staging (columns not 16-byte aligned, or a row subset): 4-byte
-    // cp.async copies, one commit group per group of columns and thread
-    auto stage = [&](int g, int b) {
+    // GATHER: 4-byte cp.async copies of the subset's rows, one commit group per group of columns and thread
+    auto stage = [&](int g) {
         const int i0 = g * SPB;
         const int ncol = min(SPB, A.mb - i0) * R;
         for (int c = 0; c < ncol; ++c) {
             const float* src = A.X + (size_t)(i0 * R + c) * A.ldx;
-            const uint32_t dst = st_su32(bufs + (size_t)b * buf_floats + (size_t)c * nS);
+            const uint32_t dst = st_su32(cols + (size_t)c * cs);
             // LEAN_STAGE_U elements per thread and step: the row indices of a step
             // are loaded together, so their latencies overlap
-            constexpr int nt = NT;
-            for (int k0 = threadIdx.x; k0 < n; k0 += LEAN_STAGE_U * nt) {
+            for (int k0 = threadIdx.x; k0 < n; k0 += LEAN_STAGE_U * NT) {
                 int kk[LEAN_STAGE_U];
 #pragma unroll
                 for (int u = 0; u < LEAN_STAGE_U; ++u) {
-                    const int k = k0 + u * nt;
-                    kk[u] = k < n ? (A.xrows ? __ldg(A.xrows + k) : k) : -1;
+                    const int k = k0 + u * NT;
+                    kk[u] = k < n ? __ldg(A.xrows + k) : -1;
                 }
 #pragma unroll
                 for (int u = 0; u < LEAN_STAGE_U; ++u)
                     if (kk[u] >= 0)
                         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                                         dst + 4u * (uint32_t)(k0 + u * nt)),
+                                         dst + 4u * (uint32_t)(k0 + u * NT)),
                                      "l"(src + kk[u])
                                      : "memory");
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (!BULK && (int)blockIdx.x < ngroups) stage(blockIdx.x, 0);
+    if (GATHER && (int)blockIdx.x < ngroups) stage(blockIdx.x);
 
-    // zero the column tails [n, n_pad) once: copies write only [0, n)
-    for (int q = threadIdx.x; q < A.nbuf * NC * (nS - n); q += blockDim.x) {
-        const int c = q / (nS - n), k = n + q % (nS - n);
-        bufs[(size_t)c * nS + k] = 0.f;
-    }
+    // zero the column tails once: aligned copies and gathers write only [0, n)
+    for (int q = threadIdx.x; q < NC * (cs - n); q += NT) cols[(size_t)(q / (cs - n)) * cs + n + q % (cs - n)] = 0.f;
     if (threadIdx.x == 0) {
         stop = 0;
-        if (BULK) {
-            for (int b = 0; b < 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_su32(&mbar[b])));
+        if (!GATHER) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_su32(&mbar)));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            if ((int)blockIdx.x < ngroups) issue(blockIdx.x, 0);
         }
     }
+    if (!GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // own writes to the columns
     __syncthreads();
+    if (!GATHER && threadIdx.x == 0 && (int)blockIdx.x < ngroups) issue(blockIdx.x);
 
-    int q = 0;
-    for (int g = blockIdx.x; g < ngroups; g += gridDim.x, ++q) {
+    uint32_t par = 0;
+    for (int g = blockIdx.x; g < ngroups; g += gridDim.x, par ^= 1u) {
         const int gn = g + gridDim.x;
-        const int b = A.nbuf == 2 ? (q & 1) : 0;
-        const uint32_t par = A.nbuf == 2 ? (uint32_t)((q >> 1) & 1) : (uint32_t)(q & 1);
-        float* xs = bufs + (size_t)b * buf_floats;
         const int i0 = g * SPB;
         const int nsnp = min(SPB, A.mb - i0);
         const int ncol = nsnp * R;
+        int off[NC];                           // offset of the column in its buffer
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            off[c] = ragged && c < ncol && !col_edge(i0 * R + c) ? col_off(i0 * R + c) : 0;
 
-        if (BULK) {
-            if (threadIdx.x == 0) {
-                if (A.nbuf == 2 && gn < ngroups) issue(gn, b ^ 1);
-                if (!st_mbar_wait(&mbar[b], par)) {
+        if (GATHER) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        } else {
+            if (ragged)
+                for (int c = 0; c < ncol; ++c)
+                    if (col_edge(i0 * R + c))
+                        for (int k = threadIdx.x; k < n; k += NT)
+                            cols[(size_t)c * cs + k] = __ldg(A.X + (size_t)(i0 * R + c) * A.ldx + k);
+            if (w == 0) {
+                int ok = 1;
+                if (lane == 0 && !st_mbar_wait(&mbar, par)) {
                     stop = 1;
                     atomicExch(A.err, 1);
+                    ok = 0;
+                }
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (ragged && ok) {   // the copies wrote up to three floats past each column
+                    st_mbar_try(&mbar, par);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        for (int k = n + lane; k < A.n_pad; k += 32) cols[(size_t)c * cs + off[c] + k] = 0.f;
                 }
             }
-            __syncthreads();
-            if (stop) break;
-            st_mbar_try(&mbar[b], par);
-        } else {
-            // the next group goes into the other buffer (read completely in the previous round)
-            if (A.nbuf == 2 && gn < ngroups) {
-                stage(gn, b ^ 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-            __syncthreads();
         }
-        const float4* x4 = reinterpret_cast<const float4*>(xs);
-        const int nS4 = nS / 4;
+        __syncthreads();
+        if (stop) break;
+        if (!GATHER) st_mbar_try(&mbar, par);
+
+        // Four consecutive rows of column c.  O: the offset of every column where it is known (0, or
+        // 1..3 of a single column), -1: off[c]
+        auto ld4 = [&](auto O, int c, int k4) -> float4 {
+            const float4* p = reinterpret_cast<const float4*>(cols + (size_t)c * cs) + k4;
+            const float4 x = p[0];
+            const int o = decltype(O)::value >= 0 ? decltype(O)::value : off[c];
+            if (o == 0) return x;
+            const float4 y = p[1];
+            if (o == 1) return make_float4(x.y, x.z, x.w, y.x);
+            if (o == 2) return make_float4(x.z, x.w, y.x, y.y);
+            return make_float4(x.w, y.x, y.y, y.z);
+        };
+        auto by_offset = [&](auto&& f) {
+            if constexpr (GATHER) {
+                f(std::integral_constant<int, 0>{});
+            } else if constexpr (NC == 1) {
+                switch (off[0]) {
+                    case 0: f(std::integral_constant<int, 0>{}); break;
+                    case 1: f(std::integral_constant<int, 1>{}); break;
+                    case 2: f(std::integral_constant<int, 2>{}); break;
+                    default: f(std::integral_constant<int, 3>{}); break;
+                }
+            } else {
+                if (ragged) f(std::integral_constant<int, -1>{});
+                else f(std::integral_constant<int, 0>{});
+            }
+        };
 
         // ---- pass 1: column sums and raw cross products in one sweep (the
         // zero tail adds nothing); NaN propagates, so a column whose sum is
@@ -247,107 +368,111 @@ k_snp_lean(LeanArgs A) {
         // and the sweep is repeated - rare, dosage files seldom hold NaN
         float sh[NC];                          // subtracted from every value (centring), 0 without
         float hs[NC];                          // scale of the FP16 split
-        bool cnan[NC];
         {
             constexpr int NQX = QX ? NC * LEAN_QX_L : 0;
-            constexpr int NV = NC + K2 + NQX;  // [column sums | cross products | Q'x of the raw columns]
-            constexpr int NB = NC + K2;        // sums every thread keeps (Q'x stays in shared memory)
+            constexpr int NV = NC + NU + NQX;  // [column sums | cross products | Q'x of the raw columns]
+            constexpr int NB = NC + NU;        // sums every thread keeps (Q'x stays in shared memory)
             static_assert(!QX || NC <= LEAN_QX_NC, "columns of the qx kernels");
-            float acc[NV];
             double tot[NB];
             const double* qxs = red + LEAN_MAX_WARPS * NV + NB;   // the block's Q'x sums after the last sweep
-            auto sweep = [&]() {
+            bool cnan[NC];
+            float cmean[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) cnan[c] = false;
+            for (int round = 0;; ++round) {
+                float acc[NV];
 #pragma unroll
                 for (int u = 0; u < NV; ++u) acc[u] = 0.f;
-                for (int k4 = threadIdx.x; k4 < nS4; k4 += blockDim.x) {
-                    float4 v[NC];
+                by_offset([&](auto O) {
+                    for (int k4 = threadIdx.x; k4 < A.n_pad / 4; k4 += NT) {
+                        float4 v[NC];
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        v[c] = c < ncol ? x4[(size_t)c * nS4 + k4] : make_float4(0.f, 0.f, 0.f, 0.f);
-                        acc[c] += (v[c].x + v[c].y) + (v[c].z + v[c].w);
-                    }
-                    if constexpr (QX) {
-                        // rows 4 k4 .. 4 k4 + 3 of each covariate: one 16-byte load per covariate
+                        for (int c = 0; c < NC; ++c) {
+                            v[c] = c < ncol ? ld4(O, c, k4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            acc[c] += (v[c].x + v[c].y) + (v[c].z + v[c].w);
+                        }
+                        if constexpr (QX) {
+                            // rows 4 k4 .. 4 k4 + 3 of each covariate: one 16-byte load per covariate
 #pragma unroll
-                        for (int qq = 0; qq < LEAN_QX_L; ++qq) {
-                            if (qq < A.l) {
-                                const float4 q4 = __ldg(A.Qb + (size_t)k4 * A.l + qq);
+                            for (int qq = 0; qq < LEAN_QX_L; ++qq) {
+                                if (qq < A.l) {
+                                    const float4 q4 = __ldg(A.Qb + (size_t)k4 * A.l + qq);
 #pragma unroll
-                                for (int c = 0; c < NC; ++c) {
-                                    float& a = acc[NC + K2 + c * LEAN_QX_L + qq];
-                                    a = fmaf(q4.x, v[c].x, a);
-                                    a = fmaf(q4.y, v[c].y, a);
-                                    a = fmaf(q4.z, v[c].z, a);
-                                    a = fmaf(q4.w, v[c].w, a);
+                                    for (int c = 0; c < NC; ++c) {
+                                        float& a = acc[NC + NU + c * LEAN_QX_L + qq];
+                                        a = fmaf(q4.x, v[c].x, a);
+                                        a = fmaf(q4.y, v[c].y, a);
+                                        a = fmaf(q4.z, v[c].z, a);
+                                        a = fmaf(q4.w, v[c].w, a);
+                                    }
                                 }
                             }
                         }
+#pragma unroll
+                        for (int s2 = 0; s2 < SPB; ++s2)
+#pragma unroll
+                            for (int a = 0; a < R; ++a)
+#pragma unroll
+                                for (int bb = a; bb < R; ++bb) {
+                                    const float4 xa = v[s2 * R + a], xb = v[s2 * R + bb];
+                                    float& d = acc[NC + s2 * NP + lean_pair<R>(a, bb)];
+                                    d = fmaf(xa.x, xb.x, d);
+                                    d = fmaf(xa.y, xb.y, d);
+                                    d = fmaf(xa.z, xb.z, d);
+                                    d = fmaf(xa.w, xb.w, d);
+                                }
                     }
-#pragma unroll
-                    for (int s2 = 0; s2 < SPB; ++s2)
-#pragma unroll
-                        for (int a = 0; a < R; ++a)
-#pragma unroll
-                            for (int bb = 0; bb < R; ++bb) {
-                                const float4 xa = v[s2 * R + a], xb = v[s2 * R + bb];
-                                float& d = acc[NC + (s2 * R + a) * R + bb];
-                                d = fmaf(xa.x, xb.x, d);
-                                d = fmaf(xa.y, xb.y, d);
-                                d = fmaf(xa.z, xb.z, d);
-                                d = fmaf(xa.w, xb.w, d);
-                            }
-                }
+                });
                 block_sum_fd<NWARP, NV, NB>(acc, tot, red);
-            };
-            sweep();
-            bool any_nan = false;
-            float cmean[NC];
+                if (round == 1) break;
+                bool any_nan = false;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                cnan[c] = (c < ncol) && isnan(tot[c]);
-                any_nan |= cnan[c];
-                cmean[c] = (float)(tot[c] / (double)n);
-            }
-            if (any_nan) {   // block-uniform: count and sum the observed values, impute in place
+                for (int c = 0; c < NC; ++c) {
+                    cnan[c] = (c < ncol) && isnan(tot[c]);
+                    any_nan |= cnan[c];
+                    cmean[c] = (float)(tot[c] / (double)n);
+                }
+                if (!any_nan) break;
+                // block-uniform: count and sum the observed values, impute in place
                 __syncthreads();   // every thread has read the sums before the scratch is reused
-                float cs[2 * NC];
+                float ns[2 * NC];
                 double ct[2 * NC];
 #pragma unroll
-                for (int u = 0; u < 2 * NC; ++u) cs[u] = 0.f;
+                for (int u = 0; u < 2 * NC; ++u) ns[u] = 0.f;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     if (cnan[c]) {
-                        const float* col = xs + (size_t)c * nS;
-                        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+                        const float* col = cols + (size_t)c * cs + off[c];
+                        for (int k = threadIdx.x; k < n; k += NT) {
                             const float v = col[k];
-                            if (isnan(v)) cs[NC + c] += 1.f;
-                            else cs[c] += v;
+                            if (isnan(v)) ns[NC + c] += 1.f;
+                            else ns[c] += v;
                         }
                     }
                 }
-                block_sum_fd<NWARP, 2 * NC>(cs, ct, red);
+                block_sum_fd<NWARP, 2 * NC>(ns, ct, red);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     if (cnan[c]) {
                         cmean[c] = (float)(ct[c] / ((double)n - ct[NC + c]));
-                        float* col = xs + (size_t)c * nS;
-                        for (int k = threadIdx.x; k < n; k += blockDim.x)
+                        float* col = cols + (size_t)c * cs + off[c];
+                        for (int k = threadIdx.x; k < n; k += NT)
                             if (isnan(col[k])) col[k] = cmean[c];
                     }
                 }
                 __syncthreads();
-                sweep();
             }
 #pragma unroll
-            for (int c = 0; c < NC; ++c) sh[c] = A.center ? cmean[c] : 0.f;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) hs[c] = 1.f;
+            for (int c = 0; c < NC; ++c) {
+                sh[c] = A.center ? cmean[c] : 0.f;
+                hs[c] = 1.f;
+            }
             if (A.xscale) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     // sum of squares of the shifted column; the second term keeps it an upper bound
                     // where the FP32 sums cancel (a column that is constant but for its last digits)
-                    const double raw = tot[NC + c * R + c % R], s0 = sh[c];
+                    const double raw = tot[NC + c / R * NP + lean_pair<R>(c % R, c % R)], s0 = sh[c];
                     const double d = raw - 2.0 * s0 * tot[c] + (double)n * s0 * s0;
                     float inv = 1.f;
                     hs[c] = half_scale(fmax(d, 0.0) + raw * 0x1p-18, &inv);
@@ -373,155 +498,119 @@ k_snp_lean(LeanArgs A) {
                         if (cnan[c]) atomicOr(A.has_nan, 1);
                     }
                 }
-                // X'X of the columns taken relative to sh over the n rows:
-                // sum x_a x_b - s_a sum x_b - s_b sum x_a + n s_a s_b
+            }
+            // X'X of the columns taken relative to sh over the n rows, pairs spread over the warps:
+            // sum x_a x_b - s_a sum x_b - s_b sum x_a + n s_a s_b
 #pragma unroll
-                for (int s2 = 0; s2 < SPB; ++s2)
+            for (int s2 = 0; s2 < SPB; ++s2)
 #pragma unroll
-                    for (int a = 0; a < R; ++a)
+                for (int a = 0; a < R; ++a)
 #pragma unroll
-                        for (int bb = 0; bb < R; ++bb) {
-                            const int ca = s2 * R + a, cb = s2 * R + bb, u = (s2 * R + a) * R + bb;
+                    for (int bb = a; bb < R; ++bb) {
+                        const int ca = s2 * R + a, cb = s2 * R + bb, u = s2 * NP + lean_pair<R>(a, bb);
+                        if (lane == 0 && w == u % NWARP && s2 < nsnp) {
                             const double sa = sh[ca], sb = sh[cb];
-                            const double d = tot[NC + u] - sa * tot[cb] - sb * tot[ca] + (double)n * sa * sb;
-                            if (s2 < nsnp) A.D[(size_t)i0 * R * R + u] = (float)d;
+                            const float d = (float)(tot[NC + u] - sa * tot[cb] - sb * tot[ca] + (double)n * sa * sb);
+                            A.D[(size_t)(i0 + s2) * R * R + a * R + bb] = d;
+                            A.D[(size_t)(i0 + s2) * R * R + bb * R + a] = d;
                         }
-            }
+                    }
         }
 
-        // ---- pass 2: BF16 hi/lo split of the centred columns (tensor-core
-        // form) and, with several columns per group, the centred columns
-        // interleaved by row for the set pass; 8 rows per thread and step.
-        // The tail rows [n, n_pad) get -sh: the other operands of the GEMMs
-        // are zero there.
-        if (A.write_split || use_xi) {
-            const int np8 = nS / 8;
-            for (int k8 = threadIdx.x; k8 < np8; k8 += blockDim.x) {
-                float e[NC][8];
+        // ---- pass 2: 16-bit hi/lo split of the shifted columns, 4 rows per thread and step (eight
+        // rows, two 16-byte loads at a 32-byte stride, cost two wavefronts for one).  The tail rows
+        // [n, n_pad) get -sh: the other operands of the GEMMs are zero there.
+        if (A.write_split) {
+            by_offset([&](auto O) {
+#pragma unroll 2
+                for (int k4 = threadIdx.x; k4 < A.n_pad / 4; k4 += NT) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
-                    if (c < ncol) {
-                        p0 = x4[(size_t)c * nS4 + 2 * k8];
-                        p1 = x4[(size_t)c * nS4 + 2 * k8 + 1];
-                    }
-                    const float s0 = sh[c];
-                    e[c][0] = p0.x - s0;
-                    e[c][1] = p0.y - s0;
-                    e[c][2] = p0.z - s0;
-                    e[c][3] = p0.w - s0;
-                    e[c][4] = p1.x - s0;
-                    e[c][5] = p1.y - s0;
-                    e[c][6] = p1.z - s0;
-                    e[c][7] = p1.w - s0;
-                    if (A.write_split && c < ncol) {
-                        uint4 h, o;
-                        const float4 lo4 = make_float4(e[c][0], e[c][1], e[c][2], e[c][3]);
-                        const float4 hi4 = make_float4(e[c][4], e[c][5], e[c][6], e[c][7]);
+                    for (int c = 0; c < NC; ++c) {
+                        if (c >= ncol) continue;
+                        const float s0 = sh[c];
+                        float4 p = ld4(O, c, k4);
+                        p.x -= s0; p.y -= s0; p.z -= s0; p.w -= s0;
+                        uint2 h, o;
                         if (A.xscale)
-                            split8h(lo4, hi4, hs[c], h, o);
+                            split4h(p, hs[c], h, o);
                         else
-                            split8(lo4, hi4, h, o);
-                        reinterpret_cast<uint4*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k8] = h;
-                        reinterpret_cast<uint4*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k8] = o;
+                            split4(p, h, o);
+                        reinterpret_cast<uint2*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k4] = h;
+                        reinterpret_cast<uint2*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k4] = o;
                     }
                 }
-                if (!use_xi) {
-                } else if constexpr (NC == 2) {
-                    float4* d = reinterpret_cast<float4*>(xi + (size_t)k8 * 16);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        d[u] = make_float4(e[0][2 * u], e[1][2 * u], e[0][2 * u + 1], e[1][2 * u + 1]);
-                } else if constexpr (NC == 4) {
-                    float4* d = reinterpret_cast<float4*>(xi + (size_t)k8 * 32);
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) d[u] = make_float4(e[0][u], e[1][u], e[2][u], e[3][u]);
-                } else if constexpr (NC > 1) {
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) xi[(size_t)(8 * k8 + u) * NC + c] = e[c][u];
-                }
-            }
-            if (use_xi) __syncthreads();   // xi is read by other warps in the set pass
+            });
         }
 
-        // ---- pass 3: X'X over each row set, by work items
+        // ---- pass 3: X'X over each row set, by work items.  The pad row holds the column's shift,
+        // so that empty slots add (x - sh)^2 = 0 (every warp writes it for itself: the same value)
+        if (A.npass > 0) {
+            if (lane == 0)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) cols[(size_t)c * cs + off[c] + A.n_pad] = sh[c];
+            __syncwarp();
+        }
         for (int ps = 0; ps < A.npass; ++ps) {
             const int s0 = __ldg(A.pass_off + ps), s1 = __ldg(A.pass_off + ps + 1);
             const int it0 = __ldg(A.set_item_off + s0), it1 = __ldg(A.set_item_off + s1);
             for (int item = it0 + w; item < it1; item += NWARP) {
-                const int ra = __ldg(A.item_start + item), rb = __ldg(A.item_start + item + 1);
-                float sacc[K2];
+                const int2 it = __ldg(A.items + item);
+                float sacc[NU];
 #pragma unroll
-                for (int u = 0; u < K2; ++u) sacc[u] = 0.f;
-                constexpr int U = LEAN_ITEM_ROWS / 32;
-                int kid[U];
+                for (int u = 0; u < NU; ++u) sacc[u] = 0.f;
+                const uint4* blk = A.item_rows + (size_t)it.x * 32 + lane;
+                for (int left = it.y; left > 0; left -= LEAN_BLOCK_ROWS, blk += 32) {
+                    const uint4 q = __ldg(blk);
+                    const uint32_t kid[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int kk = ra + 32 * u + lane;
-                    kid[u] = kk < rb ? __ldg(A.rows + kk) : -1;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (kid[u] >= 0) {
+                    for (int u = 0; u < LEAN_BLOCK_ROWS / 32; ++u) {
+                        if ((u == 2 || u == 4) && left <= 32 * u) break;   // warp-uniform
+                        const int k = (int)(u % 2 ? kid[u / 2] >> 16 : kid[u / 2] & 0xffffu);
                         float x[NC];
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            if (NC == 1 || !use_xi) {
-                                x[c] = xs[(size_t)c * nS + kid[u]] - sh[c];
-                            } else if constexpr (NC % 4 == 0) {
-                                if (c % 4 == 0) {
-                                    const float4 q4 = reinterpret_cast<const float4*>(xi + (size_t)kid[u] * NC)[c / 4];
-                                    x[c] = q4.x;
-                                    x[c + 1] = q4.y;
-                                    x[c + 2] = q4.z;
-                                    x[c + 3] = q4.w;
-                                }
-                            } else {
-                                if (c % 2 == 0) {
-                                    const float2 q2 = reinterpret_cast<const float2*>(xi + (size_t)kid[u] * NC)[c / 2];
-                                    x[c] = q2.x;
-                                    x[c + 1] = q2.y;
-                                }
-                            }
-                        }
+                        for (int c = 0; c < NC; ++c) x[c] = cols[(size_t)c * cs + off[c] + k] - sh[c];
 #pragma unroll
                         for (int s = 0; s < SPB; ++s)
 #pragma unroll
                             for (int a = 0; a < R; ++a)
 #pragma unroll
-                                for (int bb = 0; bb < R; ++bb)
-                                    sacc[(s * R + a) * R + bb] = fmaf(x[s * R + a], x[s * R + bb], sacc[(s * R + a) * R + bb]);
+                                for (int bb = a; bb < R; ++bb) {
+                                    float& d = sacc[s * NP + lean_pair<R>(a, bb)];
+                                    d = fmaf(x[s * R + a], x[s * R + bb], d);
+                                }
                     }
                 }
-#pragma unroll
-                for (int u = 0; u < K2; ++u) {
-                    const float v = warp_sumf(sacc[u]);
-                    if (lane == 0) part[(size_t)(item - it0) * K2 + u] = v;
-                }
+                warp_sums<NU>(sacc, [&](int u, float sum) { part[(size_t)(item - it0) * NU + u] = sum; });
             }
             __syncthreads();
-            for (int u = threadIdx.x; u < (s1 - s0) * K2; u += blockDim.x) {
-                const int set = s0 + u / K2, e = u % K2;
-                const int s = e / (R * R), f = e % (R * R);
+            for (int u = threadIdx.x; u < (s1 - s0) * NU; u += NT) {
+                const int set = s0 + u / NU, e = u % NU;
+                const int s = e / NP, f = e % NP;
                 const int a0 = __ldg(A.set_item_off + set), a1 = __ldg(A.set_item_off + set + 1);
                 float sum = 0.f;
-                for (int it = a0; it < a1; ++it) sum += part[(size_t)(it - it0) * K2 + e];
-                if (s < nsnp) A.Dset[((size_t)set * A.mb + i0 + s) * R * R + f] = sum;
+                for (int it = a0; it < a1; ++it) sum += part[(size_t)(it - it0) * NU + e];
+                if (s < nsnp) {
+                    int a = 0, bb = 0;
+#pragma unroll
+                    for (int x = 0; x < R; ++x)
+                        if (f >= lean_pair<R>(x, x)) a = x;
+                    bb = a + f - (a * R - a * (a - 1) / 2);
+                    float* d = A.Dset + ((size_t)set * A.mb + i0 + s) * R * R;
+                    d[a * R + bb] = sum;
+                    if (a != bb) d[bb * R + a] = sum;
+                }
             }
-            __syncthreads();
+            if (ps + 1 < A.npass) __syncthreads();   // the partial sums are read before the next pass's
         }
-        __syncthreads();   // every reader of this buffer is done before it is refilled
-        if (BULK && A.nbuf == 1 && threadIdx.x == 0 && gn < ngroups) issue(gn, 0);
-        if (!BULK && A.nbuf == 1 && gn < ngroups) stage(gn, 0);
+        if (!GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // own writes to the columns
+        __syncthreads();   // every reader of the columns is done before they are refilled
+        if (!GATHER && threadIdx.x == 0 && gn < ngroups) issue(gn);
+        if (GATHER && gn < ngroups) stage(gn);
     }
-    if (!BULK) asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing in flight at exit
-    if (BULK && threadIdx.x == 0 && stop) {
-        st_mbar_wait(&mbar[0], 0, true);
-        st_mbar_wait(&mbar[0], 1, true);
-        st_mbar_wait(&mbar[1], 0, true);
-        st_mbar_wait(&mbar[1], 1, true);
+    if (GATHER) asm volatile("cp.async.wait_group 0;" ::: "memory");   // nothing in flight at exit
+    if (!GATHER && threadIdx.x == 0 && stop) {
+        st_mbar_wait(&mbar, 0, true);
+        st_mbar_wait(&mbar, 1, true);
     }
 }
 

@@ -56,22 +56,20 @@ cudaError_t oa_launch_snp_stats(int R, int LP, const StatsArgs& A, int grid, siz
 
 template <int R, int SPB, bool QX, int NT = 256>
 static cudaError_t go_lean(const LeanArgs& A, int grid, size_t smem, cudaStream_t st) {
-    const bool bulk = !A.xrows && (A.n % 4 == 0) && (A.ldx % 4 == 0) &&
-                      ((reinterpret_cast<uintptr_t>(A.X) & 15) == 0);
-    static int set_bulk[64], set_plain[64];
+    static int set_bulk[64], set_gather[64];
     int dev = 0;
     cudaGetDevice(&dev);
     const int d = dev & 63;
-    int* done = bulk ? set_bulk : set_plain;
+    int* done = A.xrows ? set_gather : set_bulk;
     if (done[d] < (int)smem) {
-        cudaError_t e = bulk ? cudaFuncSetAttribute(k_snp_lean<R, SPB, true, QX, NT>,
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024)
-                             : cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QX, NT>,
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
+        cudaError_t e = A.xrows ? cudaFuncSetAttribute(k_snp_lean<R, SPB, true, QX, NT>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024)
+                                : cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QX, NT>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
         if (e != cudaSuccess) return e;
         done[d] = 227 * 1024 - 1024;
     }
-    if (bulk)
+    if (A.xrows)
         k_snp_lean<R, SPB, true, QX, NT><<<grid, NT, smem, st>>>(A);
     else
         k_snp_lean<R, SPB, false, QX, NT><<<grid, NT, smem, st>>>(A);
@@ -81,9 +79,9 @@ static cudaError_t go_lean(const LeanArgs& A, int grid, size_t smem, cudaStream_
 template <int R, int SPB, bool QX, int NT = 256>
 static int lean_occ(size_t smem) {
     int nb = 0;
-    if (cudaFuncSetAttribute(k_snp_lean<R, SPB, true, QX, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QX, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              227 * 1024 - 1024) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_snp_lean<R, SPB, true, QX, NT>, NT, smem) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_snp_lean<R, SPB, false, QX, NT>, NT, smem) !=
             cudaSuccess) {
         cudaGetLastError();
         return 0;

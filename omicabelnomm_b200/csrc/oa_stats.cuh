@@ -283,8 +283,8 @@ k_snp_stats(StatsArgs A) {
         }
 
         if (A.write_split) {
-            // BF16 or scaled FP16 hi/lo of each column, 8 elements (two 16-byte stores) per thread and step
-            const int np8 = A.n_pad / 8;
+            // BF16 or scaled FP16 hi/lo of each column, 4 elements per thread and step
+            const int np4 = A.n_pad / 4;
             for (int c = 0; c < ncol; ++c) {
                 const float* col = xs + (size_t)c * nS;
                 const float s0 = cshift[c];
@@ -294,20 +294,20 @@ k_snp_stats(StatsArgs A) {
                     sc = half_scale(d, &inv);
                     if (threadIdx.x == 0) A.xscale[i0 * R + c] = inv;
                 }
-                uint4* hi = reinterpret_cast<uint4*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad);
-                uint4* lo = reinterpret_cast<uint4*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad);
-                for (int k8 = threadIdx.x; k8 < np8; k8 += blockDim.x) {
-                    float e[8];
+                uint2* hi = reinterpret_cast<uint2*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad);
+                uint2* lo = reinterpret_cast<uint2*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad);
+                for (int k4 = threadIdx.x; k4 < np4; k4 += blockDim.x) {
+                    float e[4];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) e[u] = k8 * 8 + u < n ? col[k8 * 8 + u] - s0 : 0.f;
-                    const float4 p0 = make_float4(e[0], e[1], e[2], e[3]), p1 = make_float4(e[4], e[5], e[6], e[7]);
-                    uint4 h, o;
+                    for (int u = 0; u < 4; ++u) e[u] = k4 * 4 + u < n ? col[k4 * 4 + u] - s0 : 0.f;
+                    const float4 p = make_float4(e[0], e[1], e[2], e[3]);
+                    uint2 h, o;
                     if (A.xscale)
-                        split8h(p0, p1, sc, h, o);
+                        split4h(p, sc, h, o);
                     else
-                        split8(p0, p1, h, o);
-                    hi[k8] = h;
-                    lo[k8] = o;
+                        split4(p, h, o);
+                    hi[k4] = h;
+                    lo[k4] = o;
                 }
             }
         }
