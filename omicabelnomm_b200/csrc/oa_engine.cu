@@ -619,11 +619,40 @@ oa_status exact_trait_sets(oa_engine* e, const float* Y, int t, const std::vecto
     return OA_OK;
 }
 
-// The per-SNP covariate sums of the current trait block come from the pre-GEMM (else from row gathers,
-// which handle neither the quirk, nor padding columns, nor 8 columns per SNP).
+// Default SNPs per chunk: about 16,384/r, rounded so that the tensor-core
+// GEMM's 128 x 256 tiles fill whole waves of the persistent grid (one CTA
+// per SM): the M-tile count is a multiple of sm_count / gcd(sm_count, N-tiles).
+int wave_chunk(const oa_engine* e, int t) {
+    const int r = e->r;
+    const int n_tiles = std::max(1, (std::max(t, 1) + 255) / 256);
+    int a = e->sm_count, b = n_tiles;
+    while (b) {
+        const int q = a % b;
+        a = b;
+        b = q;
+    }
+    const int unit = e->sm_count / a;                       // M-tiles per whole number of waves
+    const int mt = std::max(unit, (16384 / r * r / 128 + unit - 1) / unit * unit);
+    return mt * 128 / r;
+}
+
+// SNPs per device chunk of the current trait block.
+int chunk_for(const oa_engine* e) {
+    return std::min(e->cfg.max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : wave_chunk(e, e->t));
+}
+
+// The per-SNP covariate sums of the current trait block come from the pre-GEMM, else from row gathers
+// (k_snp_stats, which handles neither the quirk, nor padding columns, nor 8 columns per SNP).  The
+// pre-GEMM is the faster one whatever the row sets (statistics stage, gathers / pre-GEMM: 100 patterns of
+// 50 rows at n = 1,000 0.67 / 0.16 ms, 128 of 24 rows at n = 8,000 2.60 / 0.59 ms, of 1,200 rows 13.2 / 1.3
+// ms, 1,000 of 3 rows at n = 6,000 4.4 / 1.0 ms); the gathers stay for blocks whose column matrix and
+// products would take more than PRE_BYTES (thousands of row sets with many covariates).
+constexpr size_t PRE_BYTES = 4ull << 30;
 bool use_pre_for(const oa_engine* e) {
-    return quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1 ||
-           (e->req.stats_path != 2 && e->c2 <= std::max(e->t, 256));
+    if (quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1) return true;
+    if (e->req.stats_path == 2) return false;
+    return e->c2 <= std::max(e->t, 256) ||
+           (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES;
 }
 
 oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_ptr) {
@@ -813,23 +842,6 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
 // the first time a trait block needs it.
 oa_status lean_plan(oa_engine* e);
 
-// Default SNPs per chunk: about 16,384/r, rounded so that the tensor-core
-// GEMM's 128 x 256 tiles fill whole waves of the persistent grid (one CTA
-// per SM): the M-tile count is a multiple of sm_count / gcd(sm_count, N-tiles).
-int wave_chunk(const oa_engine* e, int t) {
-    const int r = e->r;
-    const int n_tiles = std::max(1, (std::max(t, 1) + 255) / 256);
-    int a = e->sm_count, b = n_tiles;
-    while (b) {
-        const int q = a % b;
-        a = b;
-        b = q;
-    }
-    const int unit = e->sm_count / a;                       // M-tiles per whole number of waves
-    const int mt = std::max(unit, (16384 / r * r / 128 + unit - 1) / unit * unit);
-    return mt * 128 / r;
-}
-
 // A buffer of at least `want` elements that keeps its first `keep`.
 template <class T>
 oa_status grow_keep(oa_engine* e, DBuf<T>& b, size_t keep, size_t want) {
@@ -853,7 +865,7 @@ bool combined_columns(const oa_engine* e) {
 
 oa_status prepare_tuning(oa_engine* e) {
     const int l = e->l, n = e->n;
-    e->chunk = std::min(e->cfg.max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : wave_chunk(e, e->t));
+    e->chunk = chunk_for(e);
     // default pipeline: CTA pairs with 64-wide K-blocks (the fastest at wide trait blocks; blocks of
     // at most 128 traits take the 1-SM narrow tiles whatever the variant)
     e->variant = (e->req.gemm_variant >= 1 && e->req.gemm_variant <= 4) ? e->req.gemm_variant : 4;
