@@ -83,7 +83,7 @@ struct EpiArgs {
     unsigned long long* rec_valid;   // rows written (null: not counted)
     long long cap;
     unsigned long long* n_singular;
-    // dense outputs (optional): beta/se/t [t][mb][r], r2 [t][mb], sig [t][mb]
+    // dense outputs (optional): beta/se/t [t][mb][r], r2 [t][mb], sig [t][mb] (or null)
     float* d_beta;
     float* d_se;
     float* d_t;

@@ -994,9 +994,6 @@ int lean_threads(const oa_engine* e) {
     return long_col ? LEAN_MAX_THREADS : 256;
 }
 
-// Shared memory of a group that takes several SNPs by itself: at least four CTAs per SM.
-constexpr size_t LEAN_GROUP_BYTES = 50 * 1024;
-
 int lean_group(const oa_engine* e) {
     if (lean_threads(e) == LEAN_MAX_THREADS) return 1;   // the 512-thread kernel takes one SNP per group
     const int cap = want_lean_qx(e) ? LEAN_QX_NC / e->r : 8 / e->r;

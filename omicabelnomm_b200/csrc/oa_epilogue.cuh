@@ -174,7 +174,7 @@ __device__ __forceinline__ bool epi_core(const EpiArgs& E, int i, int j, const f
         const float nanf_ = __int_as_float(0x7fc00000);
         const bool pos = rss > 0.0;
         E.d_r2[o] = pos ? r2 : nanf_;
-        E.d_sig[o] = pos ? rc.sig : nanf_;
+        if (E.d_sig) E.d_sig[o] = pos ? rc.sig : nanf_;
 #pragma unroll
         for (int a = 0; a < R; ++a) {
             E.d_beta[o * R + a] = pos ? rc.b[a] : nanf_;
@@ -241,7 +241,7 @@ __device__ __forceinline__ bool epi_decide(const EpiArgs& E, int i, int j, const
         const float nanf_ = __int_as_float(0x7fc00000);
         const bool pos = rss > 0.0;
         E.d_r2[off] = pos ? o.r2 : nanf_;
-        E.d_sig[off] = pos ? sqrtf(fmaxf(o.sig2, 0.f)) : nanf_;
+        if (E.d_sig) E.d_sig[off] = pos ? sqrtf(fmaxf(o.sig2, 0.f)) : nanf_;
 #pragma unroll
         for (int a = 0; a < R; ++a) {
             E.d_beta[off * R + a] = pos ? o.b[a] : nanf_;
@@ -286,7 +286,7 @@ __device__ __forceinline__ void epi_dense_nan(const EpiArgs& E, int i, const Tra
     const size_t o = (size_t)tp.orig * E.dense_ld + E.snp_base + i;
     const float nanf_ = __int_as_float(0x7fc00000);
     E.d_r2[o] = nanf_;
-    E.d_sig[o] = nanf_;
+    if (E.d_sig) E.d_sig[o] = nanf_;
 #pragma unroll
     for (int a = 0; a < R; ++a) E.d_beta[o * R + a] = E.d_se[o * R + a] = E.d_t[o * R + a] = nanf_;
     if (E.d_flags) E.d_flags[o] = OA_TEST_SINGULAR;

@@ -224,7 +224,8 @@ k_set_gram(const double* __restrict__ Q64, int n, int l, const int* __restrict__
 // and BF16 hi/lo for the tensor-core form), RSS0, SST and the constants the
 // epilogue folds: a_r2 = (n-1)/((n_corr-1) SST), 1/n_corr, (n-miss)/n.
 // With yscale (the FP32-accurate tensor-core form) the split is FP16 of the
-// scaled residuals, written once RSS0 is known, and yscale[jj] = 1 / scale.
+// scaled residuals, written once RSS0 is known, and yscale[jj] = 1 / scale;
+// Yt may be null there (the residuals are then formed twice).
 static __global__ void __launch_bounds__(OA_NTHREADS)
 k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, int p,
               const double* __restrict__ Q64, const double* __restrict__ sums,
@@ -249,21 +250,21 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
     }
     __syncthreads();
     const float* y = Y + (size_t)j * ldy;
-    float* out = Yt + (size_t)jj * n_pad;
+    float* out = Yt ? Yt + (size_t)jj * n_pad : nullptr;
+    auto resid = [&](int k) -> double {   // 0 on missing rows and past the end
+        if (k >= n) return 0.0;
+        const float x = y[k];
+        if (isnan(x)) return 0.0;
+        double fit = 0.0;
+        for (int q = 0; q < l; ++q) fit += Q64[(size_t)q * n + k] * b0[q];
+        return (double)x - fit;
+    };
     double rss = 0.0;
     for (int k = threadIdx.x; k < n_pad; k += blockDim.x) {
-        float e = 0.0f;
-        if (k < n) {
-            const float x = y[k];
-            if (!isnan(x)) {
-                double fit = 0.0;
-                for (int q = 0; q < l; ++q) fit += Q64[(size_t)q * n + k] * b0[q];
-                const double d = (double)x - fit;
-                rss += d * d;
-                e = (float)d;
-            }
-        }
-        out[k] = e;
+        const double d = resid(k);
+        rss += d * d;
+        const float e = (float)d;
+        if (out) out[k] = e;
         if (Yhi && !yscale) {
             const __nv_bfloat16 hi = __float2bfloat16_rn(e);
             Yhi[(size_t)jj * n_pad + k] = hi;
@@ -297,7 +298,8 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
         const float sc = half_s;
         __half* yh = reinterpret_cast<__half*>(Yhi) + (size_t)jj * n_pad;
         __half* yl = reinterpret_cast<__half*>(Ylo) + (size_t)jj * n_pad;
-        for (int k = threadIdx.x; k < n_pad; k += blockDim.x) split_half(out[k] * sc, yh[k], yl[k]);   // own writes
+        for (int k = threadIdx.x; k < n_pad; k += blockDim.x)
+            split_half((out ? out[k] : (float)resid(k)) * sc, yh[k], yl[k]);   // out: own writes
     }
 }
 

@@ -74,6 +74,9 @@ __host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int
            (size_t)(LEAN_MAX_WARPS + 1) * NQ * 8 + 64;
 }
 
+// Shared memory of a group that takes several SNPs by itself: at least four CTAs per SM.
+constexpr size_t LEAN_GROUP_BYTES = 50 * 1024;
+
 // Rows per work item of the set pass: one block of a set where that gives the eight warps few items,
 // else up to four (each item ends in a shuffle reduction, which with 150 sets of 600 rows took more of
 // the shared-memory pipe than the rows themselves).

@@ -28,6 +28,7 @@
 
 #include "oa_kernels.cuh"
 #include "oa_launch.h"
+#include "oa_lean.cuh"
 
 namespace oa {
 namespace na {
@@ -195,40 +196,108 @@ __global__ void k_na_rank(const double* __restrict__ R1, const double* __restric
     }
 }
 
+// Inclusive block-wide sum over 1024 threads (all of them call it).
+__device__ __forceinline__ int block_scan(int v, int* warp_tot /* [32] */) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    __syncthreads();   // the previous scan's totals are read
+    if (lane == 31) warp_tot[w] = v;
+    __syncthreads();
+    int before = 0;
+    for (int q = 0; q < w; ++q) before += warp_tot[q];
+    return v + before;
+}
+
 // Row sets with every trait its own missingness pattern, plus one zero set
 // per trait that has observed values exactly 0.  counts[j] = (missing, zeros).
-__global__ void k_na_sets(const int* __restrict__ counts, int t, int* __restrict__ pat, int* __restrict__ zset,
-                          int* __restrict__ tperm, int* __restrict__ set_off, int* __restrict__ set_rep,
-                          int* __restrict__ set_kind, int* __restrict__ set_slot,
-                          int* __restrict__ info /* [0] Z, [1] rows */) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int z = 0, off = 0;
-    for (int j = 0; j < t; ++j) {
-        pat[j] = j;
-        tperm[j] = j;
-        set_off[j] = off;
-        set_rep[j] = j;
-        set_kind[j] = 0;
-        set_slot[j] = j;
-        off += counts[2 * j];
-    }
-    for (int j = 0; j < t; ++j) {
-        if (counts[2 * j + 1] > 0) {
-            const int s = t + z;
-            zset[j] = z;
-            set_off[s] = off;
-            set_rep[s] = j;
-            set_kind[s] = 1;
-            set_slot[s] = z;
-            off += counts[2 * j + 1];
-            ++z;
-        } else {
-            zset[j] = -1;
+// Also the index blocks of the sets (LEAN_BLOCK_ROWS rows each), whether the
+// first covariate is a constant, and the totals the host reads.  One block of
+// 1024 threads.
+__global__ void __launch_bounds__(1024)
+k_na_sets(const int* __restrict__ counts, int t, const float* __restrict__ xl, int n, int* __restrict__ pat,
+          int* __restrict__ zset, int* __restrict__ tperm, int* __restrict__ set_off, int* __restrict__ set_rep,
+          int* __restrict__ set_kind, int* __restrict__ set_slot, int* __restrict__ blk_off,
+          int* __restrict__ pass_off, int* __restrict__ info /* [0] Z, [1] rows, [6] constant, [7] blocks */) {
+    __shared__ int wt[32];
+    __shared__ int base[3];   // sets, rows, blocks so far
+    if (threadIdx.x < 3) base[threadIdx.x] = 0;
+    __syncthreads();
+    int varies = 0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) varies |= !(xl[k] == xl[0]);
+    for (int kind = 0; kind < 2; ++kind)   // the patterns, then the zero sets
+        for (int j0 = 0; j0 < t; j0 += blockDim.x) {
+            const int j = j0 + (int)threadIdx.x;
+            const int c = j < t ? counts[2 * j + kind] : 0;
+            const int has = j < t && (kind == 0 || c > 0);
+            const int blk = (c + LEAN_BLOCK_ROWS - 1) / LEAN_BLOCK_ROWS;
+            const int si = block_scan(has, wt), ri = block_scan(has ? c : 0, wt), bi = block_scan(has ? blk : 0, wt);
+            if (has) {
+                const int s = base[0] + si - 1;
+                set_off[s] = base[1] + ri - c;
+                blk_off[s] = base[2] + bi - blk;
+                set_rep[s] = j;
+                set_kind[s] = kind;
+                set_slot[s] = kind ? s - t : j;
+            }
+            if (j < t) {
+                if (kind == 0) pat[j] = tperm[j] = j;
+                else zset[j] = has ? base[0] + si - 1 - t : -1;
+            }
+            __syncthreads();
+            if (threadIdx.x == blockDim.x - 1) {
+                base[0] += si;
+                base[1] += ri;
+                base[2] += bi;
+            }
+            __syncthreads();
         }
+    varies = __syncthreads_or(varies);
+    if (threadIdx.x == 0) {
+        set_off[base[0]] = base[1];
+        blk_off[base[0]] = base[2];
+        pass_off[0] = 0;
+        pass_off[1] = base[0];
+        info[0] = base[0] - t;
+        info[1] = base[1];
+        info[6] = !varies && xl[0] != 0.f;
+        info[7] = base[2];
     }
-    set_off[t + z] = off;
-    info[0] = z;
-    info[1] = off;
+}
+
+// Work items of the column-statistics kernel: one per index block.
+__global__ void k_na_items(const int* __restrict__ set_off, const int* __restrict__ blk_off, int nsets,
+                           int2* __restrict__ items) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nsets) return;
+    int left = set_off[s + 1] - set_off[s];
+    for (int b = blk_off[s]; b < blk_off[s + 1]; ++b, left -= LEAN_BLOCK_ROWS)
+        items[b] = make_int2(b, min(left, LEAN_BLOCK_ROWS));
+}
+
+// The FP32 basis by blocks of four rows (k_snp_lean's projection) and its column sums; block = covariate.
+__global__ void __launch_bounds__(256)
+k_na_qblocks(const float* __restrict__ Qr, int LP, int n, int n_pad, int l, float* __restrict__ qb,
+             double* __restrict__ qsum) {
+    __shared__ double red[8];
+    const int q = blockIdx.x;
+    double s = 0.0;
+    for (int k = threadIdx.x; k < n_pad; k += blockDim.x) {
+        const float v = k < n ? Qr[(size_t)k * LP + q] : 0.f;
+        qb[((size_t)(k / 4) * l + q) * 4 + k % 4] = v;
+        s += (double)v;
+    }
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += red[w];
+        qsum[q] = t;
+    }
 }
 
 // Bump allocator over the scratch array (256-byte aligned pieces).
@@ -315,13 +384,15 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
     double* W = cv.take<double>((size_t)t * l * l);
     double* zQ = cv.take<double>((size_t)t * l * l);
     uint8_t* pat_bad = cv.take<uint8_t>(t);
-    float* Yt = cv.take<float>((size_t)t * n_pad);
     double* rss0 = cv.take<double>(t);
     float* sst = cv.take<float>(t);
     int* nobs = cv.take<int>(t);
     double* b0 = cv.take<double>((size_t)t * l);
-    float* mean = cv.take<float>((size_t)mb * r);
     int* has_nan = cv.take<int>(1);
+    const Carve per_trait = cv;   // both forms of the scan lay out the rest of the array from here
+    // FP32 form (below): also the measure of what the call accepts
+    float* Yt = cv.take<float>((size_t)t * n_pad);
+    float* mean = cv.take<float>((size_t)mb * r);
     float* varx = cv.take<float>((size_t)mb * r);
     double* sinv = cv.take<double>((size_t)t * mb * r * r);
     uint8_t* sing = cv.take<uint8_t>((size_t)t * mb);
@@ -330,6 +401,10 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         return fail(OA_ERR_UNSUPPORTED,
                     "oa_scan_dense_noalloc: n=%d t=%d mb=%d r=%d needs more than the %u-byte scratch array", n, t, mb,
                     r, (unsigned)OA_NOALLOC_SCRATCH_BYTES);
+    // tensor-core form: the sets' index blocks (in space the FP32 form writes later)
+    Carve tc = per_trait;
+    int* blk_off = tc.take<int>((size_t)2 * t + 1);
+    int* pass_off = tc.take<int>(2);
 
     // everything that must start at zero
     NA_CU(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st));
@@ -351,7 +426,8 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
     // traits: missing counts, sums, Q'y; one row set per trait
     TraitStatsOut tso{tsums, tcounts, thash};
     k_trait_stats<<<t, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, l, Q64, tso);
-    k_na_sets<<<1, 1, 0, st>>>(tcounts, t, pat, zset, tperm, set_off, set_rep, set_kind, set_slot, info);
+    k_na_sets<<<1, 1024, 0, st>>>(tcounts, t, xl, n, pat, zset, tperm, set_off, set_rep, set_kind, set_slot, blk_off,
+                                  pass_off, info);
     NA_CU(cudaGetLastError());
     int hinfo[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     NA_CU(cudaMemcpyAsync(hinfo, info, sizeof hinfo, cudaMemcpyDeviceToHost, st));
@@ -371,6 +447,185 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         return fail(OA_ERR_UNSUPPORTED,
                     "oa_scan_dense_noalloc: these inputs need %zu bytes of scratch, the array holds %u", cv.used,
                     (unsigned)OA_NOALLOC_SCRATCH_BYTES);
+    // statistics of mc SNPs from the block's SNP c0 on, dense outputs only
+    auto epi = [&](int mc, int c0) {
+        EpiArgs E{};
+        E.n = n;
+        E.l = l;
+        E.r = r;
+        E.p = l + r;
+        E.mb = mc;
+        E.G = t;
+        E.pat = pat;
+        E.zset = zset;
+        E.tperm = tperm;
+        E.rss0 = rss0;
+        E.a_r2 = a_r2;
+        E.inv_ncorr = inv_ncorr;
+        E.vf = vf;
+        E.b0 = b0;
+        E.zQ = zQ;
+        E.W = W;
+        E.store_all = 1;
+        E.rec = nullptr;
+        E.rec_count = counters;
+        E.rec_valid = nullptr;
+        E.cap = 0;
+        E.n_singular = counters + 1;
+        E.d_beta = beta;
+        E.d_se = se;
+        E.d_t = tstat;
+        E.d_r2 = r2;
+        E.t = t;
+        E.snp_base = c0;
+        E.dense_ld = mb;
+        return E;
+    };
+    auto finish = [&]() -> oa_status {
+        unsigned long long hc[4];
+        NA_CU(cudaMemcpyAsync(hc, counters, sizeof hc, cudaMemcpyDeviceToHost, st));
+        NA_CU(cudaStreamSynchronize(st));
+        if (hc[3]) return fail(OA_ERR_CUDA, "a device staging wait timed out");
+        return OA_OK;
+    };
+    // Tensor-core form: column statistics, one product with [Y~ | B2] per chunk of SNPs and the tests from
+    // it, as the engine's plain form.  Taken with an intercept as the first covariate (the columns are then
+    // centred; uncentred ones cancel more than the tensor-core sums keep) where its buffers fit the array
+    // with chunks of 256 SNPs or the whole block.  At n = 2,000 with 200 traits and 4,000 SNPs the FP32
+    // form's row gathers and SIMT product took 1.10 of 1.35 ms.
+    const bool qx = r >= 2 && l <= LEAN_QX_L;
+    if (hinfo[6] && (r == 1 || qx) && n_pad < 65536) {
+        const int nblk = hinfo[7], c2 = l * (1 + nsets), cols = t + c2;
+        int* rows = tc.take<int>((size_t)(nrows > 0 ? nrows : 1));
+        uint16_t* item_rows = tc.take<uint16_t>((size_t)(nblk > 0 ? nblk : 1) * LEAN_BLOCK_ROWS);
+        int2* items = tc.take<int2>((size_t)(nblk > 0 ? nblk : 1));
+        __nv_bfloat16* bhi = tc.take<__nv_bfloat16>((size_t)cols * n_pad);
+        __nv_bfloat16* blo = tc.take<__nv_bfloat16>((size_t)cols * n_pad);
+        float* cscale = tc.take<float>(cols);
+        const bool need_aobs = Z > 0;
+        const size_t per_snp = (size_t)r * n_pad * 4 + (size_t)r * cols * 4 + (size_t)r * 12 +
+                               (size_t)r * r * (4 + 4 * (size_t)nsets + 8 * (size_t)t) + t + (qx ? r * LEAN_QX_L * 8 : 0) +
+                               (need_aobs ? 4 * ((size_t)t * l * r + (size_t)Z * (l * r + r * r)) : 0);
+        // alignment of the pieces below, and the basis blocks
+        const size_t slack = 16 * 256 + (qx ? (size_t)n_pad * l * 4 + (size_t)l * 8 : 0);
+        const long long room = (long long)OA_NOALLOC_SCRATCH_BYTES - (long long)tc.used - (long long)slack;
+        long long fit = room > 0 ? room / (long long)per_snp : 0;
+        if (fit < mb) fit = fit / 256 * 256;
+        const int chunk = (int)(fit < mb ? fit : mb);
+        // column-statistics kernel: SNPs per group, threads and shared memory as the engine plans them
+        const int threads = r == 1 && (size_t)n_pad * 4 >= (size_t)64 * 1024 ? LEAN_MAX_THREADS : 256;
+        int spb = 1;
+        if (threads == 256)
+            while (spb * 2 * r <= (qx ? LEAN_QX_NC : 8) && lean_smem_bytes(r, n_pad, spb * 2, 0, qx) <= LEAN_GROUP_BYTES)
+                spb *= 2;
+        const size_t smem = lean_smem_bytes(r, n_pad, spb, nblk > 0 ? nblk : 1, qx);
+        if (chunk > 0 && smem <= 227 * 1024 - 1024) {
+            float* mean_c = tc.take<float>((size_t)chunk * r);
+            float* varx_c = tc.take<float>((size_t)chunk * r);
+            float* xscale = tc.take<float>((size_t)chunk * r);
+            float* D = tc.take<float>((size_t)chunk * r * r);
+            float* Dset = tc.take<float>((size_t)nsets * chunk * r * r);
+            __nv_bfloat16* xhi = tc.take<__nv_bfloat16>((size_t)chunk * r * n_pad);
+            __nv_bfloat16* xlo = tc.take<__nv_bfloat16>((size_t)chunk * r * n_pad);
+            float* C = tc.take<float>((size_t)cols * chunk * r);
+            double* sinv_c = tc.take<double>((size_t)t * chunk * r * r);
+            uint8_t* sing_c = tc.take<uint8_t>((size_t)t * chunk);
+            double* afull = qx ? tc.take<double>((size_t)chunk * r * LEAN_QX_L) : nullptr;
+            float* aobs_c = need_aobs ? tc.take<float>((size_t)t * chunk * l * r) : nullptr;
+            float* zA_c = need_aobs ? tc.take<float>((size_t)Z * chunk * l * r) : nullptr;
+            float* zD_c = need_aobs ? tc.take<float>((size_t)Z * chunk * r * r) : nullptr;
+            float* qb = nullptr;
+            double* qsum = nullptr;
+            if (qx) {
+                qb = tc.take<float>((size_t)n_pad * l);
+                qsum = tc.take<double>(l);
+            }
+            if (tc.used <= OA_NOALLOC_SCRATCH_BYTES) {
+                k_set_rows<<<nsets, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, rows);
+                k_set_gram<<<nsets, OA_NTHREADS, 0, st>>>(Q64, n, l, set_kind, set_off, rows, W, zQ, set_slot, pat_bad);
+                k_na_items<<<(nsets + 255) / 256, 256, 0, st>>>(set_off, blk_off, nsets, items);
+                k_item_rows<<<nsets, 1024, 0, st>>>(rows, set_off, blk_off, n_pad, item_rows);
+                k_trait_resid<<<t, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, n_pad, l, l + r, Q64, tsums, tcounts, pat, W,
+                                                        tperm, nullptr, bhi, blo, rss0, sst, nobs, b0, a_r2, inv_ncorr,
+                                                        vf, cscale);
+                const size_t ny = (size_t)t * n_pad, nb2 = (size_t)c2 * n_pad;
+                k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, st>>>(Qr, LP, n, n_pad, l, c2, 1, bhi + ny, blo + ny);
+                k_b2_scatter<<<nsets, 256, 0, st>>>(Qr, LP, n_pad, l, set_off, rows, 1, bhi + ny, blo + ny);
+                k_fill<<<(c2 + 255) / 256, 256, 0, st>>>(cscale + t, c2, 1.f / HALF_SCALE_Q);
+                if (qx) k_na_qblocks<<<l, 256, 0, st>>>(Qr, LP, n, n_pad, l, qb, qsum);
+                NA_CU(cudaGetLastError());
+                int sms = 148;
+                NA_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+                int* err = reinterpret_cast<int*>(counters + 3);
+                LeanArgs A{};
+                A.ldx = (size_t)n;
+                A.n = n;
+                A.n_pad = n_pad;
+                A.nsets = nsets;
+                A.item_rows = reinterpret_cast<const uint4*>(item_rows);
+                A.items = items;
+                A.set_item_off = blk_off;
+                A.pass_off = pass_off;
+                A.npass = 1;
+                A.items_cap = nblk > 0 ? nblk : 1;
+                A.mean = mean_c;
+                A.has_nan = has_nan;
+                A.D = D;
+                A.Dset = Dset;
+                A.Xhi = xhi;
+                A.Xlo = xlo;
+                A.write_split = 1;
+                A.xscale = xscale;
+                A.center = 1;
+                A.err = err;
+                if (qx) {
+                    A.Qb = reinterpret_cast<const float4*>(qb);
+                    A.l = l;
+                    A.qsum = qsum;
+                    A.Afull = afull;
+                }
+                SchurArgs S{};
+                S.l = l;
+                S.G = t;
+                S.Z = Z;
+                S.ldc = chunk * r;
+                S.C2 = C + (size_t)t * chunk * r;
+                S.D = D;
+                S.Dset = Dset;
+                S.W = W;
+                S.pat_bad = pat_bad;
+                S.sinv = sinv_c;
+                S.sing = sing_c;
+                S.varx = varx_c;
+                S.aobs = aobs_c;
+                S.zA = zA_c;
+                S.zD = zD_c;
+                S.rr = r;
+                S.Afull_lean = afull;
+                const int per_sm = (int)(227 * 1024 / (smem + 2048));
+                for (int c0 = 0; c0 < mb; c0 += chunk) {
+                    const int mc = mb - c0 < chunk ? mb - c0 : chunk;
+                    A.X = xr + (size_t)c0 * r * n;
+                    A.mb = mc;
+                    S.mb = mc;
+                    const int groups = (mc + spb - 1) / spb, most = sms * (per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm));
+                    NA_CU(oa_launch_snp_lean(r, spb, A, groups < most ? groups : most, threads, smem, st));
+                    NA_CU(oa_launch_gemm_tcp(xhi, xlo, mc * r, bhi, blo, cols, n_pad, xscale, cscale, C, chunk * r, err,
+                                             st));
+                    NA_CU(oa_launch_schur(r, S, st));
+                    EpiArgs E = epi(mc, c0);
+                    E.sinv = sinv_c;
+                    E.varx = varx_c;
+                    E.sing = sing_c;
+                    E.aobs = aobs_c;
+                    E.zA = zA_c;
+                    E.zD = zD_c;
+                    NA_CU(oa_launch_test_stats(r, E, C, chunk * r, 0, t, st));
+                }
+                return finish();
+            }
+        }
+    }
     k_set_rows<<<nsets, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, set_rows);
     k_set_gram<<<nsets, OA_NTHREADS, 0, st>>>(Q64, n, l, set_kind, set_off, set_rows, W, zQ, set_slot, pat_bad);
     if (nrows > 0)
@@ -427,47 +682,14 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
     NA_CU(oa_launch_snp_stats(r, LP, A, groups < sms ? groups : sms, stats_smem_bytes(r, LP, n, spb, nbuf, spp), st));
 
     // XR'Y~ with the fused statistics, dense outputs only
-    EpiArgs E{};
-    E.n = n;
-    E.l = l;
-    E.r = r;
-    E.p = l + r;
-    E.mb = mb;
-    E.G = t;
-    E.pat = pat;
-    E.zset = zset;
-    E.tperm = tperm;
-    E.rss0 = rss0;
-    E.a_r2 = a_r2;
-    E.inv_ncorr = inv_ncorr;
-    E.vf = vf;
-    E.b0 = b0;
+    EpiArgs E = epi(mb, 0);
     E.sinv = sinv;
     E.varx = varx;
     E.sing = sing;
     E.aobs = aobs;
     E.zA = zA;
     E.zD = zD;
-    E.zQ = zQ;
-    E.W = W;
-    E.store_all = 1;
-    E.rec = nullptr;
-    E.rec_count = counters;
-    E.rec_valid = nullptr;
-    E.cap = 0;
-    E.n_singular = counters + 1;
-    E.d_beta = beta;
-    E.d_se = se;
-    E.d_t = tstat;
-    E.d_r2 = r2;
     E.d_sig = dsig;
-    E.t = t;
-    E.snp_base = 0;
-    E.dense_ld = mb;
     NA_CU(oa_launch_gemm_simt(r, xr, (size_t)n, mb * r, Yt, (size_t)n_pad, t, n, mean, has_nan, E, st));
-    unsigned long long hc[4];
-    NA_CU(cudaMemcpyAsync(hc, counters, sizeof hc, cudaMemcpyDeviceToHost, st));
-    NA_CU(cudaStreamSynchronize(st));
-    if (hc[3]) return fail(OA_ERR_CUDA, "a device staging wait timed out");
-    return OA_OK;
+    return finish();
 }
