@@ -18,10 +18,13 @@ constexpr int EPI_WARPS_TC = 8;   // epilogue warps per tensor-core GEMM CTA (ea
 namespace oa {
 
 // Per-trait constants of the epilogue, gathered once per tile.
-struct TraitP {
+struct alignas(16) TraitP {
+    float rss0f, cw;   // rss0 in FP32, inv_ncorr * vf: what epi_screen reads, with g, in one load
+    int g, zs;
     double rss0;
-    float a_r2, inv_ncorr, vf;
-    int g, zs, orig;
+    float a_r2, inv_ncorr;
+    float vf;
+    int orig;
 };
 
 // One stored row (a (trait, SNP) test with at least one stored SNP term),
@@ -77,6 +80,7 @@ struct EpiArgs {
     // thresholds
     float min_r2, min_t;
     int store_all;
+    float screen_t2;                 // > 0: tests are screened in FP32 first (epi_screen); slightly below min_t^2
     // outputs
     void* rec;                       // RecOf<R> records
     unsigned long long* rec_count;   // record slots handed out (written rows and unused slots of reserved blocks)
@@ -94,6 +98,13 @@ struct EpiArgs {
     int snp_base;            // index of the block's first SNP within the API call
     long long dense_ld;      // SNPs per trait row of the dense outputs
 };
+
+// Thresholds from which most warps of 32 null tests store nothing (P < 0.01: 0.72 of them), so that
+// screening them in FP32 first saves more than it costs.
+constexpr float SCREEN_MIN_T = 2.6f;
+inline float screen_threshold(float min_t, int store_all) {
+    return !store_all && min_t >= SCREEN_MIN_T ? 0.998f * min_t * min_t : 0.f;
+}
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     // splitmix64 finaliser (Steele, Lea, Flood 2014)

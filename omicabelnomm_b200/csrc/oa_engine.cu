@@ -1193,6 +1193,7 @@ EpiArgs epi_args(oa_engine* e, int mbc, int snp_base) {
     E.min_r2 = e->cfg.min_r2_store;
     E.min_t = e->cfg.min_t_store;
     E.store_all = e->cfg.store_all;
+    E.screen_t2 = screen_threshold(E.min_t, E.store_all);
     E.rec = e->rec.p;
     E.rec_count = e->counters.p;
     E.rec_valid = e->counters.p + 4;

@@ -32,7 +32,39 @@ __device__ __forceinline__ TraitP load_trait(const EpiArgs& E, int j) {
     p.g = E.pat[j];
     p.zs = E.zset[j];
     p.orig = E.tperm[j];
+    p.rss0f = (float)p.rss0;
+    p.cw = p.inv_ncorr * p.vf;
     return p;
+}
+
+// True if a regular test surely stores no row: every |t| is below the store threshold by more than the
+// rounding of this FP32 evaluation.  z' beta and beta sum terms S_ab z_b whose sizes m bound their error:
+// beta is taken 1e-5 m larger, and the residual sum of squares must keep a tenth of its start and
+// 1/300 of the terms it is formed from (its relative error is then below 1e-4, against the 2e-3 the
+// threshold is lowered by).  Anything else, NaN included, is left to the full evaluation.
+template <int R>
+__device__ __forceinline__ bool epi_screen(const EpiArgs& E, const float* z, const TraitP& tp, const float* Sf,
+                                           const float* vx) {
+    float h[R], zz = 0.f, q = 0.f;
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+        float b = 0.f, m = 0.f;
+#pragma unroll
+        for (int c = 0; c < R; ++c) {
+            const float p = Sf[a * R + c] * z[c];
+            b += p;
+            m += fabsf(p);
+        }
+        zz = fmaf(z[a], b, zz);
+        q = fmaf(fabsf(z[a]), m, q);
+        h[a] = fmaf(1e-5f, m, fabsf(b));
+    }
+    const float rss = tp.rss0f - zz;
+    bool none = rss > 0.1f * tp.rss0f && q < 300.f * rss;
+    const float lim = E.screen_t2 * (rss * tp.cw);
+#pragma unroll
+    for (int a = 0; a < R; ++a) none = none && h[a] * h[a] < lim * vx[a];
+    return none;
 }
 
 // Status bits of an evaluated (non-singular) test (OA_TEST_*, include/omicabel_b200.h):

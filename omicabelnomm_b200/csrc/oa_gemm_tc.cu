@@ -220,13 +220,15 @@ __device__ __forceinline__ void tmem_wait8(uint32_t (&v)[8]) {
 // TMEM at taddr (8 columns per tcgen05.ld, the next 8 loading while these are
 // evaluated when PREFETCH), trait constants from tps.  FAST: no quirk terms,
 // no dense outputs and no zero sets among the tile's traits (epi_decide).
-template <int R, int BN, bool FAST, bool PREFETCH>
+// SCREEN: columns in which no lane can store a row are passed over (epi_screen).
+template <int R, int BN, bool FAST, bool PREFETCH, bool SCREEN = false>
 __device__ __forceinline__ void epi_columns(const EpiArgs& E, uint32_t taddr, int n0, int t, int lane, int i,
                                             bool lead, const float* vx, const TraitP* tps, int cb, int ce,
                                             Emitter& em) {
     int cg = -1;            // pattern whose Schur inverse is cached
     bool csing = true;
     double S[R * R];
+    float Sf[R * R];        // the same in FP32, for the screening
     if (!(cb < ce && n0 + cb < t)) return;
     uint32_t v[EPI_COLS], vn[EPI_COLS];
     if constexpr (PREFETCH) {
@@ -256,7 +258,12 @@ __device__ __forceinline__ void epi_columns(const EpiArgs& E, uint32_t taddr, in
             if (tp.g != cg) {    // traits are sorted by pattern: reloads are rare
                 cg = tp.g;
                 csing = lead ? !load_schur<R>(E, cg, i, S) : true;
+                if constexpr (SCREEN)
+#pragma unroll
+                    for (int a = 0; a < R * R; ++a) Sf[a] = csing ? 0.f : (float)S[a];
             }
+            if constexpr (SCREEN)   // no lane can store a row: the usual case at high thresholds
+                if (!__any_sync(0xffffffffu, lead && (csing || !epi_screen<R>(E, z, tp, Sf, vx)))) continue;
             EpiTest<R> o;
             bool st = false;
             if (lead) {
@@ -279,22 +286,38 @@ __device__ __forceinline__ void epi_columns(const EpiArgs& E, uint32_t taddr, in
     }
 }
 
+// Tiles with quirk terms, dense outputs or zero sets, out of line: their registers stay out of the usual
+// case's.
+template <int R, int BN, bool PREFETCH>
+__device__ __noinline__ void epi_columns_rare(const EpiArgs& E, uint32_t taddr, int n0, int t, int lane, int i,
+                                              bool lead, const float* vx, const TraitP* tps, int cb, int ce,
+                                              Emitter& em) {
+    epi_columns<R, BN, false, PREFETCH>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
+}
+
 // The statistics epilogue of one tile for one warp.  With one or two columns
 // per SNP a tile without quirk terms, dense outputs or zero sets takes the
-// FAST evaluation; the split-copy forms also prefetch the next 8 TMEM columns
-// (their register budget has room; the fused forms and r >= 4 do not).
+// FAST evaluation, at high thresholds behind the screening; the split-copy forms
+// also prefetch the next 8 TMEM columns (their register budget has room; the
+// fused forms and r >= 4 do not).
 template <int R, int BN, bool FUSED>
 __device__ __forceinline__ void epi_tile(bool fast, const EpiArgs& E, uint32_t taddr, int n0, int t, int lane,
                                          int i, bool lead, const float* vx, const TraitP* tps, int cb, int ce,
                                          Emitter& em) {
     constexpr bool PF = !FUSED && R <= 2;
     if constexpr (R <= 2) {
+        if (PF && fast && E.screen_t2 > 0.f) {
+            epi_columns<R, BN, true, PF, PF>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
+            return;
+        }
         if (fast) {
             epi_columns<R, BN, true, PF>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
             return;
         }
+        epi_columns_rare<R, BN, PF>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
+    } else {
+        epi_columns<R, BN, false, PF>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
     }
-    epi_columns<R, BN, false, PF>(E, taddr, n0, t, lane, i, lead, vx, tps, cb, ce, em);
 }
 
 // Trait constants of a tile's columns for the statistics epilogue (each
@@ -618,6 +641,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
+// Arrival on the leader's barrier after the TMEM reads before it (ordered by tcgen05.fence and
+// tcgen05.wait::ld): nothing written to memory has to be visible to the leader, and a release at cluster
+// scope would wait for this warp's earlier stores in every K-block.
+__device__ __forceinline__ void mbar_arrive_drained(uint32_t bar_cluster) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+}
+
 template <int R, class SH>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 k_gemm_tc2(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
@@ -793,7 +823,7 @@ k_gemm_tc2(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUt
                                         lane, i, lead, vx, tps, cb, cb + BN / 2, em);
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_rank(&acc_empty[acc], 0));
+                if (lane == 0) mbar_arrive_drained(map_to_rank(&acc_empty[acc], 0));
             }
             if (++acc == 2) {
                 acc = 0;
@@ -1830,9 +1860,12 @@ cudaError_t oa_launch_gemm_tcp(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xl
 
 template <int R>
 static cudaError_t go_ts(const EpiArgs& E, const float* z, int ldz, int j0, int nt, cudaStream_t st) {
-    const long long items = (long long)((E.mb + TS_THREADS - 1) / TS_THREADS) * ((nt + TS_TRAITS - 1) / TS_TRAITS);
-    const int grid = (int)std::min<long long>(items, (long long)TS_CTAS_PER_SM * tc::sm_count());
-    k_test_stats<R><<<grid, TS_THREADS, 0, st>>>(E, z, ldz, j0, nt);
+    // traits per item: 64, fewer (at least TS_COLS) while that leaves the chip with under two items per CTA
+    const long long sblocks = (E.mb + TS_THREADS - 1) / TS_THREADS, ctas = (long long)TS_CTAS_PER_SM * tc::sm_count();
+    int seg = TS_TRAITS;
+    while (seg > TS_COLS && sblocks * ((nt + seg - 1) / seg) < 2 * ctas) seg /= 2;
+    const int grid = (int)std::min<long long>(sblocks * ((nt + seg - 1) / seg), ctas);
+    k_test_stats<R><<<grid, TS_THREADS, 0, st>>>(E, z, ldz, j0, nt, seg);
     return cudaGetLastError();
 }
 

@@ -458,7 +458,7 @@ k_gemm_tcp2(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CU
                 drain_kblock<SH::GPW>(tlane + (uint32_t)(acc * BN), h, nc, sum);
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_rank(&acc_empty[acc], 0));
+                if (lane == 0) mbar_arrive_drained(map_to_rank(&acc_empty[acc], 0));
                 if (++acc == ACCS) {
                     acc = 0;
                     aph ^= 1u;
