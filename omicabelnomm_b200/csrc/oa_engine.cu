@@ -464,37 +464,67 @@ struct ModelW {
 // SNP i's columns go to out_r columns of `out`: the model's columns first,
 // zero padding after them (engines whose kernels take 4 or 8 columns per SNP
 // for r = 3, 5, 6, 7).
-static __global__ void k_column_model(const float* __restrict__ in, int n, int in_cols, ModelW W, int combine,
-                                      const float* __restrict__ inter, int n_inter, int keep, int out_r,
-                                      float* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Output columns of ldo floats, rows [n, ldo) zero.  A thread takes MODEL_ROWS rows, so that as many loads
+// of a file column are in flight (with one row each the kernel took 3.5 ms for the 2.5 GB of 50,665 SNPs at
+// n = 12,545 with one interaction, a third of HBM's rate).
+constexpr int MODEL_ROWS = 8;
+static __global__ void __launch_bounds__(256)
+k_column_model(const float* __restrict__ in, int n, int in_cols, ModelW W, int combine,
+               const float* __restrict__ inter, int n_inter, int keep, int out_r, size_t ldo,
+               float* __restrict__ out) {
+    const int k0 = blockIdx.x * 256 * MODEL_ROWS + threadIdx.x;
     const int i = blockIdx.y;
-    if (k >= n) return;
-    const float* src = in + (size_t)i * in_cols * n + k;
-    float* dst = out + (size_t)i * out_r * n + k;
+    const float* src = in + (size_t)i * in_cols * n;
+    float* dst = out + (size_t)i * out_r * ldo;
+    auto load = [&](const float* col, float (&x)[MODEL_ROWS]) {
+#pragma unroll
+        for (int u = 0; u < MODEL_ROWS; ++u) x[u] = k0 + 256 * u < n ? __ldg(col + k0 + 256 * u) : 0.f;
+    };
+    auto store = [&](int c, const float (&x)[MODEL_ROWS]) {
+#pragma unroll
+        for (int u = 0; u < MODEL_ROWS; ++u)
+            if ((size_t)(k0 + 256 * u) < ldo) dst[(size_t)c * ldo + k0 + 256 * u] = x[u];
+    };
     int written;
     if (combine) {   // a zero factor drops its column (the reference does not read it)
-        float acc = 0.f;
+        float acc[MODEL_ROWS], x[MODEL_ROWS];
+#pragma unroll
+        for (int u = 0; u < MODEL_ROWS; ++u) acc[u] = 0.f;
         bool any = false;
         for (int c = 0; c < in_cols; ++c) {
             if (W.w[c] == 0.f) continue;
-            const float x = src[(size_t)c * n];
-            acc = any ? fmaf(W.w[c], x, acc) : W.w[c] * x;
+            load(src + (size_t)c * n, x);
+#pragma unroll
+            for (int u = 0; u < MODEL_ROWS; ++u) acc[u] = any ? fmaf(W.w[c], x[u], acc[u]) : W.w[c] * x[u];
             any = true;
         }
         if (n_inter == 0) {
-            dst[0] = acc;
+            store(0, acc);
             written = 1;
         } else {   // [I_1 x, ..., I_k x (, x)] (src/AIOwrapper.cpp:808-840)
-            for (int h = 0; h < n_inter; ++h) dst[(size_t)h * n] = inter[(size_t)h * n + k] * acc;
-            if (keep) dst[(size_t)n_inter * n] = acc;
+            for (int h = 0; h < n_inter; ++h) {
+                load(inter + (size_t)h * n, x);
+#pragma unroll
+                for (int u = 0; u < MODEL_ROWS; ++u) x[u] = k0 + 256 * u < n ? x[u] * acc[u] : 0.f;
+                store(h, x);
+            }
+            if (keep) store(n_inter, acc);
             written = n_inter + keep;
         }
     } else {
-        for (int c = 0; c < in_cols; ++c) dst[(size_t)c * n] = W.w[c] * src[(size_t)c * n];
+        float x[MODEL_ROWS];
+        for (int c = 0; c < in_cols; ++c) {
+            load(src + (size_t)c * n, x);
+#pragma unroll
+            for (int u = 0; u < MODEL_ROWS; ++u) x[u] = k0 + 256 * u < n ? W.w[c] * x[u] : 0.f;
+            store(c, x);
+        }
         written = in_cols;
     }
-    for (int c = written; c < out_r; ++c) dst[(size_t)c * n] = 0.f;
+    float zero[MODEL_ROWS];
+#pragma unroll
+    for (int u = 0; u < MODEL_ROWS; ++u) zero[u] = 0.f;
+    for (int c = written; c < out_r; ++c) store(c, zero);
 }
 
 // The reference's r >= 2 downdate is reproduced (quirk mode; with r = 1 it
@@ -511,6 +541,10 @@ bool padded(const oa_engine* e) { return e->ru != e->r; }
 
 // A chunk passes through k_column_model (a dosage model, interactions or zero padding).
 bool column_pass(const oa_engine* e) { return e->in_cols > 0 || padded(e); }
+
+// Floats per column of its output: a multiple of 4 with a zero tail, so that the statistics kernel copies
+// aligned columns whatever n (the row-gather kernel takes columns of n).
+size_t model_ld(const oa_engine* e) { return e->use_pre ? ((size_t)e->n + 3) & ~(size_t)3 : (size_t)e->n; }
 
 // With the pre-GEMM statistics path nothing after the column statistics reads
 // the FP32 chunk (the GEMMs read its split), so a row subset is gathered by
@@ -678,7 +712,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->tcounts.ensure((size_t)t * 2));
     OA_CHECK(e->thash.ensure((size_t)t * 4));
     TraitStatsOut tso{e->tsums.p, e->tcounts.p, e->thash.p};
-    k_trait_stats<<<t, OA_NTHREADS, 0, e->st>>>(Y, (size_t)n, n, l, e->Q64.p, tso);
+    launch_trait_stats(t, Y, (size_t)n, n, l, e->Q64.p, tso, e->st);
     ++e->launches;
     OA_CU(cudaGetLastError());
     std::vector<int> counts((size_t)t * 2);
@@ -789,7 +823,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     h2d.add(e->set_blk_off.p, blk_off);
     h2d.add(e->set_item_off.p, e->h_set_item_off);
     OA_CHECK(flush_h2d(e, h2d));
-    k_set_rows<<<e->nsets, OA_NTHREADS, 0, e->st>>>(Y, (size_t)n, n, e->set_rep.p, e->set_kind.p, e->set_off.p,
+    k_set_rows<<<e->nsets, SET_THREADS, 0, e->st>>>(Y, (size_t)n, n, e->set_rep.p, e->set_kind.p, e->set_off.p,
                                                    e->set_rows.p);
     k_set_gram<<<e->nsets, OA_NTHREADS, 0, e->st>>>(e->Q64.p, n, l, e->set_kind.p, e->set_off.p, e->set_rows.p,
                                                    e->W.p, e->zQ.p, e->set_slot.p, e->pat_bad.p);
@@ -825,7 +859,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->inv_ncorr.ensure(t));
     OA_CHECK(e->vf.ensure(t));
     const bool mixed = e->cfg.precision == OA_MIXED_BF16X3;
-    k_trait_resid<<<t, OA_NTHREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
+    k_trait_resid<<<t, TRAIT_THREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
                                                e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, e->Yt.p, e->Yhi.p,
                                                e->Ylo.p, e->rss0.p, e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p,
                                                e->inv_ncorr.p, e->vf.p, mixed ? nullptr : e->cscale.p);
@@ -1069,6 +1103,7 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     LeanArgs A{};
     A.X = X;
     A.ldx = ldx;
+    A.padded = X == e->Xmodel.p;
     A.xrows = xrows;
     A.n = e->n;
     A.n_pad = e->n_pad;
@@ -1402,8 +1437,10 @@ oa_status enqueue_block(oa_engine* e, const float* xr, int mb, bool host_input, 
             ModelW W;
             const bool model = e->in_cols > 0;   // else the caller's ru columns as they are
             for (int c = 0; c < OA_MODEL_MAX_COLS; ++c) W.w[c] = model ? e->model_w[c] : 1.f;
-            k_column_model<<<dim3((unsigned)((e->n + 255) / 256), (unsigned)mbc), 256, 0, e->st>>>(
-                X, e->n, IC, W, model ? e->model_combine : 0, e->inter.p, e->n_inter, e->inter_keep, R,
+            ldx = model_ld(e);
+            constexpr unsigned rows = 256 * MODEL_ROWS;
+            k_column_model<<<dim3((unsigned)((ldx + rows - 1) / rows), (unsigned)mbc), 256, 0, e->st>>>(
+                X, e->n, IC, W, model ? e->model_combine : 0, e->inter.p, e->n_inter, e->inter_keep, R, ldx,
                 e->Xmodel.p);
             ++e->launches;
             OA_CU(cudaGetLastError());
@@ -1584,7 +1621,7 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         }
         if (!lean_gathers(e)) OA_CHECK(e->Xstage[0].ensure((size_t)e->chunk * e->r * e->n));
     }
-    if (column_pass(e)) OA_CHECK(e->Xmodel.ensure((size_t)e->chunk * e->r * e->n));
+    if (column_pass(e)) OA_CHECK(e->Xmodel.ensure((size_t)e->chunk * e->r * model_ld(e)));
     if (host_input) {
         if (!e->cp) OA_CU(cudaStreamCreateWithFlags(&e->cp, cudaStreamNonBlocking));
         for (int b = 0; b < 2; ++b) {

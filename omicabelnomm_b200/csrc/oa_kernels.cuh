@@ -26,21 +26,32 @@ struct TraitStatsOut {
     unsigned long long* hashes; // [t][4]: missing h1 h2, zero h1 h2
 };
 
-static __global__ void __launch_bounds__(OA_NTHREADS)
+// One CTA per trait.  A trait's rows are few passes of a wide CTA (512 threads: with 256 the 18 passes at
+// n = 4,713 were 18 dependent memory latencies, 66 us); LC: covariates held in registers (l <= LC).
+constexpr int TRAIT_THREADS = 512;
+constexpr int TRAIT_WARPS = TRAIT_THREADS / 32;
+
+template <int LC>
+static __global__ void __launch_bounds__(TRAIT_THREADS)
 k_trait_stats(const float* __restrict__ Y, size_t ldy, int n, int l, const double* __restrict__ Q64,
               TraitStatsOut out) {
-    __shared__ double red[8 * (2 + OA_MAX_L)];
-    __shared__ unsigned long long hred[8 * 4];
-    __shared__ int cred[8 * 2];
+    constexpr int NV = 2 + LC;
+    __shared__ double red[TRAIT_WARPS * NV];
+    __shared__ unsigned long long hred[TRAIT_WARPS * 4];
+    __shared__ int cred[TRAIT_WARPS * 2];
     const int j = blockIdx.x;
     const float* y = Y + (size_t)j * ldy;
-    double v[2 + OA_MAX_L];
+    double v[NV];
 #pragma unroll
-    for (int q = 0; q < 2 + OA_MAX_L; ++q) v[q] = 0.0;
+    for (int q = 0; q < NV; ++q) v[q] = 0.0;
     int miss = 0, zc = 0;
     unsigned long long h1 = 0, h2 = 0, z1 = 0, z2 = 0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+#pragma unroll 2
+    for (int k = threadIdx.x; k < n; k += TRAIT_THREADS) {
         const float x = y[k];
+        double qk[LC];
+#pragma unroll
+        for (int q = 0; q < LC; ++q) qk[q] = q < l ? Q64[(size_t)q * n + k] : 0.0;
         if (isnan(x)) {
             ++miss;
             h1 += mix64((unsigned long long)k);
@@ -54,13 +65,16 @@ k_trait_stats(const float* __restrict__ Y, size_t ldy, int n, int l, const doubl
                 z2 += mix64((unsigned long long)k ^ 0xa5a5a5a55a5a5a5aULL);
             }
 #pragma unroll
-            for (int q = 0; q < OA_MAX_L; ++q)
-                if (q < l) v[2 + q] += Q64[(size_t)q * n + k] * (double)x;
+            for (int q = 0; q < LC; ++q) v[2 + q] += qk[q] * (double)x;
         }
     }
-    block_sum<2 + OA_MAX_L>(v, red);
     // integer and hash sums (addition is order independent: deterministic)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        const double s = warp_sum(v[q]);
+        if (lane == 0) red[w * NV + q] = s;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         miss += __shfl_xor_sync(0xffffffffu, miss, o);
@@ -79,43 +93,49 @@ k_trait_stats(const float* __restrict__ Y, size_t ldy, int n, int l, const doubl
         hred[w * 4 + 3] = z2;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int cm = 0, cz = 0;
-        unsigned long long a = 0, b = 0, c = 0, d = 0;
-        for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) {
-            cm += cred[ww * 2];
-            cz += cred[ww * 2 + 1];
-            a += hred[ww * 4];
-            b += hred[ww * 4 + 1];
-            c += hred[ww * 4 + 2];
-            d += hred[ww * 4 + 3];
-        }
-        out.counts[j * 2] = cm;
-        out.counts[j * 2 + 1] = cz;
-        out.hashes[j * 4] = a;
-        out.hashes[j * 4 + 1] = b;
-        out.hashes[j * 4 + 2] = c;
-        out.hashes[j * 4 + 3] = d;
-        for (int q = 0; q < 2 + OA_MAX_L; ++q) out.sums[(size_t)j * (2 + OA_MAX_L) + q] = v[q];
+    const int q = threadIdx.x;
+    if (q < NV) {
+        double s = 0.0;
+        for (int ww = 0; ww < TRAIT_WARPS; ++ww) s += red[ww * NV + q];
+        out.sums[(size_t)j * (2 + OA_MAX_L) + q] = s;
+    } else if (q < 2 + OA_MAX_L) {
+        out.sums[(size_t)j * (2 + OA_MAX_L) + q] = 0.0;
+    } else if (q >= 32 && q < 34) {
+        int s = 0;
+        for (int ww = 0; ww < TRAIT_WARPS; ++ww) s += cred[ww * 2 + q - 32];
+        out.counts[j * 2 + q - 32] = s;
+    } else if (q >= 64 && q < 68) {
+        unsigned long long s = 0;
+        for (int ww = 0; ww < TRAIT_WARPS; ++ww) s += hred[ww * 4 + q - 64];
+        out.hashes[j * 4 + q - 64] = s;
     }
+}
+
+static inline void launch_trait_stats(int t, const float* Y, size_t ldy, int n, int l, const double* Q64,
+                                      TraitStatsOut out, cudaStream_t st) {
+    if (l <= 4)
+        k_trait_stats<4><<<t, TRAIT_THREADS, 0, st>>>(Y, ldy, n, l, Q64, out);
+    else if (l <= 8)
+        k_trait_stats<8><<<t, TRAIT_THREADS, 0, st>>>(Y, ldy, n, l, Q64, out);
+    else
+        k_trait_stats<16><<<t, TRAIT_THREADS, 0, st>>>(Y, ldy, n, l, Q64, out);
 }
 
 // Ordered list of the rows of each row set.  kind 0: NaN rows of the
 // representative trait (a missingness pattern); kind 1: observed rows
 // whose value is exactly 0 (a zero set).
-static __global__ void __launch_bounds__(OA_NTHREADS)
+constexpr int SET_THREADS = 1024;
+static __global__ void __launch_bounds__(SET_THREADS)
 k_set_rows(const float* __restrict__ Y, size_t ldy, int n, const int* __restrict__ set_rep,
            const int* __restrict__ set_kind, const int* __restrict__ set_off, int* __restrict__ rows) {
-    __shared__ int wcount[8];
-    __shared__ int wbase[8];
-    __shared__ int total;
+    __shared__ int wcount[2][32];   // double-buffered: one barrier per 1,024 rows
     const int s = blockIdx.x;
     const float* y = Y + (size_t)set_rep[s] * ldy;
     const int kind = set_kind[s];
     int* out = rows + set_off[s];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int base = 0;
-    for (int c0 = 0; c0 < n; c0 += blockDim.x) {
+    for (int c0 = 0, b = 0; c0 < n; c0 += SET_THREADS, b ^= 1) {
         const int k = c0 + threadIdx.x;
         bool pred = false;
         if (k < n) {
@@ -123,20 +143,12 @@ k_set_rows(const float* __restrict__ Y, size_t ldy, int n, const int* __restrict
             pred = kind == 0 ? isnan(x) : (x == 0.0f);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pred);
-        if (lane == 0) wcount[w] = __popc(m);
+        if (lane == 0) wcount[b][w] = __popc(m);
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int acc = 0;
-            for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) {
-                wbase[ww] = acc;
-                acc += wcount[ww];
-            }
-            total = acc;
-        }
-        __syncthreads();
-        if (pred) out[base + wbase[w] + __popc(m & ((1u << lane) - 1u))] = k;
-        base += total;
-        __syncthreads();
+        const int c = wcount[b][lane];
+        const int before = __reduce_add_sync(0xffffffffu, lane < w ? c : 0);
+        if (pred) out[base + before + __popc(m & ((1u << lane) - 1u))] = k;
+        base += __reduce_add_sync(0xffffffffu, c);
     }
 }
 
@@ -181,41 +193,79 @@ k_trait_masks(const float* __restrict__ Y, size_t ldy, int n, int nw, unsigned* 
 
 // Per row set: G = sum over the set's rows of q q' (FP64).  Patterns store
 // W = (I - G)^-1 (Q orthonormal over all rows, so Q_obs'Q_obs = I - G);
-// zero sets store G.  sing_out[s] = 1 if I - G is not positive definite.
+// zero sets store G.  pat_bad = 1 if I - G is not positive definite (a pivot
+// at or below 1e-12 of its diagonal).  Rows are staged GRAM_TILE at a time; a
+// thread sums one pair over every `groups`-th row of a tile, and one warp inverts
+// by Gauss-Jordan steps (whose pivots are the Cholesky factorisation's).  With
+// a thread per pair over all rows and a single-threaded inverse the kernel took 41
+// us for 11 sets of 400 rows and six covariates.
+constexpr int GRAM_TILE = 64;
 static __global__ void __launch_bounds__(OA_NTHREADS)
 k_set_gram(const double* __restrict__ Q64, int n, int l, const int* __restrict__ set_kind,
            const int* __restrict__ set_off, const int* __restrict__ rows, double* __restrict__ W,
            double* __restrict__ zQ, const int* __restrict__ set_slot, uint8_t* __restrict__ pat_bad) {
-    __shared__ double G[OA_MAX_L * OA_MAX_L];
+    __shared__ double tile[OA_MAX_L][GRAM_TILE + 1];
+    __shared__ double psum[OA_NTHREADS];
+    __shared__ double A[OA_MAX_L][OA_MAX_L + 1];
     const int s = blockIdx.x;
     const int r0 = set_off[s], r1 = set_off[s + 1];
-    const int npair = l * l;
-    for (int pq = threadIdx.x; pq < npair; pq += blockDim.x) {
-        const int a = pq / l, b = pq % l;
-        double acc = 0.0;
-        if (b <= a)
-            for (int k = r0; k < r1; ++k) {
-                const int row = rows[k];
-                acc += Q64[(size_t)a * n + row] * Q64[(size_t)b * n + row];
-            }
-        G[pq] = acc;
+    const int npair = l * (l + 1) / 2, groups = OA_NTHREADS / npair;   // npair <= 136
+    const int pr = threadIdx.x % npair, grp = threadIdx.x / npair;
+    int a = 0;   // pair pr = (a, b), b <= a
+    while ((a + 1) * (a + 2) / 2 <= pr) ++a;
+    const int b = pr - a * (a + 1) / 2;
+    double acc = 0.0;
+    for (int k0 = r0; k0 < r1; k0 += GRAM_TILE) {
+        const int nr = min(GRAM_TILE, r1 - k0);
+        for (int q = threadIdx.x; q < GRAM_TILE * l; q += OA_NTHREADS) {
+            const int k = q % GRAM_TILE, c = q / GRAM_TILE;
+            tile[c][k] = k < nr ? Q64[(size_t)c * n + rows[k0 + k]] : 0.0;
+        }
+        __syncthreads();
+        if (grp < groups)
+            for (int k = grp; k < nr; k += groups) acc += tile[a][k] * tile[b][k];
+        __syncthreads();
+    }
+    psum[threadIdx.x] = acc;
+    __syncthreads();
+    if ((int)threadIdx.x < npair) {
+        double g = 0.0;
+        for (int q = 0; q < groups; ++q) g += psum[q * npair + pr];
+        A[a][b] = A[b][a] = g;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int a = 0; a < l; ++a)
-            for (int b = a + 1; b < l; ++b) G[a * l + b] = G[b * l + a];
-        const int slot = set_slot[s];
-        if (set_kind[s] == 1) {
-            for (int q = 0; q < l * l; ++q) zQ[(size_t)slot * l * l + q] = G[q];
-        } else {
-            double A[OA_MAX_L * OA_MAX_L];
-            for (int a = 0; a < l; ++a)
-                for (int b = 0; b < l; ++b) A[a * l + b] = (a == b ? 1.0 : 0.0) - G[a * l + b];
-            const bool ok = spd_inverse<OA_MAX_L>(A, l, 1e-12);
-            pat_bad[slot] = ok ? 0 : 1;
-            for (int q = 0; q < l * l; ++q) W[(size_t)slot * l * l + q] = ok ? A[q] : 0.0;
-        }
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, slot = set_slot[s];
+    if (set_kind[s] == 1) {
+        for (int q = lane; q < l * l; q += 32) zQ[(size_t)slot * l * l + q] = A[q / l][q % l];
+        return;
     }
+    for (int q = lane; q < l * l; q += 32) A[q / l][q % l] = (q / l == q % l ? 1.0 : 0.0) - A[q / l][q % l];
+    __syncwarp();
+    bool ok = true;
+    // lane c < l keeps the diagonal it started from (the pivots' reference)
+    const double diag = lane < l ? A[lane][lane] : 1.0;
+    for (int j = 0; j < l && ok; ++j) {
+        const double piv = A[j][j], d0 = __shfl_sync(0xffffffffu, diag, j);
+        ok = piv > 1e-12 * fmax(fabs(d0), 1e-300);   // the same value on every lane
+        if (!ok) break;
+        const double inv = 1.0 / piv;
+        for (int q = lane; q < l * l; q += 32) {     // everything off row and column j
+            const int i = q / l, c = q % l;
+            if (i != j && c != j) A[i][c] -= A[i][j] * inv * A[j][c];
+        }
+        __syncwarp();
+        if (lane < l && lane != j) {
+            A[lane][j] *= -inv;                      // column j: -a_ij / piv
+            A[j][lane] *= inv;                       // row j: a_jc / piv
+        }
+        if (lane == j) A[j][j] = inv;
+        __syncwarp();
+    }
+    if (lane == 0) pat_bad[slot] = ok ? 0 : 1;
+    // symmetric by construction up to rounding: the mean of the two halves
+    for (int q = lane; q < l * l; q += 32)
+        W[(size_t)slot * l * l + q] = ok ? 0.5 * (A[q / l][q % l] + A[q % l][q / l]) : 0.0;
 }
 
 // y~ = y - Q b0 on observed rows (0 on missing rows), b0 = W Q'y.
@@ -226,7 +276,7 @@ k_set_gram(const double* __restrict__ Q64, int n, int l, const int* __restrict__
 // With yscale (the FP32-accurate tensor-core form) the split is FP16 of the
 // scaled residuals, written once RSS0 is known, and yscale[jj] = 1 / scale;
 // Yt may be null there (the residuals are then formed twice).
-static __global__ void __launch_bounds__(OA_NTHREADS)
+static __global__ void __launch_bounds__(TRAIT_THREADS)
 k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, int p,
               const double* __restrict__ Q64, const double* __restrict__ sums,
               const int* __restrict__ counts, const int* __restrict__ pat,
@@ -237,7 +287,7 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
               float* __restrict__ vf, float* __restrict__ yscale = nullptr) {
     __shared__ float half_s;
     __shared__ double b0[OA_MAX_L];
-    __shared__ double red[8];
+    __shared__ double red[TRAIT_WARPS];
     const int jj = blockIdx.x;
     const int j = tperm[jj];
     const double* sj = sums + (size_t)j * (2 + OA_MAX_L);

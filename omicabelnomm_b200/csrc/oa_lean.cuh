@@ -23,6 +23,7 @@ namespace oa {
 struct LeanArgs {
     const float* X;       // SNP block, column c at X + c*ldx
     size_t ldx;
+    int padded;           // columns are 16-byte aligned and zero from row n to the next multiple of 4
     const int* xrows;     // row k of a column is X[c*ldx + xrows[k]] (a row subset), or null: X[c*ldx + k]
     int n, n_pad, mb;
     int nsets;
@@ -228,14 +229,15 @@ k_snp_lean(LeanArgs A) {
     const int ngroups = (A.mb + SPB - 1) / SPB;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // some column starts or ends off a 16-byte boundary: copies write past column ends
-    const bool ragged = !GATHER && (((n | (int)(A.ldx & 3)) & 3) != 0 || (reinterpret_cast<uintptr_t>(A.X) & 15) != 0);
+    const bool ragged = !GATHER && !A.padded &&
+                        (((n | (int)(A.ldx & 3)) & 3) != 0 || (reinterpret_cast<uintptr_t>(A.X) & 15) != 0);
 
     // Offset (floats) of column c of the block below its first element, and whether the 16-byte
     // boundaries around it may lie outside the block.
     auto col_off = [&](int c) { return (int)((reinterpret_cast<uintptr_t>(A.X + (size_t)c * A.ldx) >> 2) & 3); };
     auto col_edge = [&](int c) {
         const int o = col_off(c);
-        return (c == 0 && o != 0) || (c == A.mb * R - 1 && ((o + n) & 3) != 0);
+        return !A.padded && ((c == 0 && o != 0) || (c == A.mb * R - 1 && ((o + n) & 3) != 0));
     };
     // thread 0: bulk copies of a group's columns
     auto issue = [&](int g) {

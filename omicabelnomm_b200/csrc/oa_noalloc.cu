@@ -425,7 +425,7 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
     Q64 = Q1;
     // traits: missing counts, sums, Q'y; one row set per trait
     TraitStatsOut tso{tsums, tcounts, thash};
-    k_trait_stats<<<t, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, l, Q64, tso);
+    launch_trait_stats(t, y, (size_t)n, n, l, Q64, tso, st);
     k_na_sets<<<1, 1024, 0, st>>>(tcounts, t, xl, n, pat, zset, tperm, set_off, set_rep, set_kind, set_slot, blk_off,
                                   pass_off, info);
     NA_CU(cudaGetLastError());
@@ -541,11 +541,11 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
                 qsum = tc.take<double>(l);
             }
             if (tc.used <= OA_NOALLOC_SCRATCH_BYTES) {
-                k_set_rows<<<nsets, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, rows);
+                k_set_rows<<<nsets, SET_THREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, rows);
                 k_set_gram<<<nsets, OA_NTHREADS, 0, st>>>(Q64, n, l, set_kind, set_off, rows, W, zQ, set_slot, pat_bad);
                 k_na_items<<<(nsets + 255) / 256, 256, 0, st>>>(set_off, blk_off, nsets, items);
                 k_item_rows<<<nsets, 1024, 0, st>>>(rows, set_off, blk_off, n_pad, item_rows);
-                k_trait_resid<<<t, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, n_pad, l, l + r, Q64, tsums, tcounts, pat, W,
+                k_trait_resid<<<t, TRAIT_THREADS, 0, st>>>(y, (size_t)n, n, n_pad, l, l + r, Q64, tsums, tcounts, pat, W,
                                                         tperm, nullptr, bhi, blo, rss0, sst, nobs, b0, a_r2, inv_ncorr,
                                                         vf, cscale);
                 const size_t ny = (size_t)t * n_pad, nb2 = (size_t)c2 * n_pad;
@@ -626,11 +626,11 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
             }
         }
     }
-    k_set_rows<<<nsets, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, set_rows);
+    k_set_rows<<<nsets, SET_THREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, set_rows);
     k_set_gram<<<nsets, OA_NTHREADS, 0, st>>>(Q64, n, l, set_kind, set_off, set_rows, W, zQ, set_slot, pat_bad);
     if (nrows > 0)
         k_set_qrows<<<(unsigned)(((long long)nrows * LP + 255) / 256), 256, 0, st>>>(set_rows, nrows, Qr, LP, qrows);
-    k_trait_resid<<<t, OA_NTHREADS, 0, st>>>(y, (size_t)n, n, n_pad, l, l + r, Q64, tsums, tcounts, pat, W, tperm,
+    k_trait_resid<<<t, TRAIT_THREADS, 0, st>>>(y, (size_t)n, n, n_pad, l, l + r, Q64, tsums, tcounts, pat, W, tperm,
                                             Yt, nullptr, nullptr, rss0, sst, nobs, b0, a_r2, inv_ncorr, vf);
     NA_CU(cudaGetLastError());
 

@@ -208,3 +208,39 @@ def test_noalloc_forms_match_oracle(case):
         check_plain(ds, 1, tuple(np.ascontiguousarray(a[:, pick]) for a in got))
     else:
         check_plain(ds, r, noalloc_dense(ds, r))
+
+
+@pytest.mark.parametrize("prec", [E.PLAIN, E.MIXED])
+@pytest.mark.parametrize("model", ["additive", "interaction", "three"])
+@pytest.mark.parametrize("n", [517, 518, 2051])
+def test_model_columns_give_the_direct_columns_bits(n, model, prec):
+    """Dosage models, interactions and zero-padded columns formed on the device (aligned columns with a zero
+    tail whatever n) against the same columns passed in."""
+    ds = synth.generate(synth.scaled(0, n=n, m=99, t=24, l=4, miss_mode="patterns", n_patterns=4, seed=395 + n))
+    rng = np.random.Generator(np.random.PCG64(n))
+    r = {"additive": 1, "interaction": 2, "three": 3}[model]
+    if model == "additive":
+        P = rng.random((99, 3, n)).astype(np.float32)
+        raw = P.reshape(297, n)
+        direct = np.float32(2.0) * P[:, 0] + P[:, 1]         # 2 x is exact: one rounding, as the fused product
+    elif model == "interaction":
+        raw = ds.XR
+        direct = np.stack([ds.XR * ds.XL[1], ds.XR], 1).reshape(198, n)
+    else:
+        raw = direct = ds.XR
+    out = []
+    for cols, formed in ((raw, True), (direct, False)):
+        m = cols.shape[0] // (r if model == "three" or not formed else cols.shape[0] // 99)
+        eng = E.Engine(n, 4, r, 24, m, precision=prec, store_all=True, min_t_store=1.6, min_r2_store=1e-6)
+        eng.set_covariates(ds.XL)
+        eng.set_traits(ds.Y)
+        if formed and model == "additive":
+            eng.set_column_model(3, [2.0, 1.0, 0.0])
+        elif formed and model == "interaction":
+            eng.set_interactions(ds.XL[1:2])
+        eng.enable_dense(True)
+        eng.run(np.ascontiguousarray(cols))
+        out.append(eng.dense(m))
+        eng.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
