@@ -1008,8 +1008,7 @@ oa_status stats_gather(oa_engine* e, const float* X, int mbc) {
 
 // Lean path: k_snp_lean (imputation, 16-bit split, X'X over all rows and over
 // each row set) -> pre-GEMM C2 = [Q | Q o m_1 | ...]'X -> k_schur.
-// SNPs per CTA group of k_snp_lean: requested, else as many (a power of two <= 8 / r) as
-// LEAN_GROUP_BYTES of shared memory hold
+// SNPs per CTA group of k_snp_lean: requested (a power of two <= 8 / r), else lean_auto_spb
 // With two or more columns per SNP and at most LEAN_QX_L covariates, k_snp_lean also sums the
 // all-rows covariate projection A = Q'X of every column (short FP32 partial sums, FP64 across
 // warps) for k_schur: the pre-GEMM's A (FP32 sums over all n rows; BF16 hi/lo products in the mixed
@@ -1018,14 +1017,10 @@ oa_status stats_gather(oa_engine* e, const float* X, int mbc) {
 // groups of at most LEAN_QX_NC columns.
 bool want_lean_qx(const oa_engine* e) { return e->ru >= 2 && e->l <= LEAN_QX_L && e->r <= LEAN_QX_NC; }
 
-// Threads per k_snp_lean CTA, from the column length alone (so that every tuning sums in the same
-// order and gives the same bits): 512 with one column per SNP where the column takes 64 KB or more
-// of shared memory (n >= 16,384: at most three CTAs fit on an SM, and the plan then keeps one SNP
-// per group), else 256 (more, smaller CTAs per SM with cheaper block barriers).
+// Threads per k_snp_lean CTA (OA_LEAN_THREADS asks for 256 or 512 where long columns run 512).
 int lean_threads(const oa_engine* e) {
-    const bool long_col = e->r == 1 && (size_t)e->n_pad * 4 >= (size_t)64 * 1024;
-    if (e->lean_threads_req) return long_col ? e->lean_threads_req : 256;
-    return long_col ? LEAN_MAX_THREADS : 256;
+    const int t = lean_threads_for(e->r, e->n_pad);
+    return t == LEAN_MAX_THREADS && e->lean_threads_req ? e->lean_threads_req : t;
 }
 
 int lean_group(const oa_engine* e) {
@@ -1036,9 +1031,7 @@ int lean_group(const oa_engine* e) {
         while (s * 2 <= e->lean_spb) s *= 2;
         return std::min(s, cap);
     }
-    int s = 1;
-    while (s * 2 <= cap && lean_smem_bytes(e->r, e->n_pad, s * 2, 0, want_lean_qx(e)) <= LEAN_GROUP_BYTES) s *= 2;
-    return s;
+    return std::min(cap, lean_auto_spb(e->r, e->n_pad, want_lean_qx(e), e->chunk, e->sm_count));
 }
 
 // Launch plan of k_snp_lean for the current trait block and tuning: SNPs per

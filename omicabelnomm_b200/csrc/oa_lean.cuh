@@ -55,8 +55,8 @@ struct LeanArgs {
     double* Afull;        // [mb*R][LEAN_QX_L]: A of column c, covariate q at Afull[c * LEAN_QX_L + q]
 };
 
-// Threads per CTA (the template's NT): 256; one column per group may also run 512 (launched where
-// the column fills so much shared memory that few CTAs fit on an SM).  Shared scratch is sized
+// Threads per CTA (the template's NT): 256; groups of one SNP may also run 512 (launched where
+// its columns fill so much shared memory that few CTAs fit on an SM).  Shared scratch is sized
 // for 512.
 constexpr int LEAN_MAX_THREADS = 512;
 constexpr int LEAN_MAX_WARPS = LEAN_MAX_THREADS / 32;
@@ -75,8 +75,32 @@ __host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int
            (size_t)(LEAN_MAX_WARPS + 1) * NQ * 8 + 64;
 }
 
-// Shared memory of a group that takes several SNPs by itself: at least four CTAs per SM.
-constexpr size_t LEAN_GROUP_BYTES = 50 * 1024;
+// Threads per CTA, from the columns' length alone (so that every tuning sums in the same order and gives the
+// same bits): 512 where a SNP's columns leave an SM at most three CTAs (one column: n >= 16,384) or, with
+// two or four, two; the plan then keeps one SNP per group.  Else 256: more, smaller CTAs per SM with
+// cheaper block barriers.  (Statistics stage with 256 / 512 threads, two columns: 20,000 SNPs at
+// n = 12,545 1.67 / 1.38 ms, n = 10,001 1.01 / 0.90, n = 9,500 0.97 / 0.98; 10,000 at n = 14,411 with 85 sets
+// of 1,441 rows 4.98 / 3.97.)
+inline int lean_threads_for(int R, int n_pad) {
+    const size_t col = (size_t)n_pad * 4;
+    const bool longc = R == 1 ? col >= 64 * 1024 : (R <= 4 && R * col >= 75 * 1024);
+    return longc ? LEAN_MAX_THREADS : 256;
+}
+
+// SNPs per group where the caller asks for none (a power of two): at most four columns, as far as they fit
+// the group's bytes and leave at least two groups per SM.  With one column per SNP two SNPs are worth going
+// down to three CTAs per SM, four to five (50,000 SNPs, statistics stage with 1 / 2 / 4 / 8 SNPs per group: n = 1,000 0.29 / 0.18 / 0.16 /
+// 0.19 ms, n = 2,000 0.33 / 0.21 / 0.20 / 0.26, n = 3,500 0.39 / 0.27 / 0.29 / 0.34, n = 7,000 0.65 / 0.62 / - / -, n = 10,000 1.37 / 1.46 / - / -);
+// with two, the covariate basis read once per group is worth two CTAs (20,000 SNPs, n = 6,000 1.27 / 1.23).
+inline int lean_auto_spb(int R, int n_pad, bool qx, int snps, int sms) {
+    int s = 1;
+    for (;;) {
+        const size_t bytes = (R > 1 ? 100 : (s == 1 ? 60 : 40)) * 1024;
+        if (s * 2 * R > 4 || lean_smem_bytes(R, n_pad, s * 2, 0, qx) > bytes || snps / (s * 2) < 2 * sms) break;
+        s *= 2;
+    }
+    return s;
+}
 
 // Rows per work item of the set pass: one block of a set where that gives the eight warps few items,
 // else up to four (each item ends in a shuffle reduction, which with 150 sets of 600 rows took more of

@@ -513,11 +513,10 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         if (fit < mb) fit = fit / 256 * 256;
         const int chunk = (int)(fit < mb ? fit : mb);
         // column-statistics kernel: SNPs per group, threads and shared memory as the engine plans them
-        const int threads = r == 1 && (size_t)n_pad * 4 >= (size_t)64 * 1024 ? LEAN_MAX_THREADS : 256;
-        int spb = 1;
-        if (threads == 256)
-            while (spb * 2 * r <= (qx ? LEAN_QX_NC : 8) && lean_smem_bytes(r, n_pad, spb * 2, 0, qx) <= LEAN_GROUP_BYTES)
-                spb *= 2;
+        const int threads = lean_threads_for(r, n_pad);
+        int sms = 148;
+        NA_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const int spb = threads == 256 ? lean_auto_spb(r, n_pad, qx, chunk, sms) : 1;
         const size_t smem = lean_smem_bytes(r, n_pad, spb, nblk > 0 ? nblk : 1, qx);
         if (chunk > 0 && smem <= 227 * 1024 - 1024) {
             float* mean_c = tc.take<float>((size_t)chunk * r);
@@ -554,8 +553,6 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
                 k_fill<<<(c2 + 255) / 256, 256, 0, st>>>(cscale + t, c2, 1.f / HALF_SCALE_Q);
                 if (qx) k_na_qblocks<<<l, 256, 0, st>>>(Qr, LP, n, n_pad, l, qb, qsum);
                 NA_CU(cudaGetLastError());
-                int sms = 148;
-                NA_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
                 int* err = reinterpret_cast<int*>(counters + 3);
                 LeanArgs A{};
                 A.ldx = (size_t)n;

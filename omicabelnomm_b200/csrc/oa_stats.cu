@@ -107,7 +107,12 @@ int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads) {
     }
     int v = 0;
     if (threads == LEAN_MAX_THREADS) {
-        v = (R == 1 && spb == 1 && !qx) ? lean_occ<1, 1, false, LEAN_MAX_THREADS>(smem) : 0;
+        switch (R * 100 + spb) {
+            case 101: v = qx ? 0 : lean_occ<1, 1, false, LEAN_MAX_THREADS>(smem); break;
+            case 201: v = qx ? lean_occ<2, 1, true, LEAN_MAX_THREADS>(smem) : lean_occ<2, 1, false, LEAN_MAX_THREADS>(smem); break;
+            case 401: v = qx ? lean_occ<4, 1, true, LEAN_MAX_THREADS>(smem) : lean_occ<4, 1, false, LEAN_MAX_THREADS>(smem); break;
+            default: v = 0;
+        }
     } else if (qx) {
         switch (R * 100 + spb) {
             case 201: v = lean_occ<2, 1, true>(smem); break;
@@ -137,9 +142,16 @@ int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads) {
 
 cudaError_t oa_launch_snp_lean(int R, int spb, const LeanArgs& A, int grid, int threads, size_t smem,
                                cudaStream_t st) {
-    if (threads == LEAN_MAX_THREADS)
-        return R == 1 && spb == 1 && !A.Afull ? go_lean<1, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st)
-                                              : cudaErrorInvalidValue;
+    if (threads == LEAN_MAX_THREADS) {
+        switch (R * 100 + spb) {
+            case 101: return A.Afull ? cudaErrorInvalidValue : go_lean<1, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
+            case 201: return A.Afull ? go_lean<2, 1, true, LEAN_MAX_THREADS>(A, grid, smem, st)
+                                     : go_lean<2, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
+            case 401: return A.Afull ? go_lean<4, 1, true, LEAN_MAX_THREADS>(A, grid, smem, st)
+                                     : go_lean<4, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
+            default: return cudaErrorInvalidValue;
+        }
+    }
     if (threads != 256) return cudaErrorInvalidValue;
     if (A.Afull) {
         switch (R * 100 + spb) {
