@@ -1572,6 +1572,34 @@ long long slots_needed(const oa_engine* e, long long mb, long long t, long long 
     return std::max<long long>(1 << 16, rows + slack);
 }
 
+// Rows up to this many come back in one piece.
+constexpr long long FEW_ROWS = 1 << 18;
+
+// Rec-sized slots that hold N rows of the final layout.
+size_t final_slots(const oa_engine* e, size_t N) { return (N * final_row_bytes(e->p) + sizeof(Rec) - 1) / sizeof(Rec); }
+
+// The NS handed-out slots' order by (trait, SNP) to perm2, unused slots last.
+template <int R>
+oa_status sort_rows(oa_engine* e, long long NS, int mb) {
+    OA_CHECK(e->keys.ensure(NS));
+    OA_CHECK(e->keys2.ensure(NS));
+    OA_CHECK(e->perm.ensure(NS));
+    OA_CHECK(e->perm2.ensure(NS));
+    // key bits: enough for t * mb with the all-ones invalid key above every valid one
+    int bits = 1;
+    while (bits < 64 && (1ull << bits) <= (unsigned long long)e->t * (unsigned long long)mb) ++bits;
+    k_rec_keys<<<(unsigned)((NS + 255) / 256), 256, 0, e->st>>>(reinterpret_cast<const RecOf<R>*>(e->rec.p), NS, mb,
+                                                                 bits, e->keys.p, e->perm.p);
+    ++e->launches;
+    size_t tmp = 0;
+    OA_CU(cub::DeviceRadixSort::SortPairs(nullptr, tmp, e->keys.p, e->keys2.p, e->perm.p, e->perm2.p, (int)NS, 0,
+                                          bits, e->st));
+    OA_CHECK(e->cub_tmp.ensure(tmp));
+    OA_CU(cub::DeviceRadixSort::SortPairs(e->cub_tmp.p, tmp, e->keys.p, e->keys2.p, e->perm.p, e->perm2.p, (int)NS, 0,
+                                          bits, e->st));
+    return OA_OK;
+}
+
 template <int R>
 oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_input, bool results_on_host,
                         oa_rows* out) {
@@ -1641,33 +1669,43 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
     // slots of the warps' reserved blocks sort last and are dropped
     const long long NS = (long long)cnt[0];   // slots handed out
     const long long N = (long long)cnt[4];    // rows written
-    // few rows: one copy of all fields (they are contiguous), converted by this thread; many: in pieces,
-    // each converted by all host threads while the next copies.  With the pieces' 7 copies each a block
-    // with 1,000 stored rows took 58 copies and 180 us of the stream
-    const bool few = N <= (1 << 18);
-    const int pieces = few ? 1 : RESULT_PIECES;
     const int l = e->l, p = e->p;
+    // few rows: formed on the device as the caller gets them and copied back at once (20 + 12 p bytes a row;
+    // the conversion of 96,000 rows with covariate terms took the host 1.3 ms of 3.5); many: 16 + 12 R bytes
+    // a row in pieces, each converted by all host threads while the next copies, so that the link carries
+    // the fewer bytes
+    const bool few = N <= FEW_ROWS;
+    if (few) {
+        OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, final_slots(e, (size_t)N), e->retired_pinned));
+        const FinalRows hf = final_rows(e->h_rec, N, p);
+        if (N > 0) {
+            OA_CHECK(sort_rows<R>(e, NS, mb));
+            OA_CHECK(e->rec2.ensure(final_slots(e, (size_t)N)));
+            k_rec_final<R><<<(unsigned)((N * p + 255) / 256), 256, 0, e->st>>>(
+                reinterpret_cast<const RecOf<R>*>(e->rec.p), e->perm2.p, N, l, e->ru, e->nobs.p,
+                e->cfg.disp_cov ? e->cov.p : nullptr, e->cfg.min_t_store, e->cfg.store_all != 0,
+                final_rows(e->rec2.p, N, p));
+            ++e->launches;
+            OA_CU(cudaGetLastError());
+            OA_CU(cudaMemcpyAsync(e->h_rec, e->rec2.p, final_row_bytes(p) * (size_t)N, cudaMemcpyDeviceToHost, e->st));
+            OA_CU(cudaStreamSynchronize(e->st));
+        }
+        out->trait = hf.trait;
+        out->snp = hf.snp;
+        out->r2 = hf.r2;
+        out->n_used = hf.n_used;
+        out->coef_mask = hf.mask;
+        out->coef_b = hf.b;
+        out->coef_se = hf.se;
+        out->coef_t = hf.t;
+        return OA_OK;
+    }
     // the packed fields of N rows (16 + 12 R bytes each) fit in N Rec-sized slots per rec_slots(R)
     OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, (size_t)N * rec_slots(R), e->retired_pinned));
     if (e->cfg.disp_cov) OA_CHECK(ensure_pinned(e->h_cov, e->h_cov_cap, (size_t)N * l * 3, e->retired_pinned));
-    if (N > 0) {
-        OA_CHECK(e->keys.ensure(NS));
-        OA_CHECK(e->keys2.ensure(NS));
-        OA_CHECK(e->perm.ensure(NS));
-        OA_CHECK(e->perm2.ensure(NS));
+    {
+        OA_CHECK(sort_rows<R>(e, NS, mb));
         OA_CHECK(e->rec2.ensure((size_t)N * rec_slots(R)));
-        // key bits: enough for t * mb with the all-ones invalid key above every valid one
-        int bits = 1;
-        while (bits < 64 && (1ull << bits) <= (unsigned long long)e->t * (unsigned long long)mb) ++bits;
-        k_rec_keys<<<(unsigned)((NS + 255) / 256), 256, 0, e->st>>>(reinterpret_cast<const RecOf<R>*>(e->rec.p), NS,
-                                                                     mb, bits, e->keys.p, e->perm.p);
-        ++e->launches;
-        size_t tmp = 0;
-        OA_CU(cub::DeviceRadixSort::SortPairs(nullptr, tmp, e->keys.p, e->keys2.p, e->perm.p, e->perm2.p, (int)NS, 0,
-                                              bits, e->st));
-        OA_CHECK(e->cub_tmp.ensure(tmp));
-        OA_CU(cub::DeviceRadixSort::SortPairs(e->cub_tmp.p, tmp, e->keys.p, e->keys2.p, e->perm.p, e->perm2.p, (int)NS,
-                                              0, bits, e->st));
         if (e->cfg.disp_cov) OA_CHECK(e->cov2.ensure((size_t)N * l * 3));
         const RowsSoA dsoa = rows_soa(e->rec2.p, N, R);   // the record buffer holds the packed fields
         k_rec_gather<R><<<(unsigned)((N + 255) / 256), 256, 0, e->st>>>(reinterpret_cast<const RecOf<R>*>(e->rec.p),
@@ -1680,13 +1718,9 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         OA_CU(cudaGetLastError());
         // the rows come back in pieces, each converted on the host while the next is in flight
         const RowsSoA hsoa = rows_soa(e->h_rec, N, R);
-        if (few) {
-            OA_CU(cudaMemcpyAsync(e->h_rec, e->rec2.p, rows_soa_bytes(N, R), cudaMemcpyDeviceToHost, e->st));
-            OA_CU(cudaEventRecord(e->ev_piece[0], e->st));
-        }
-        for (int k = 0; k < RESULT_PIECES && !few; ++k) {
+        for (int k = 0; k < RESULT_PIECES; ++k) {
             const long long q0 = N * k / RESULT_PIECES, q1 = N * (k + 1) / RESULT_PIECES, nq = q1 - q0;
-            if (nq > 0) {
+            {
                 auto d2h = [&](void* dst, const void* src, size_t bytes) {
                     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->st);
                 };
@@ -1744,15 +1778,15 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
             e->o_mask[q] = m;
         }
     };
-    const int nthr = !few ? (int)std::min<unsigned>(32u, std::max(1u, std::thread::hardware_concurrency())) : 1;
+    const int nthr = (int)std::min<unsigned>(32u, std::max(1u, std::thread::hardware_concurrency()));
     std::atomic<int> piece_err{0};
     auto convert_pieces = [&](int k0, int nk) {   // thread k0 of nk: its share of every piece, in piece order
-        for (int k = 0; k < pieces; ++k) {
-            if (N > 0 && cudaEventSynchronize(e->ev_piece[k]) != cudaSuccess) {
+        for (int k = 0; k < RESULT_PIECES; ++k) {
+            if (cudaEventSynchronize(e->ev_piece[k]) != cudaSuccess) {
                 piece_err = 1;
                 return;
             }
-            const long long q0 = N * k / pieces, q1 = N * (k + 1) / pieces;
+            const long long q0 = N * k / RESULT_PIECES, q1 = N * (k + 1) / RESULT_PIECES;
             convert(q0 + (q1 - q0) * k0 / nk, q0 + (q1 - q0) * (k0 + 1) / nk);
         }
     };
@@ -2398,13 +2432,16 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         OA_CHECK(e->keys2.ensure(cap));
         OA_CHECK(e->perm.ensure(cap));
         OA_CHECK(e->perm2.ensure(cap));
-        OA_CHECK(e->rec2.ensure(R * rec_slots(e->r)));
+        // rows in the layout they come back in: the final one up to FEW_ROWS, else the packed fields
+        const size_t back = std::max(R * (size_t)rec_slots(e->r),
+                                     final_slots(e, std::min<size_t>(R, (size_t)FEW_ROWS)));
+        OA_CHECK(e->rec2.ensure(back));
         size_t tmp = 0;
         OA_CU(cub::DeviceRadixSort::SortPairs(nullptr, tmp, e->keys.p, e->keys2.p, e->perm.p, e->perm2.p, (int)cap, 0,
                                               64, e->st));
         OA_CHECK(e->cub_tmp.ensure(tmp));
         const auto t_dev = std::chrono::steady_clock::now();
-        OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, R * rec_slots(e->r), e->retired_pinned));
+        OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, back, e->retired_pinned));
         if (e->cfg.disp_cov) {
             OA_CHECK(e->cov2.ensure(R * l * 3));
             OA_CHECK(ensure_pinned(e->h_cov, e->h_cov_cap, R * l * 3, e->retired_pinned));
@@ -2420,7 +2457,7 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
                 fprintf(stderr,
                         "[oa timing] oa_reserve: trait buffers %.1f ms, %zu row slots %.1f ms, page-locked rows "
                         "(%zu bytes) %.1f ms, stream sync %.1f ms\n",
-                        ms(api_clock.t0, t_traits), cap, ms(t_traits, t_dev), (size_t)(R * rec_slots(e->r) * sizeof(Rec)),
+                        ms(api_clock.t0, t_traits), cap, ms(t_traits, t_dev), (size_t)(back * sizeof(Rec)),
                         ms(t_dev, t_pin), ms(t_pin, t_end));
         }
     }

@@ -427,4 +427,70 @@ static __global__ void k_rec_gather(const RecOf<R>* __restrict__ rec, const int*
         for (int u = 0; u < l * 3; ++u) cov_out[(size_t)q * l * 3 + u] = cov[(size_t)src * l * 3 + u];
 }
 
+// Stored rows as the caller gets them (oa_rows): N each of trait, SNP, R2, n_used and coef_mask, then N x p
+// each of b, se, t.
+struct FinalRows {
+    int32_t* trait;
+    int32_t* snp;
+    float* r2;
+    int32_t* n_used;
+    uint32_t* mask;
+    float* b;
+    float* se;
+    float* t;
+};
+inline size_t final_row_bytes(int p) { return 20 + 12 * (size_t)p; }
+inline FinalRows final_rows(void* base, long long N, int p) {
+    int32_t* w = static_cast<int32_t*>(base);
+    FinalRows f;
+    f.trait = w;
+    f.snp = w + N;
+    f.r2 = reinterpret_cast<float*>(w + 2 * N);
+    f.n_used = w + 3 * N;
+    f.mask = reinterpret_cast<uint32_t*>(w + 4 * N);
+    f.b = reinterpret_cast<float*>(w + 5 * N);
+    f.se = f.b + N * p;
+    f.t = f.se + N * p;
+    return f;
+}
+
+// Thread = (row, coefficient): the l covariate terms (0 without them, the intercept's always) and the
+// caller's ru SNP terms of a row are p consecutive threads, so that the stores are coalesced.
+template <int R>
+static __global__ void __launch_bounds__(256)
+k_rec_final(const RecOf<R>* __restrict__ rec, const int* __restrict__ perm, long long N, int l, int ru,
+            const int* __restrict__ nobs, const float* __restrict__ cov, float min_t, int store_all, FinalRows out) {
+    const int p = l + ru;
+    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (q >= N * p) return;
+    const long long row = q / p;
+    const int h = (int)(q % p), src = perm[row];
+    const RecOf<R>& rc = rec[src];
+    const float* cv = cov ? cov + (size_t)src * l * 3 : nullptr;
+    float b = 0.f, se = 0.f, t = 0.f;
+    if (h >= l) {
+        b = rc.b[h - l];
+        se = rc.se[h - l];
+        t = rc.t[h - l];
+    } else if (cv && h > 0) {
+        b = cv[h * 3];
+        se = cv[h * 3 + 1];
+        t = cv[h * 3 + 2];
+    }
+    out.b[q] = b;
+    out.se[q] = se;
+    out.t[q] = t;
+    if (h == 0) {
+        uint32_t m = (rc.mask & ((1u << ru) - 1u)) << l;
+        if (cv)
+            for (int c = 1; c < l; ++c)
+                if (cv[c * 3 + 2] > min_t || store_all) m |= 1u << c;
+        out.trait[row] = rc.trait;
+        out.snp[row] = rc.snp;
+        out.r2[row] = rc.r2;
+        out.n_used[row] = nobs[rc.tint];
+        out.mask[row] = m;
+    }
+}
+
 }  // namespace oa
