@@ -170,42 +170,36 @@ __device__ __forceinline__ void split4h(const float4 p, float sc, uint2& hi, uin
 }
 
 // In-place inverse of a small SPD matrix (row-major k x k, k <= OA_MAX_R or
-// OA_MAX_L) by Cholesky.  Returns false if a pivot is not positive
-// relative to the diagonal scale (the system is treated as singular).
+// OA_MAX_L) by its L D L' factorisation: one division per pivot and no square
+// root (the Schur kernel solves millions of 1 x 1 and 2 x 2 systems).  Returns
+// false if a pivot (the Cholesky pivot, squared) is not positive relative to
+// its diagonal (the system is treated as singular).
 template <int K>
 __device__ __host__ inline bool spd_inverse(double* A, int k, double rel_tol) {
-    double L[K * K];
-    double dmax = 0.0;
-    for (int i = 0; i < k; ++i) dmax = fmax(dmax, fabs(A[i * k + i]));
-    if (!(dmax > 0.0)) return false;
-    for (int i = 0; i < k * k; ++i) L[i] = 0.0;
+    double L[K * K], U[K * K], di[K];   // unit lower L, U = L D below the diagonal, 1 / D
     for (int j = 0; j < k; ++j) {
         double s = A[j * k + j];
-        for (int q = 0; q < j; ++q) s -= L[j * k + q] * L[j * k + q];
+        for (int q = 0; q < j; ++q) s -= U[j * k + q] * L[j * k + q];
         if (!(s > rel_tol * fmax(fabs(A[j * k + j]), 1e-300))) return false;
-        double d = sqrt(s);
-        L[j * k + j] = d;
+        di[j] = 1.0 / s;
         for (int i = j + 1; i < k; ++i) {
             double u = A[i * k + j];
-            for (int q = 0; q < j; ++q) u -= L[i * k + q] * L[j * k + q];
-            L[i * k + j] = u / d;
+            for (int q = 0; q < j; ++q) u -= U[i * k + q] * L[j * k + q];
+            U[i * k + j] = u;
+            L[i * k + j] = u * di[j];
         }
     }
-    // inverse of L (lower), then A^-1 = L^-T L^-1
-    double Li[K * K];
-    for (int i = 0; i < k * k; ++i) Li[i] = 0.0;
-    for (int i = 0; i < k; ++i) {
-        Li[i * k + i] = 1.0 / L[i * k + i];
+    // M = L^-1 below its unit diagonal (in U), then A^-1 = M' D^-1 M
+    for (int i = 0; i < k; ++i)
         for (int j = 0; j < i; ++j) {
-            double s = 0.0;
-            for (int q = j; q < i; ++q) s += L[i * k + q] * Li[q * k + j];
-            Li[i * k + j] = -s / L[i * k + i];
+            double s = L[i * k + j];
+            for (int q = j + 1; q < i; ++q) s += L[i * k + q] * U[q * k + j];
+            U[i * k + j] = -s;
         }
-    }
     for (int i = 0; i < k; ++i)
         for (int j = 0; j <= i; ++j) {
-            double s = 0.0;
-            for (int q = i; q < k; ++q) s += Li[q * k + i] * Li[q * k + j];
+            double s = (j == i ? 1.0 : U[i * k + j]) * di[i];
+            for (int q = i + 1; q < k; ++q) s += U[q * k + i] * U[q * k + j] * di[q];
             A[i * k + j] = s;
             A[j * k + i] = s;
         }

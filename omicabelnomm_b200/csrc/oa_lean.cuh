@@ -792,23 +792,29 @@ __device__ __noinline__ void schur_quirk(const SchurArgs& S, int i, int g, size_
         for (int u = 0; u < l * R; ++u) S.aobs[gi * l * R + u] = (float)aq[u];
 }
 
-// All (SNP, pattern) systems of a SNP block in one persistent launch: a
-// thread per (SNP, slot) work item, grid-stride over the items.  Slot 0 is
-// the all-rows complement (var_x), slots 1..G the patterns, slots
-// G+1..G+Z copy the zero-set sums.
-template <int R>
-__device__ __forceinline__ void schur_item(const SchurArgs& S, int i, int slot) {
+// All (SNP, pattern) systems of a SNP block in one persistent launch.  Slot 0 is
+// the all-rows complement (var_x), slots 1..G the patterns, slots G+1..G+Z
+// copy the zero-set sums; a thread takes one SNP and up to SCHUR_SLOTS
+// consecutive slots, so that the SNP's projection, its all-rows complement and
+// that complement's factorisation (which every slot needs) are formed once for
+// them.  LC: covariates held in registers (l <= LC).  Bound by FP64 latency:
+// with one slot per thread and arrays in local memory 20,000 SNPs of two
+// columns x 151 slots took 415 us for 260 MB of sums and inverses (@S@ now).
+constexpr int SCHUR_SLOTS = 8;
+
+template <int R, int LC>
+__device__ __forceinline__ void schur_slots(const SchurArgs& S, int i, int slot0, int slot1) {
     const int l = S.l;
-    double a_full[OA_MAX_L * R];
-    if (S.Afull_lean) {
-        for (int qq = 0; qq < l; ++qq)
+    constexpr int UL = R <= 4 ? LC * R : 1;   // eight columns: arrays too large for registers, rolled loops
+    const int QL = R <= 4 ? LC : l;
+    double a_full[LC * R];
+#pragma unroll UL
+    for (int qq = 0; qq < QL; ++qq)
 #pragma unroll
-            for (int a = 0; a < R; ++a) a_full[qq * R + a] = S.Afull_lean[((size_t)i * R + a) * LEAN_QX_L + qq];
-    } else {
-        for (int qq = 0; qq < l; ++qq)
-#pragma unroll
-            for (int a = 0; a < R; ++a) a_full[qq * R + a] = (double)S.C2[(size_t)qq * S.ldc + i * R + a];
-    }
+        for (int a = 0; a < R; ++a)
+            a_full[qq * R + a] = qq >= l ? 0.0
+                                 : S.Afull_lean ? S.Afull_lean[((size_t)i * R + a) * LEAN_QX_L + qq]
+                                                : (double)S.C2[(size_t)qq * S.ldc + i * R + a];
     double Dm[R * R];
 #pragma unroll
     for (int u = 0; u < R * R; ++u) Dm[u] = (double)S.D[(size_t)i * R * R + u];
@@ -819,7 +825,9 @@ __device__ __forceinline__ void schur_item(const SchurArgs& S, int i, int slot) 
 #pragma unroll
         for (int b = 0; b < R; ++b) {
             double v = Dm[a * R + b];
-            for (int qq = 0; qq < l; ++qq) v -= a_full[qq * R + a] * a_full[qq * R + b];
+#pragma unroll UL
+            for (int qq = 0; qq < QL; ++qq)
+                if (qq < l) v -= a_full[qq * R + a] * a_full[qq * R + b];
             Sf[a * R + b] = v;
         }
     double dss[R];
@@ -831,80 +839,103 @@ __device__ __forceinline__ void schur_item(const SchurArgs& S, int i, int slot) 
     for (int a = 0; a < R; ++a)
         if (a >= S.rr) Sf[a * R + a] = dss[a] = 1.0;
     const bool full_ok = schur_inverse<R>(Sf, dss);
-    if (slot == 0) {
+    for (int slot = slot0; slot < slot1; ++slot) {
+        if (slot == 0) {
 #pragma unroll
-        for (int a = 0; a < R; ++a) S.varx[(size_t)i * R + a] = full_ok ? (float)Sf[a * R + a] : 0.f;
-        if (S.sfinv)
+            for (int a = 0; a < R; ++a) S.varx[(size_t)i * R + a] = full_ok ? (float)Sf[a * R + a] : 0.f;
+            if (S.sfinv)
 #pragma unroll
-            for (int u = 0; u < R * R; ++u) S.sfinv[(size_t)i * R * R + u] = full_ok ? Sf[u] : 0.0;
-        if (S.afull)
-            for (int u = 0; u < l * R; ++u) S.afull[(size_t)i * l * R + u] = (float)a_full[u];
-        return;
-    }
-    if (slot > S.G) {  // zero set z: its sums go to the epilogue unchanged
-        const int z = slot - 1 - S.G;
-        const size_t zi = (size_t)z * S.mb + i;
-        for (int qq = 0; qq < l; ++qq)
+                for (int u = 0; u < R * R; ++u) S.sfinv[(size_t)i * R * R + u] = full_ok ? Sf[u] : 0.0;
+            if (S.afull)
+#pragma unroll UL
+                for (int u = 0; u < QL * R; ++u)
+                    if (u < l * R) S.afull[(size_t)i * l * R + u] = (float)a_full[u];
+            continue;
+        }
+        if (slot > S.G) {  // zero set z: its sums go to the epilogue unchanged
+            const int z = slot - 1 - S.G;
+            const size_t zi = (size_t)z * S.mb + i;
+            for (int qq = 0; qq < l; ++qq)
+#pragma unroll
+                for (int a = 0; a < R; ++a)
+                    S.zA[zi * l * R + qq * R + a] = S.C2[(size_t)(l + (S.G + z) * l + qq) * S.ldc + i * R + a];
+#pragma unroll
+            for (int u = 0; u < R * R; ++u) S.zD[zi * R * R + u] = S.Dset[((size_t)(S.G + z) * S.mb + i) * R * R + u];
+            continue;
+        }
+        const int g = slot - 1;
+        const size_t gi = (size_t)g * S.mb + i;
+        double ao[LC * R];
+#pragma unroll UL
+        for (int qq = 0; qq < QL; ++qq)
 #pragma unroll
             for (int a = 0; a < R; ++a)
-                S.zA[zi * l * R + qq * R + a] = S.C2[(size_t)(l + (S.G + z) * l + qq) * S.ldc + i * R + a];
+                ao[qq * R + a] =
+                    qq < l ? a_full[qq * R + a] - (double)S.C2[(size_t)(l + g * l + qq) * S.ldc + i * R + a] : 0.0;
+        double Sg[R * R];
 #pragma unroll
-        for (int u = 0; u < R * R; ++u) S.zD[zi * R * R + u] = S.Dset[((size_t)(S.G + z) * S.mb + i) * R * R + u];
-        return;
-    }
-    const int g = slot - 1;
-    const size_t gi = (size_t)g * S.mb + i;
-    double ao[OA_MAX_L * R];
-    for (int qq = 0; qq < l; ++qq)
+        for (int u = 0; u < R * R; ++u) Sg[u] = Dm[u] - (double)S.Dset[gi * R * R + u];
+        double dso[R];
 #pragma unroll
-        for (int a = 0; a < R; ++a)
-            ao[qq * R + a] = a_full[qq * R + a] - (double)S.C2[(size_t)(l + g * l + qq) * S.ldc + i * R + a];
-    double Sg[R * R];
+        for (int a = 0; a < R; ++a) dso[a] = a < S.rr ? Sg[a * R + a] : 1.0;
+        const double* Wg = S.W + (size_t)g * l * l;
+#pragma unroll UL
+        for (int qq = 0; qq < QL; ++qq) {
+            if (qq < l) {
+                double wa[R];
 #pragma unroll
-    for (int u = 0; u < R * R; ++u) Sg[u] = Dm[u] - (double)S.Dset[gi * R * R + u];
-    double dso[R];
+                for (int b = 0; b < R; ++b) wa[b] = 0.0;
+#pragma unroll UL
+                for (int u = 0; u < QL; ++u) {
+                    if (u < l) {
+                        const double wq = Wg[qq * l + u];
 #pragma unroll
-    for (int a = 0; a < R; ++a) dso[a] = a < S.rr ? Sg[a * R + a] : 1.0;
-    const double* Wg = S.W + (size_t)g * l * l;
-    for (int qq = 0; qq < l; ++qq) {
-        double wa[R];
+                        for (int b = 0; b < R; ++b) wa[b] += wq * ao[u * R + b];
+                    }
+                }
 #pragma unroll
-        for (int b = 0; b < R; ++b) wa[b] = 0.0;
-        for (int u = 0; u < l; ++u) {
-            const double wq = Wg[qq * l + u];
+                for (int a = 0; a < R; ++a)
 #pragma unroll
-            for (int b = 0; b < R; ++b) wa[b] += wq * ao[u * R + b];
+                    for (int b = 0; b < R; ++b) Sg[a * R + b] -= ao[qq * R + a] * wa[b];
+            }
+        }
+        if (S.qK) {
+            double aoq[LC * R], Dq[R * R], dq[R];   // copies: the arrays above stay in registers
+#pragma unroll UL
+            for (int u = 0; u < QL * R; ++u) aoq[u] = ao[u];
+#pragma unroll
+            for (int u = 0; u < R * R; ++u) Dq[u] = Dm[u];
+#pragma unroll
+            for (int a = 0; a < R; ++a) dq[a] = dso[a];
+            schur_quirk<R>(S, i, g, gi, aoq, Dq, dq, full_ok);
+            continue;
         }
 #pragma unroll
         for (int a = 0; a < R; ++a)
+            if (a >= S.rr) Sg[a * R + a] = 1.0;
+        const bool ok = full_ok && !S.pat_bad[g] && schur_inverse<R>(Sg, dso);
+        S.sing[gi] = ok ? 0 : 1;
 #pragma unroll
-            for (int b = 0; b < R; ++b) Sg[a * R + b] -= ao[qq * R + a] * wa[b];
+        for (int u = 0; u < R * R; ++u) S.sinv[gi * R * R + u] = ok ? Sg[u] : 0.0;
+        if (S.aobs)
+#pragma unroll UL
+            for (int u = 0; u < QL * R; ++u)
+                if (u < l * R) S.aobs[gi * l * R + u] = (float)ao[u];
     }
-    if (S.qK) {
-        schur_quirk<R>(S, i, g, gi, ao, Dm, dso, full_ok);
-        return;
-    }
-#pragma unroll
-    for (int a = 0; a < R; ++a)
-        if (a >= S.rr) Sg[a * R + a] = 1.0;
-    const bool ok = full_ok && !S.pat_bad[g] && schur_inverse<R>(Sg, dso);
-    S.sing[gi] = ok ? 0 : 1;
-#pragma unroll
-    for (int u = 0; u < R * R; ++u) S.sinv[gi * R * R + u] = ok ? Sg[u] : 0.0;
-    if (S.aobs)
-        for (int u = 0; u < l * R; ++u) S.aobs[gi * l * R + u] = (float)ao[u];
 }
 
-// Items are numbered slot-major (consecutive threads take consecutive SNPs of one slot), so that
-// a warp's loads of the SNP-indexed sums (pre-GEMM columns, D, D_s) and its stores of the
+// Items (SNP, `per` slots) are numbered slot-major (consecutive threads take consecutive SNPs of one slot
+// range), so that a warp's loads of the SNP-indexed sums (pre-GEMM columns, D, D_s) and its stores of the
 // inverses are coalesced and the slot's W_g is one broadcast.
-template <int R>
-__global__ void __launch_bounds__(256) k_schur(SchurArgs S) {
+template <int R, int LC>
+__global__ void __launch_bounds__(256) k_schur(SchurArgs S, int per) {
     const int slots = 1 + S.G + S.Z;
-    const long long total = (long long)S.mb * slots;
+    const long long total = (long long)S.mb * ((slots + per - 1) / per);
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
-         q += (long long)gridDim.x * blockDim.x)
-        schur_item<R>(S, (int)(q % S.mb), (int)(q / S.mb));
+         q += (long long)gridDim.x * blockDim.x) {
+        const int slot0 = (int)(q / S.mb) * per;
+        schur_slots<R, LC>(S, (int)(q % S.mb), slot0, min(slots, slot0 + per));
+    }
 }
 
 }  // namespace oa

@@ -180,20 +180,38 @@ cudaError_t oa_set_wait_limit_stats(unsigned long long ns) {
     return cudaMemcpyToSymbol(c_st_wait_ns, &ns, sizeof ns);
 }
 
+template <int R>
+static void go_schur(const SchurArgs& S, int per, unsigned blocks, cudaStream_t st) {
+    if constexpr (R == 8) {
+        k_schur<R, 16><<<blocks, 256, 0, st>>>(S, per);
+    } else if (S.l > 8) {
+        k_schur<R, 16><<<blocks, 256, 0, st>>>(S, per);
+    } else if (S.l > 4) {
+        k_schur<R, 8><<<blocks, 256, 0, st>>>(S, per);
+    } else {
+        k_schur<R, 4><<<blocks, 256, 0, st>>>(S, per);
+    }
+}
+
 cudaError_t oa_launch_schur(int R, const SchurArgs& S, cudaStream_t st) {
-    const long long total = (long long)S.mb * (1 + S.G + S.Z);
-    if (total <= 0) return cudaSuccess;
+    const long long slots = 1 + S.G + S.Z;
+    if (S.mb <= 0) return cudaSuccess;
     // persistent: at most 8 resident CTAs of 256 threads per SM
     static int sms[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!sms[dev & 63]) cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
+    // slots per thread: as many as leave every resident thread an item
+    const long long room = 8LL * sms[dev & 63] * 256;
+    int per = 1;
+    while (per < SCHUR_SLOTS && (long long)S.mb * ((slots + 2 * per - 1) / (2 * per)) >= room) per *= 2;
+    const long long total = (long long)S.mb * ((slots + per - 1) / per);
     const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, 8LL * sms[dev & 63]);
     switch (R) {
-        case 1: k_schur<1><<<blocks, 256, 0, st>>>(S); break;
-        case 2: k_schur<2><<<blocks, 256, 0, st>>>(S); break;
-        case 4: k_schur<4><<<blocks, 256, 0, st>>>(S); break;
-        case 8: k_schur<8><<<blocks, 256, 0, st>>>(S); break;
+        case 1: go_schur<1>(S, per, blocks, st); break;
+        case 2: go_schur<2>(S, per, blocks, st); break;
+        case 4: go_schur<4>(S, per, blocks, st); break;
+        case 8: go_schur<8>(S, per, blocks, st); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
