@@ -77,15 +77,16 @@ __device__ __forceinline__ uint8_t test_flags(const EpiArgs& E, double rss, floa
     return mask ? OA_TEST_STORED : 0;
 }
 
-// Schur inverse of (pattern g, SNP i); false if the system is singular.
+// Schur inverse of (pattern g, SNP i); false if the system is singular (its inverse is stored as zeros,
+// so that both loads can be in flight together).
 template <int R>
 __device__ __forceinline__ bool load_schur(const EpiArgs& E, int g, int i, double* S) {
     const size_t gi = (size_t)g * E.mb + i;
-    if (E.sing[gi]) return false;
+    const uint8_t sing = E.sing[gi];
     const double* src = E.sinv + gi * (R * R);
 #pragma unroll
     for (int q = 0; q < R * R; ++q) S[q] = src[q];
-    return true;
+    return sing == 0;
 }
 
 // Fitted values of the observed rows whose y is exactly 0 leave the RSS

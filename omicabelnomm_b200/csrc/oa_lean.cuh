@@ -799,7 +799,7 @@ __device__ __noinline__ void schur_quirk(const SchurArgs& S, int i, int g, size_
 // that complement's factorisation (which every slot needs) are formed once for
 // them.  LC: covariates held in registers (l <= LC).  Bound by FP64 latency:
 // with one slot per thread and arrays in local memory 20,000 SNPs of two
-// columns x 151 slots took 415 us for 260 MB of sums and inverses (@S@ now).
+// columns x 151 slots took 415 us for 260 MB of sums and inverses (333 us now).
 constexpr int SCHUR_SLOTS = 8;
 
 template <int R, int LC>
