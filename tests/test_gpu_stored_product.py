@@ -244,3 +244,83 @@ def test_model_columns_give_the_direct_columns_bits(n, model, prec):
         eng.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", [E.PLAIN, E.MIXED])
+@pytest.mark.parametrize("l,r", [(3, 1), (4, 2), (8, 1), (9, 1), (5, 2)])
+def test_many_systems_per_thread_give_the_same_bits(l, r, prec):
+    """Schur systems taken eight row sets a thread (12,500 SNPs x 201 slots) against the same SNPs in a block
+    small enough for one a thread, covariates in 4, 8 and 16 registers."""
+    n, m, t, few = 120, 12500, 200, 67
+    ds = synth.generate(synth.scaled(0, n=n, m=m, t=t, l=l, r=r, miss_frac=0.05, seed=400 + l))
+    out = []
+    for mb in (m, few):
+        eng = E.Engine(n, l, r, t, mb, precision=prec, min_t_store=8.0, min_r2_store=1e-6)
+        eng.set_tuning(chunk_snps=m)
+        eng.set_covariates(ds.XL)
+        eng.set_traits(ds.Y)
+        eng.enable_dense(True)
+        eng.run(np.ascontiguousarray(ds.XR[:mb * r]))
+        assert eng.tuning()["stats_path"] == 1
+        out.append(eng.dense(mb))
+        eng.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a[:, :few], b)
+
+
+def test_plain_product_in_trait_segments():
+    """More traits than one stored product holds (8,192): the last segment and its edges."""
+    t = 8192 + 131
+    ds = synth.generate(synth.scaled(0, n=130, m=40, t=t, l=3, miss_mode="patterns", n_patterns=3, seed=411))
+    _, rows, dense = engine_run(ds, 1)
+    check_plain(ds, 1, dense)
+    assert rows.tests == 40 * t
+
+
+@pytest.mark.parametrize("prec", [E.PLAIN, E.MIXED])
+def test_statistics_path_changed_after_the_traits(prec):
+    """The pre-GEMM's columns are added behind a trait block that was set while the row gathers were chosen."""
+    ds = synth.generate(synth.scaled(0, n=333, m=140, t=60, l=4, miss_mode="patterns", n_patterns=7, seed=412))
+    out = []
+    for late in (False, True):
+        eng = E.Engine(333, 4, 1, 60, 140, precision=prec, store_all=True, min_t_store=1.6, min_r2_store=1e-6)
+        eng.set_tuning(stats_path=2 if late else 1)
+        eng.set_covariates(ds.XL)
+        eng.set_traits(ds.Y)
+        eng.set_tuning(stats_path=1)
+        eng.enable_dense(True)
+        eng.run(ds.XR)
+        out.append(eng.dense(140))
+        eng.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,r", [(9599, 2), (9600, 2), (9601, 2), (16384, 1), (12800, 4)])
+def test_long_columns(n, r):
+    """Either side of the lengths from which a SNP's columns take a group of 512 threads."""
+    ds = QC.multicol(r, 420, n=n, m=19, t=6, n_patterns=2) if r > 2 else synth.generate(
+        synth.scaled(0, n=n, m=19, t=6, l=4, r=r, miss_mode="patterns", n_patterns=2, seed=420))
+    _, _, dense = engine_run(ds, r)
+    check_plain(ds, r, dense)
+
+
+def test_few_and_many_rows_with_covariate_terms():
+    """Rows with every covariate term: one block whose rows come back in pieces against two that are formed on
+    the device as the caller gets them."""
+    t, m = 64, 4099
+    ds = synth.generate(synth.scaled(0, n=150, m=m, t=t, l=5, miss_mode="patterns", n_patterns=4, seed=430))
+    _, whole, _ = engine_run(ds, 1, disp_cov=True)
+    assert len(whole.trait) > 1 << 18
+    half = []
+    for lo, hi in ((0, 2050), (2050, m)):
+        part = type(ds)(**{**ds.__dict__, "XR": np.ascontiguousarray(ds.XR[lo:hi])})
+        _, rows, _ = engine_run(part, 1, disp_cov=True)
+        assert len(rows.trait) <= 1 << 18
+        half.append((rows, lo))
+    key = np.concatenate([rows.trait.astype(np.int64) * m + rows.snp + lo for rows, lo in half])
+    order = np.argsort(key)
+    np.testing.assert_array_equal(key[order], whole.trait.astype(np.int64) * m + whole.snp)
+    for field in ("r2", "mask", "B", "SE", "T"):
+        got = np.concatenate([getattr(rows, field) for rows, _ in half])[order]
+        np.testing.assert_array_equal(got, getattr(whole, field))
