@@ -53,7 +53,7 @@ typedef enum oa_status {
 } oa_status;
 
 typedef enum oa_precision {
-    OA_PLAIN_FP32 = 0,   /* FP32 data, FP32 SIMT GEMM, FP64 small systems */
+    OA_PLAIN_FP32 = 0,   /* FP32 data, tcgen05 products of FP16 hi/lo splits summed in FP32, FP64 small systems */
     OA_MIXED_BF16X3 = 1  /* XR'Y on tcgen05 tensor cores, BF16 hi/lo 3-product, FP32 accumulate */
 } oa_precision;
 
@@ -232,7 +232,7 @@ oa_status oa_scan_dense_noalloc(const float* xl_dev, const float* y_dev, const f
  * fixed at src/Algorithm.cpp:361-372). */
 typedef struct oa_tuning {
     int32_t chunk_snps;    /* SNPs per device chunk: one launch of each per-block kernel */
-    int32_t gemm_variant;  /* tensor-core pipeline: 1 = K-block 32 x 4 stages, 2 = K-block 64 x 2 stages,
+    int32_t gemm_variant;  /* mixed form: tensor-core pipeline: 1 = K-block 32 x 4 stages, 2 = K-block 64 x 2,
                               3 = CTA pairs on neighbouring SMs (2-SM MMA, 256 x 256 tiles), K-block 32 x 6,
                               4 = CTA pairs, K-block 64 x 3 (the default); trait blocks of at most 128
                               traits use 1-SM tiles of 64 or 128 columns whatever the variant */

@@ -5,9 +5,12 @@
 //   k_trait_stats -> host groups traits by missingness pattern (and by the
 //   set of observed exact zeros) -> k_set_rows -> k_set_gram -> k_trait_resid
 // Per SNP chunk (≙ src/Algorithm.cpp:610-813):
-//   k_snp_lean -> pre-GEMM [Q | Q o m_1 | ...]'X -> k_schur   (few row sets)
-//   or k_snp_stats (one kernel with row gathers; many row sets)
-//   -> XR'Y~ GEMM with fused statistics epilogue -> (covariate terms)
+//   k_snp_lean -> pre-GEMM [Q | Q o m_1 | ...]'X -> k_schur
+//   or k_snp_stats (one kernel with row gathers; thousands of row sets)
+//   -> mixed: XR'Y~ GEMM with fused statistics epilogue
+//      plain, narrow mixed blocks: stored product X'[Y~ | B2] (traits and
+//      pre-GEMM columns in one launch) -> k_schur -> k_test_stats
+//   -> (covariate terms)
 // Per API call: sort of the stored rows into reference order (trait, SNP).
 #include <algorithm>
 #include <chrono>

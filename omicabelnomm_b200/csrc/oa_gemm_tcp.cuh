@@ -17,7 +17,10 @@
 // What bounds it: 12 tcgen05.mma per K-block and 256 x 256 pair tile, 128
 // cycles each, while the drain of that K-block (128 columns of 32 lanes per
 // warp: tcgen05.ld + FADD) takes about a third of them; at small column
-// counts the reading of X.
+// counts the reading of X.  Measured (60,000 SNPs x 1,084 columns, n =
+// 10,000): FP32 SIMT 26.5 + 5.0 ms in two launches a chunk, this 2.87 ms =
+// 1.36 PFLOP/s of FP16 products (the power-capped rate of a dense GEMM);
+// error against 64 bits 1.6e-6 -> 2.7e-7 of the outputs' 2-norm.
 //
 // The product is stored (not evaluated in the epilogue): the register sums
 // leave no registers for the statistics, and z is 4 bytes per test against

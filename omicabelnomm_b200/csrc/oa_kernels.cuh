@@ -9,7 +9,7 @@
 //  k_set_rows     ordered row list of each row set (missing pattern / zero set)
 //  k_set_gram     per pattern W = (Q_obs'Q_obs)^-1, per zero set sum q q'
 //                 (≙ generate_correction_missings_Stl, src/Algorithm.cpp:1324-1362)
-//  k_trait_resid  y~ = y - Q_obs W Q'y on observed rows, RSS0, SST
+//  k_trait_resid  y~ = y - Q_obs W Q'y on observed rows (hi / lo split), RSS0, SST
 //  k_snp_stats    per SNP column: NaN mean-imputation, X'X diagonal block,
 //                 Q'X, missing-row downdates per row set, FP64 Schur
 //                 complements and their inverses per (pattern, SNP)

@@ -9,7 +9,8 @@
 //     (x-only gathers, no covariate loads);
 //   * Q'X and (Q o m_s)'X for every row set s: a GEMM of the SNP block with
 //     the column matrix B2 = [Q | Q o m_1 | ... | Q o m_S] ("pre-GEMM", on
-//     the same tensor-core / SIMT kernels as the main contraction);
+//     the tensor cores, in one launch with the traits where their product is
+//     stored as well);
 // and k_schur forms, per (pattern, SNP), the FP64 Schur complement
 //     (D - D_g) - (A - A_g)' W_g (A - A_g)
 // and its inverse, plus var_x from the all-rows complement D - A'A.
@@ -89,8 +90,9 @@ inline int lean_threads_for(int R, int n_pad) {
 
 // SNPs per group where the caller asks for none (a power of two): at most four columns, as far as they fit
 // the group's bytes and leave at least two groups per SM.  With one column per SNP two SNPs are worth going
-// down to three CTAs per SM, four to five (50,000 SNPs, statistics stage with 1 / 2 / 4 / 8 SNPs per group: n = 1,000 0.29 / 0.18 / 0.16 /
-// 0.19 ms, n = 2,000 0.33 / 0.21 / 0.20 / 0.26, n = 3,500 0.39 / 0.27 / 0.29 / 0.34, n = 7,000 0.65 / 0.62 / - / -, n = 10,000 1.37 / 1.46 / - / -);
+// down to three CTAs per SM, four to five (50,000 SNPs, statistics stage with 1 / 2 / 4 / 8 SNPs per group:
+// n = 1,000 0.29 / 0.18 / 0.16 / 0.19 ms, n = 2,000 0.33 / 0.21 / 0.20 / 0.26, n = 3,500 0.39 / 0.27 / 0.29 /
+// 0.34, n = 7,000 0.65 / 0.62 / - / -, n = 10,000 1.37 / 1.46 / - / -);
 // with two, the covariate basis read once per group is worth two CTAs (20,000 SNPs, n = 6,000 1.27 / 1.23).
 inline int lean_auto_spb(int R, int n_pad, bool qx, int snps, int sms) {
     int s = 1;

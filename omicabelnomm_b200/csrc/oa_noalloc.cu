@@ -4,9 +4,10 @@
 // Some callers cannot call cudaMalloc: plug-ins inside host frameworks that
 // own the device memory pool (and forbid raw allocations), and processes
 // under a hard device-memory cap whose memory was reserved up front.  This
-// entry point gives them the engine's plain-FP32 block scan (the SIMT GEMM
-// with fused statistics, plus the small kernels that prepare its tables)
-// with every intermediate buffer carved from one file-scope
+// entry point gives them the engine's plain-FP32 block scan (column
+// statistics, one stored tensor-core product, Schur systems and tests, in
+// chunks of SNPs; or row gathers and the SIMT GEMM with fused statistics
+// where that does not fit) with every intermediate buffer carved from one file-scope
 // `static __device__` array of OA_NOALLOC_SCRATCH_BYTES.  It calls no
 // cudaMalloc / cudaFree and no allocating library routine, and allocates no
 // host heap memory either.

@@ -6,9 +6,11 @@
 // consecutive SNPs), the Schur inverses and var_x are coalesced loads and no
 // shuffle gathers a SNP's columns; a work item is 256 SNPs x 64 traits whose
 // constants sit in shared memory.  z is read eight traits at a time before
-// they are evaluated.  Bound by instruction issue (about 40 slots per test,
-// most of them the FP64 residual sum): two CTAs of eight warps per SM keep
-// the FP64 chain's latency covered within 128 registers a thread.
+// they are evaluated.  Bound by instruction issue (77 warp instructions per 32
+// tests in full, most of them the FP64 residual sum; fewer where the FP32
+// screening drops a warp's tests: 60 M tests 0.41 -> 0.23 ms): two CTAs of
+// eight warps per SM keep the FP64 chain's latency covered within 128
+// registers a thread.
 #pragma once
 #include "oa_epilogue.cuh"
 
