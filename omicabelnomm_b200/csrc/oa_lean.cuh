@@ -550,7 +550,8 @@ k_snp_lean(LeanArgs A) {
 
         // ---- pass 2: 16-bit hi/lo split of the shifted columns, 4 rows per thread and step (eight
         // rows, two 16-byte loads at a 32-byte stride, cost two wavefronts for one).  The tail rows
-        // [n, n_pad) get -sh: the other operands of the GEMMs are zero there.
+        // [n, n_pad) are zero: the other operands of the GEMMs are too, but 0 - sh times the FP16 scale
+        // (which the shifted column's norm bounds, not its mean) would overflow, and inf x 0 is NaN.
         if (A.write_split) {
             by_offset([&](auto O) {
 #pragma unroll 2
@@ -561,6 +562,12 @@ k_snp_lean(LeanArgs A) {
                         const float s0 = sh[c];
                         float4 p = ld4(O, c, k4);
                         p.x -= s0; p.y -= s0; p.z -= s0; p.w -= s0;
+                        if (4 * k4 + 4 > n) {
+                            if (4 * k4 >= n) p.x = 0.f;
+                            if (4 * k4 + 1 >= n) p.y = 0.f;
+                            if (4 * k4 + 2 >= n) p.z = 0.f;
+                            p.w = 0.f;
+                        }
                         uint2 h, o;
                         if (A.xscale)
                             split4h(p, hs[c], h, o);
