@@ -209,6 +209,94 @@ __host__ __device__ constexpr int lean_pair(int a, int b) {
     return a * R - a * (a - 1) / 2 + (b - a);
 }
 
+// A column whose sum of squares `raw` is 8 times that of the centred column or more (1 + mean^2 / variance): the
+// difference of the raw FP32 sums keeps 2^-24 times this ratio of the centred one.  Dosages of the minor
+// allele stay below 3; an expression level of 8 +- 2 has 17, one of 12 +- 0.05 57,601 (n = 1,000, beta's
+// error from the raw sums 1.8e-3, from the moved column's 1.6e-7).
+__device__ __forceinline__ bool lean_narrow(float raw, float mean, int n) {
+    return 8.f * (float)n * mean * mean > 7.f * raw;
+}
+
+// Moves the narrow columns of a group to their means in place (moved[c]: what was taken off, untouched
+// elsewhere) and sums their SNPs again in FP64, into the block's sums (bc: column sums, cross products,
+// Q'x with l covariates, Qb); offs: two bits of offset per column.  A constant column becomes exact zeros,
+// whatever its mean was rounded to.  Called by the whole block, out of line: rare, and its code and
+// registers stay out of the usual case's.
+template <int R, int NC, bool QX>
+__device__ __noinline__ void lean_recentre(float* cols, int cs, unsigned offs, int n, int ncol, double* red, double* bc,
+                                           float* moved, const float4* Qb, int l) {
+    constexpr int NP = R * (R + 1) / 2, NU = NC / R * NP;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto column = [&](int c) { return cols + (size_t)c * cs + (offs >> (2 * c) & 3u); };
+    auto block_total = [&](double v, double* out) {
+        v = warp_sum(v);
+        if (lane == 0) red[w] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0.0;
+            for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += red[q];
+            *out = s;
+        }
+        __syncthreads();
+    };
+    __syncthreads();   // the columns are swept, the sums read
+#pragma unroll 1
+    for (int i = 0; i < ncol; i += R) {
+        int narrow = 0;
+#pragma unroll
+        for (int a = 0; a < R; ++a) {
+            const float mean = (float)(bc[i + a] / (double)n);
+            if (lean_narrow((float)bc[NC + i / R * NP + lean_pair<R>(a, a)], mean, n)) narrow |= 1 << a;
+        }
+        if (!narrow) continue;   // block-uniform
+#pragma unroll 1
+        for (int a = 0; a < R; ++a) {
+            if (!(narrow >> a & 1)) continue;
+            float* col = column(i + a);
+            const float first = col[0], mean = (float)(bc[i + a] / (double)n);
+            int differs = 0;
+            for (int k = threadIdx.x; k < n; k += blockDim.x) differs |= col[k] != first;
+            const float shift = __syncthreads_or(differs) ? mean : first;
+            for (int k = threadIdx.x; k < n; k += blockDim.x) col[k] -= shift;
+            if (threadIdx.x == 0) moved[i + a] = shift;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int a = 0; a < R; ++a) {
+            const float* xa = column(i + a);
+#pragma unroll 1
+            for (int b = a; b < R; ++b) {
+                if (!(narrow >> a & 1) && !(narrow >> b & 1)) continue;
+                const float* xb = column(i + b);
+                double sum = 0.0, prod = 0.0;
+                for (int k = threadIdx.x; k < n; k += blockDim.x) {
+                    sum += (double)xa[k];
+                    prod += (double)xa[k] * (double)xb[k];
+                }
+                if (b == a) block_total(sum, bc + i + a);
+                block_total(prod, bc + NC + i / R * NP + lean_pair<R>(a, b));
+            }
+            if (QX && (narrow >> a & 1))
+#pragma unroll 1
+                for (int q = 0; q < l; ++q) {
+                    double dot = 0.0;
+                    for (int k = threadIdx.x; k < n; k += blockDim.x)
+                        dot += (double)reinterpret_cast<const float*>(Qb + (size_t)(k / 4) * l + q)[k % 4] * (double)xa[k];
+                    block_total(dot, bc + NC + NU + (i + a) * LEAN_QX_L + q);
+                }
+        }
+    }
+}
+
+// Resident CTAs the register allocation leaves room for: 64 registers a thread for groups of one or two
+// columns or of four SNPs, 48 for two SNPs and 40 for a gathered one (where shared memory holds five and
+// six CTAs of 256 threads), else 128.
+constexpr int lean_min_ctas(int R, int SPB, bool gather, int NT) {
+    if (R == 1 && SPB == 2) return 5;
+    if (R == 1 && SPB == 1 && gather) return 1536 / NT;
+    return R * SPB <= 2 || (R == 1 && SPB == 4) ? 1024 / NT : 512 / NT;
+}
+
 // One CTA handles SPB SNPs (SPB*R columns) per group in a persistent loop over groups:
 //   staging the group's columns stream into shared memory by TMA bulk copies.  A column that does not
 //           start on a 16-byte boundary (any n that is no multiple of 4) is copied from the boundary
@@ -223,7 +311,9 @@ __host__ __device__ constexpr int lean_pair(int a, int b) {
 //           intercept among the covariates every later sum uses x - mean
 //           (the Schur complements, X'y~ and var_x do not change; the sums
 //           lose their large common part); X'X of the shifted columns
-//           follows from the raw sums in FP64
+//           follows from the raw sums in FP64, and where that difference
+//           would cancel (lean_narrow) the column is moved to its mean in
+//           place and summed again first
 //   pass 2  16-bit hi/lo split of the shifted columns
 //   pass 3  X'X over each row set: work items of up to four index blocks of one set
 //           (fixed per trait block) go round-robin to the warps; a warp's item
@@ -238,7 +328,7 @@ __host__ __device__ constexpr int lean_pair(int a, int b) {
 // rate); with 20 sets of 500 rows the set pass takes the shared-memory pipe to 0.6 and it runs at
 // 4.8 TB/s (n = 10,000).  Unaligned columns: 0.86 ms where 4-byte copies took 1.27 (n = 12,347).
 template <int R, int SPB, bool GATHER, bool QX = false, int NT = 256>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, lean_min_ctas(R, SPB, GATHER, NT))
 k_snp_lean(LeanArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int NC = SPB * R;                 // columns per group
@@ -252,6 +342,7 @@ k_snp_lean(LeanArgs A) {
         (reinterpret_cast<uintptr_t>(part + (size_t)A.items_cap * NU) + 7) & ~(uintptr_t)7);   // [LEAN_MAX_WARPS + 1][NQ]
     __shared__ __align__(8) uint64_t mbar;
     __shared__ int stop;
+    __shared__ float moved[NC];                 // taken off the staged column (lean_recentre)
     const int ngroups = (A.mb + SPB - 1) / SPB;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // some column starts or ends off a 16-byte boundary: copies write past column ends
@@ -410,6 +501,7 @@ k_snp_lean(LeanArgs A) {
             float cmean[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) cnan[c] = false;
+            if ((int)threadIdx.x < NC) moved[threadIdx.x] = 0.f;   // before the sums' barriers
             for (int round = 0;; ++round) {
                 float acc[NV];
 #pragma unroll
@@ -493,6 +585,24 @@ k_snp_lean(LeanArgs A) {
                 }
                 __syncthreads();
             }
+            if (A.center) {
+                bool narrow = false;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    narrow |= c < ncol && lean_narrow((float)tot[NC + c / R * NP + lean_pair<R>(c % R, c % R)], cmean[c], n);
+                if (narrow) {   // block-uniform
+                    unsigned offs = 0;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) offs |= (unsigned)off[c] << (2 * c);
+                    double* bc = red + LEAN_MAX_WARPS * NV;
+                    lean_recentre<R, NC, QX>(cols, cs, offs, n, ncol, red, bc, moved, A.Qb, A.l);
+#pragma unroll
+                    for (int u = 0; u < NB; ++u) tot[u] = bc[u];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (moved[c] != 0.f) cmean[c] = (float)(tot[c] / (double)n);
+                }
+            }
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 sh[c] = A.center ? cmean[c] : 0.f;
@@ -525,7 +635,7 @@ k_snp_lean(LeanArgs A) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     if (c < ncol) {
-                        A.mean[i0 * R + c] = A.center ? cmean[c] : (cnan[c] ? cmean[c] : 0.f);
+                        A.mean[i0 * R + c] = A.center ? moved[c] + cmean[c] : (cnan[c] ? cmean[c] : 0.f);
                         if (cnan[c]) atomicOr(A.has_nan, 1);
                     }
                 }
@@ -553,31 +663,39 @@ k_snp_lean(LeanArgs A) {
         // [n, n_pad) are zero: the other operands of the GEMMs are too, but 0 - sh times the FP16 scale
         // (which the shifted column's norm bounds, not its mean) would overflow, and inf x 0 is NaN.
         if (A.write_split) {
+            auto store = [&](int c, int k4, const float4& p) {
+                uint2 h, o;
+                if (A.xscale)
+                    split4h(p, hs[c], h, o);
+                else
+                    split4(p, h, o);
+                reinterpret_cast<uint2*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k4] = h;
+                reinterpret_cast<uint2*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k4] = o;
+            };
             by_offset([&](auto O) {
 #pragma unroll 2
-                for (int k4 = threadIdx.x; k4 < A.n_pad / 4; k4 += NT) {
+                for (int k4 = threadIdx.x; k4 < n / 4; k4 += NT) {
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
                         if (c >= ncol) continue;
                         const float s0 = sh[c];
                         float4 p = ld4(O, c, k4);
                         p.x -= s0; p.y -= s0; p.z -= s0; p.w -= s0;
-                        if (4 * k4 + 4 > n) {
-                            if (4 * k4 >= n) p.x = 0.f;
-                            if (4 * k4 + 1 >= n) p.y = 0.f;
-                            if (4 * k4 + 2 >= n) p.z = 0.f;
-                            p.w = 0.f;
-                        }
-                        uint2 h, o;
-                        if (A.xscale)
-                            split4h(p, hs[c], h, o);
-                        else
-                            split4(p, h, o);
-                        reinterpret_cast<uint2*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k4] = h;
-                        reinterpret_cast<uint2*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k4] = o;
+                        store(c, k4, p);
                     }
                 }
             });
+            // the last rows and the tail, by the last warp (n_pad - n < 64: at most 16 blocks of four rows)
+            const int k4 = n / 4 + (int)threadIdx.x - (NT - 32);
+            if ((int)threadIdx.x >= NT - 32 && k4 < A.n_pad / 4) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (c >= ncol) continue;
+                    const float* q = cols + (size_t)c * cs + off[c] + 4 * k4;
+                    store(c, k4, make_float4(4 * k4 < n ? q[0] - sh[c] : 0.f, 4 * k4 + 1 < n ? q[1] - sh[c] : 0.f,
+                                             4 * k4 + 2 < n ? q[2] - sh[c] : 0.f, 0.f));
+                }
+            }
         }
 
         // ---- pass 3: X'X over each row set, by work items.  The pad row holds the column's shift,

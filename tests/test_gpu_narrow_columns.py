@@ -45,7 +45,7 @@ def narrow_dataset(n, r):
     return ds
 
 
-def check_narrow(ds, r, dense):
+def check_narrow(ds, r, dense, kappa=None):
     res, _, _ = oracle_dense(ds, r)
     D = res.dense
     assert not D.singular.any()
@@ -55,7 +55,8 @@ def check_narrow(ds, r, dense):
     # the systems are differences of FP32 column sums: each term is rounded to 2^-24 of x^2, the difference
     # is the spread, so the sums keep 2^-24 (1 + mean^2 / var) of it; four such (two sums, two sides)
     x = ds.XR.astype(np.float64)
-    kappa = (1.0 + x.mean(1) ** 2 / x.var(1)).reshape(-1, r).max(1)[None, :, None]
+    if kappa is None:
+        kappa = (1.0 + x.mean(1) ** 2 / x.var(1)).reshape(-1, r).max(1)[None, :, None]
     t_sys = np.abs(t_ref).max(2, keepdims=True)
     lim = (T_REL + 2.0 ** -22 * kappa) * t_sys + T_ABS
     dt = np.abs(tt - np.abs(t_ref))
@@ -70,6 +71,17 @@ def test_narrow_columns_plain(n, r):
     _, rows, dense = engine_run(ds, r)
     check_narrow(ds, r, dense)
     assert rows.singular == 0
+
+
+@pytest.mark.parametrize("r", [1, 2, 4])
+@pytest.mark.parametrize("n", SIZES)
+def test_centred_sums_do_not_cancel(n, r):
+    """With an intercept the sums are those of the centred columns: the bar of ordinary columns, whatever the
+    mean."""
+    ds = narrow_dataset(n, r)
+    _, _, dense = engine_run(ds, r)
+    check_narrow(ds, r, dense, kappa=0.0)
+    check_narrow(ds, r, noalloc_dense(ds, r), kappa=0.0)
 
 
 @pytest.mark.parametrize("r", [1, 2, 4])
