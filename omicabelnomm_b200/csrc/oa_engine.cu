@@ -678,18 +678,28 @@ int chunk_for(const oa_engine* e) {
     return std::min(e->cfg.max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : wave_chunk(e, e->t));
 }
 
-// The per-SNP covariate sums of the current trait block come from the pre-GEMM, else from row gathers
-// (k_snp_stats, which handles neither the quirk, nor padding columns, nor 8 columns per SNP).  The
+// Blocks with more pre-GEMM columns than traits (and than one 256-column tile) whose per-SNP covariate sums the
+// row gathers could take as well: k_snp_stats handles neither the quirk, nor padding columns, nor 8 columns
+// per SNP.
+bool wide_block(const oa_engine* e) {
+    return !quirk_on(e) && !padded(e) && e->r <= 4 && e->c2 > std::max(e->t, 256);
+}
+
+// The per-SNP covariate sums of the current trait block come from the pre-GEMM, else from row gathers.  The
 // pre-GEMM is the faster one whatever the row sets (statistics stage, gathers / pre-GEMM: 100 patterns of
 // 50 rows at n = 1,000 0.67 / 0.16 ms, 128 of 24 rows at n = 8,000 2.60 / 0.59 ms, of 1,200 rows 13.2 / 1.3
-// ms, 1,000 of 3 rows at n = 6,000 4.4 / 1.0 ms); the gathers stay for blocks whose column matrix and
-// products would take more than PRE_BYTES (thousands of row sets with many covariates).
+// ms, 1,000 of 3 rows at n = 6,000 4.4 / 1.0 ms).  The gathers stay for wide blocks
+//   * of uncentred columns (no intercept), where D - A'A cancels more than the products keep (n = 10,000,
+//     own patterns, dosages: beta's error 2.8e-7 / 4.5e-7 in the plain form, 3.5e-5 / 9.6e-5 in the mixed one;
+//     columns of 8 +- 2: 6.0e-7 / 3.9e-6 and 5.4e-5 / 1.2e-3);
+//   * whose column matrix and products would take more than PRE_BYTES (thousands of row sets with many
+//     covariates).
 constexpr size_t PRE_BYTES = 4ull << 30;
 bool use_pre_for(const oa_engine* e) {
     if (quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1) return true;
     if (e->req.stats_path == 2) return false;
-    return e->c2 <= std::max(e->t, 256) ||
-           (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES;
+    return !wide_block(e) ||
+           (e->center && (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES);
 }
 
 oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_ptr) {
