@@ -296,7 +296,7 @@ struct oa_engine {
     DBuf<float> Qr;
     DBuf<float> Qb;      // [n_pad / 4][l][4] the basis by blocks of four rows (k_snp_lean's projection)
     DBuf<double> qsum;   // [l] column sums of the FP32 basis
-    DBuf<double> Afull_lean;   // [chunk*r][LEAN_QX_L] all-rows projection from k_snp_lean
+    DBuf<double> Afull_lean;   // [chunk*r][ql] all-rows projection from k_snp_lean
     bool have_cov = false;
     bool center = false;   // the first covariate is constant: SNP columns are taken relative to their means
     bool fuse_split = false;  // the tensor-core GEMMs split FP32 columns in shared memory where they can
@@ -305,8 +305,9 @@ struct oa_engine {
     int t = 0;
     DBuf<float> Yraw, Yt;
     // 16-bit hi / lo of the GEMMs' column operand, n_pad values per column: the traits' residuals Y~
-    // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  BF16 in the mixed form; FP16
-    // of scaled columns in the plain form, with cscale = 1 / scale of each column
+    // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  BF16; with `half` FP16
+    // of scaled columns, with cscale = 1 / scale of each column
+    bool half = false;   // the trait block's products are FP16 hi / lo summed in FP32 (half_block)
     DBuf<__nv_bfloat16> Yhi, Ylo;
     DBuf<float> cscale;
     DBuf<double> tsums, rss0, b0, W, zQ;
@@ -337,7 +338,7 @@ struct oa_engine {
     long long tune_gen = 0;
     std::vector<int> h_nobs;
     // the chunk's GEMM stores z = X'Y~ (and the pre-GEMM's columns beside it, from one read of X) and
-    // k_test_stats evaluates it: the plain form, and narrow mixed blocks (combined_columns)
+    // k_test_stats evaluates it: FP16 products, and narrow mixed blocks (combined_columns)
     bool stored_z = false;
     // SNP chunk buffers
     int chunk = 0;
@@ -353,8 +354,9 @@ struct oa_engine {
     int n_inter = 0, inter_keep = 0;
     DBuf<__nv_bfloat16> Xhi, Xlo;
     DBuf<float> mean, varx, aobs, afull, zA, zD;
-    DBuf<float> D, Dset, C2T;   // X'X, per-set X'X; stored products (pre-GEMM columns and / or z)
-    DBuf<float> xscale;         // plain form: 1 / scale of each SNP column's FP16 split
+    DBuf<double> D;             // X'X
+    DBuf<float> Dset, C2T;      // per-set X'X; stored products (pre-GEMM columns and / or z)
+    DBuf<float> xscale;         // FP16 products: 1 / scale of each SNP column's FP16 split
     DBuf<int> has_nan;
     DBuf<double> sinv, sfinv;
     DBuf<float> qdel;           // quirk mode: per (pattern, SNP) terms of the reference's r >= 2 downdate
@@ -685,6 +687,23 @@ bool wide_block(const oa_engine* e) {
     return !quirk_on(e) && !padded(e) && e->r <= 4 && e->c2 > std::max(e->t, 256);
 }
 
+// Covariate slots of the projection A = Q'X that k_snp_lean sums itself (0: A from the pre-GEMM): with two
+// or more columns per SNP and at most eight covariates, and for wide blocks of centred columns.  The
+// pre-GEMM's A (in the mixed form BF16 hi / lo products in a truncating accumulator) is the largest error of the
+// Schur complements and of var_x when D - A'A cancels, which two correlated columns per SNP make likely (an
+// interaction with a covariate), and which the row gathers' FP32 sums, whose place wide blocks' take, kept.
+int lean_ql(const oa_engine* e) {
+    if (e->r > 4) return 0;
+    if (e->ru >= 2) return e->l <= 8 ? 8 : 0;
+    return wide_block(e) && e->center ? (e->l <= 4 ? 4 : (e->l <= 8 ? 8 : 16)) : 0;
+}
+
+// The block's products are FP16 hi / lo splits summed in FP32: the plain form, and the mixed form's wide
+// blocks that leave the row gathers (for their covariate sums' sake; z comes with them).
+bool half_block(const oa_engine* e) {
+    return e->cfg.precision == OA_PLAIN_FP32 || (wide_block(e) && e->center && lean_ql(e) > 0);
+}
+
 // The per-SNP covariate sums of the current trait block come from the pre-GEMM, else from row gathers.  The
 // pre-GEMM is the faster one whatever the row sets (statistics stage, gathers / pre-GEMM: 100 patterns of
 // 50 rows at n = 1,000 0.67 / 0.16 ms, 128 of 24 rows at n = 8,000 2.60 / 0.59 ms, of 1,200 rows 13.2 / 1.3
@@ -692,6 +711,7 @@ bool wide_block(const oa_engine* e) {
 //   * of uncentred columns (no intercept), where D - A'A cancels more than the products keep (n = 10,000,
 //     own patterns, dosages: beta's error 2.8e-7 / 4.5e-7 in the plain form, 3.5e-5 / 9.6e-5 in the mixed one;
 //     columns of 8 +- 2: 6.0e-7 / 3.9e-6 and 5.4e-5 / 1.2e-3);
+//   * of two or four columns per SNP with more than eight covariates (no lean_ql);
 //   * whose column matrix and products would take more than PRE_BYTES (thousands of row sets with many
 //     covariates).
 constexpr size_t PRE_BYTES = 4ull << 30;
@@ -699,7 +719,7 @@ bool use_pre_for(const oa_engine* e) {
     if (quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1) return true;
     if (e->req.stats_path == 2) return false;
     return !wide_block(e) ||
-           (e->center && (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES);
+           (e->center && lean_ql(e) > 0 && (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES);
 }
 
 oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_ptr) {
@@ -860,6 +880,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     e->b2_ready = false;
     e->lp = oa_engine::LeanPlan{};
     OA_CHECK(e->Yt.ensure((size_t)t * e->n_pad));
+    e->half = half_block(e);
     const size_t ycols = (size_t)t + (use_pre_for(e) ? e->c2 : 0);   // B2 follows Y~
     OA_CHECK(e->Yhi.ensure(ycols * e->n_pad));
     OA_CHECK(e->Ylo.ensure(ycols * e->n_pad));
@@ -871,11 +892,10 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->a_r2.ensure(t));
     OA_CHECK(e->inv_ncorr.ensure(t));
     OA_CHECK(e->vf.ensure(t));
-    const bool mixed = e->cfg.precision == OA_MIXED_BF16X3;
     k_trait_resid<<<t, TRAIT_THREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
                                                e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, e->Yt.p, e->Yhi.p,
                                                e->Ylo.p, e->rss0.p, e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p,
-                                               e->inv_ncorr.p, e->vf.p, mixed ? nullptr : e->cscale.p);
+                                               e->inv_ncorr.p, e->vf.p, e->half ? e->cscale.p : nullptr);
     ++e->launches;
     OA_CU(cudaGetLastError());
     OA_CU(cudaStreamSynchronize(e->st));
@@ -907,7 +927,7 @@ oa_status grow_keep(oa_engine* e, DBuf<T>& b, size_t keep, size_t want) {
 // Mixed blocks whose traits and pre-GEMM columns fit one 256-column tile: both products come from one
 // launch that reads the split columns once (reading them is what bounds such a block).
 bool combined_columns(const oa_engine* e) {
-    return e->cfg.precision == OA_MIXED_BF16X3 && e->use_pre && !e->fuse_split && e->t + e->c2 <= 256;
+    return !e->half && e->use_pre && !e->fuse_split && e->t + e->c2 <= 256;
 }
 
 oa_status prepare_tuning(oa_engine* e) {
@@ -921,26 +941,25 @@ oa_status prepare_tuning(oa_engine* e) {
     e->use_pre = use_pre_for(e);
     if (e->use_pre && !e->b2_ready) {
         const size_t ny = (size_t)e->t * e->n_pad, nb2 = (size_t)e->c2 * e->n_pad;
-        const bool half = e->cfg.precision == OA_PLAIN_FP32;
         OA_CHECK(grow_keep(e, e->Yhi, ny, ny + nb2));   // the tuning may have changed since the traits were set
         OA_CHECK(grow_keep(e, e->Ylo, ny, ny + nb2));
         OA_CHECK(grow_keep(e, e->cscale, e->t, (size_t)e->t + e->c2));
-        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, half,
+        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, e->half,
                                                                    e->Yhi.p + ny, e->Ylo.p + ny);
         ++e->launches;
         if (e->nsets > 0) {
-            k_b2_scatter<<<e->nsets, 256, 0, e->st>>>(e->Qr.p, e->LP, e->n_pad, l, e->set_off.p, e->set_rows.p, half,
-                                                      e->Yhi.p + ny, e->Ylo.p + ny);
+            k_b2_scatter<<<e->nsets, 256, 0, e->st>>>(e->Qr.p, e->LP, e->n_pad, l, e->set_off.p, e->set_rows.p,
+                                                      e->half,                                                      e->Yhi.p + ny, e->Ylo.p + ny);
             ++e->launches;
         }
-        if (half) {
+        if (e->half) {
             k_fill<<<(e->c2 + 255) / 256, 256, 0, e->st>>>(e->cscale.p + e->t, e->c2, 1.f / HALF_SCALE_Q);
             ++e->launches;
         }
         OA_CU(cudaGetLastError());
         e->b2_ready = true;
     }
-    e->stored_z = e->cfg.precision == OA_PLAIN_FP32 || combined_columns(e);
+    e->stored_z = e->half || combined_columns(e);
     if (e->use_pre) OA_CHECK(lean_plan(e));
     return OA_OK;
 }
@@ -977,7 +996,7 @@ StatsArgs stats_args(oa_engine* e, const float* X, int mbc, int LP, int spb, int
     A.zA = e->zA.p;
     A.zD = e->zD.p;
     A.write_split = 1;
-    A.xscale = e->cfg.precision == OA_PLAIN_FP32 ? e->xscale.p : nullptr;
+    A.xscale = e->half ? e->xscale.p : nullptr;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
@@ -1021,14 +1040,6 @@ oa_status stats_gather(oa_engine* e, const float* X, int mbc) {
 
 // Lean path: k_snp_lean (imputation, 16-bit split, X'X over all rows and over
 // each row set) -> pre-GEMM C2 = [Q | Q o m_1 | ...]'X -> k_schur.
-// SNPs per CTA group of k_snp_lean: requested (a power of two <= 8 / r), else lean_auto_spb
-// With two or more columns per SNP and at most LEAN_QX_L covariates, k_snp_lean also sums the
-// all-rows covariate projection A = Q'X of every column (short FP32 partial sums, FP64 across
-// warps) for k_schur: the pre-GEMM's A (FP32 sums over all n rows; BF16 hi/lo products in the mixed
-// form) is the largest error of the Schur complements and of var_x when D - A'A cancels, which two
-// correlated columns per SNP make likely (an interaction with a covariate).  Those kernels take
-// groups of at most LEAN_QX_NC columns.
-bool want_lean_qx(const oa_engine* e) { return e->ru >= 2 && e->l <= LEAN_QX_L && e->r <= LEAN_QX_NC; }
 
 // Threads per k_snp_lean CTA (OA_LEAN_THREADS asks for 256 or 512 where long columns run 512).
 int lean_threads(const oa_engine* e) {
@@ -1036,15 +1047,16 @@ int lean_threads(const oa_engine* e) {
     return t == LEAN_MAX_THREADS && e->lean_threads_req ? e->lean_threads_req : t;
 }
 
+// SNPs per CTA group of k_snp_lean: requested (a power of two <= 8 / r), else lean_auto_spb.
 int lean_group(const oa_engine* e) {
     if (lean_threads(e) == LEAN_MAX_THREADS) return 1;   // the 512-thread kernel takes one SNP per group
-    const int cap = want_lean_qx(e) ? LEAN_QX_NC / e->r : 8 / e->r;
+    const int ql = lean_ql(e), cap = ql == 16 ? 1 : (ql ? 4 : 8) / e->r;   // the instantiated forms
     if (e->lean_spb > 0) {
         int s = 1;
         while (s * 2 <= e->lean_spb) s *= 2;
         return std::min(s, cap);
     }
-    return std::min(cap, lean_auto_spb(e->r, e->n_pad, want_lean_qx(e), e->chunk, e->sm_count));
+    return std::min(cap, lean_auto_spb(e->r, e->n_pad, ql, e->chunk, e->sm_count));
 }
 
 // Launch plan of k_snp_lean for the current trait block and tuning: SNPs per
@@ -1054,9 +1066,9 @@ oa_status lean_plan(oa_engine* e) {
     const int R = e->r;
     const size_t limit = 227 * 1024 - 1024;
     int spb = lean_group(e);
-    const bool qx = want_lean_qx(e);
-    while (spb > 1 && lean_smem_bytes(R, e->n_pad, spb, 0, qx) > 200 * 1024) spb /= 2;
-    const size_t base = lean_smem_bytes(R, e->n_pad, spb, 0, qx);
+    const int ql = lean_ql(e);
+    while (spb > 1 && lean_smem_bytes(R, e->n_pad, spb, 0, ql) > 200 * 1024) spb /= 2;
+    const size_t base = lean_smem_bytes(R, e->n_pad, spb, 0, ql);
     const size_t per_item = (size_t)spb * (R * (R + 1) / 2) * 4;
     int max_items = 1;
     for (int s2 = 0; s2 < e->nsets; ++s2)
@@ -1083,7 +1095,7 @@ oa_status lean_plan(oa_engine* e) {
     e->lp.spb = spb;
     e->lp.items_cap = cap;
     e->lp.npass = e->nsets > 0 ? (int)passes.size() - 1 : 0;
-    e->lp.smem = lean_smem_bytes(R, e->n_pad, spb, cap, qx);
+    e->lp.smem = lean_smem_bytes(R, e->n_pad, spb, cap, ql);
     return OA_OK;
 }
 
@@ -1094,7 +1106,7 @@ oa_status lean_plan(oa_engine* e) {
 // floats, and a GEMM shape that has a fused form (OA_FUSED_SPLIT at engine
 // creation: 1 takes the fused forms, 0 keeps the split copy).
 bool fused_chunk(const oa_engine* e, const float* X, size_t ldx, const int* xrows) {
-    return e->fuse_split && e->cfg.precision == OA_MIXED_BF16X3 && e->use_pre && e->c2 <= 128 && !xrows &&
+    return e->fuse_split && !e->half && e->use_pre && e->c2 <= 128 && !xrows &&
            ldx == (size_t)e->n && e->n % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 &&
            oa_gemm_tc_fusable(e->variant, e->t);
 }
@@ -1126,22 +1138,25 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     A.D = e->D.p;
     A.Dset = e->Dset.p;
     A.write_split = fused ? 0 : 1;
-    A.xscale = e->cfg.precision == OA_PLAIN_FP32 ? e->xscale.p : nullptr;
+    A.xscale = e->half ? e->xscale.p : nullptr;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
     A.err = reinterpret_cast<int*>(e->counters.p + 3);
-    const bool qx = want_lean_qx(e) && oa_lean_has_qx(R, spb);
-    if (qx) {
-        OA_CHECK(e->Afull_lean.ensure((size_t)e->chunk * R * LEAN_QX_L));
+    const bool f64 = wide_block(e);
+    const int ql = oa_lean_has_qx(R, spb, lean_ql(e), f64) ? lean_ql(e) : 0;
+    if (ql) {
+        OA_CHECK(e->Afull_lean.ensure((size_t)e->chunk * R * ql));
         A.Qb = reinterpret_cast<const float4*>(e->Qb.p);
         A.l = e->l;
+        A.ql = ql;
+        A.f64 = f64;
         A.qsum = e->qsum.p;
         A.Afull = e->Afull_lean.p;
     }
     const int groups = (mbc + spb - 1) / spb;
     const int threads = lean_threads(e);
-    const int per_sm = std::max(1, oa_lean_ctas_per_sm(R, spb, smem, qx, threads));
+    const int per_sm = std::max(1, oa_lean_ctas_per_sm(R, spb, smem, ql, threads, ql && f64));
     const int grid = std::min(groups, e->sm_count * per_sm);
     OA_CU(oa_launch_snp_lean(R, spb, A, grid, threads, smem, e->st));
     ++e->launches;
@@ -1185,7 +1200,8 @@ oa_status schur(oa_engine* e, const float* C2, int mbc) {
     S.rr = e->ru;
     S.qdel = quirk_on(e) ? e->qdel.p : nullptr;
     S.qK = quirk_on(e) ? e->qK.p : nullptr;
-    S.Afull_lean = want_lean_qx(e) && oa_lean_has_qx(R, e->lp.spb) ? e->Afull_lean.p : nullptr;
+    S.ql = lean_ql(e);
+    S.Afull_lean = oa_lean_has_qx(R, e->lp.spb, S.ql, wide_block(e)) ? e->Afull_lean.p : nullptr;
     OA_CU(oa_launch_schur(R, S, e->st));
     ++e->launches;
     return OA_OK;
@@ -1280,7 +1296,7 @@ constexpr int Z_TRAITS = 8192;   // traits per stored product
 
 // Name of the kernel that forms the stored product.
 const char* stored_name(const oa_engine* e) {
-    if (e->cfg.precision != OA_PLAIN_FP32) return "k_gemm_tc";
+    if (!e->half) return "k_gemm_tc";
     return std::min(e->t, Z_TRAITS) + (e->use_pre && e->t <= Z_TRAITS ? e->c2 : 0) > 128 ? "k_gemm_tcp2"
                                                                                           : "k_gemm_tcp";
 }
@@ -1289,12 +1305,11 @@ template <int R>
 oa_status gemm_dispatch(oa_engine* e, const float* X, int mbc, int snp_base, bool fused) {
     EpiArgs E = epi_args(e, mbc, snp_base);
     if (e->stored_z) {
-        const bool plain = e->cfg.precision == OA_PLAIN_FP32;
         const int ldc = e->chunk * R, c2 = e->use_pre ? e->c2 : 0;
         int* err = reinterpret_cast<int*>(e->counters.p + 3);
         auto product = [&](int col0, int cols) -> oa_status {   // columns [col0, col0 + cols) of [Y~ | B2] to C2T
             const __nv_bfloat16 *bh = e->Yhi.p + (size_t)col0 * e->n_pad, *bl = e->Ylo.p + (size_t)col0 * e->n_pad;
-            OA_CU(plain ? oa_launch_gemm_tcp(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->xscale.p,
+            OA_CU(e->half ? oa_launch_gemm_tcp(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->xscale.p,
                                              e->cscale.p + col0, e->C2T.p, ldc, err, e->st)
                         : oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->C2T.p, ldc, err,
                                            e->st));
@@ -1361,7 +1376,7 @@ oa_status ensure_chunk_buffers(oa_engine* e) {
     }
     OA_CHECK(e->Xhi.ensure(mb * r * e->n_pad));
     OA_CHECK(e->Xlo.ensure(mb * r * e->n_pad));
-    if (e->cfg.precision == OA_PLAIN_FP32) OA_CHECK(e->xscale.ensure(mb * r));
+    if (e->half) OA_CHECK(e->xscale.ensure(mb * r));
     if (e->use_pre) {
         OA_CHECK(e->D.ensure(mb * r * r));
         OA_CHECK(e->Dset.ensure((size_t)std::max(e->nsets, 1) * mb * r * r));

@@ -9,12 +9,12 @@ struct LeanArgs;
 struct SchurArgs;
 cudaError_t oa_launch_snp_stats(int R, int LP, const StatsArgs& A, int grid, size_t smem, cudaStream_t st);
 // spb: SNPs per CTA group, a power of two <= 8 / R; threads: 256 per CTA, or 512 with one SNP per group and
-// R = 1, 2 or 4 (lean_threads_for)
+// R = 1, 2 or 4 (lean_threads_for); A.Afull: with the in-kernel projection (oa_lean_has_qx)
 cudaError_t oa_launch_snp_lean(int R, int spb, const LeanArgs& A, int grid, int threads, size_t smem,
                                cudaStream_t st);
 // resident CTAs of k_snp_lean per SM for this shared-memory size and thread count (0 on error)
-int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads);
-bool oa_lean_has_qx(int R, int spb);
+int oa_lean_ctas_per_sm(int R, int spb, size_t smem, int ql, int threads, bool f64);
+bool oa_lean_has_qx(int R, int spb, int ql, bool f64);
 cudaError_t oa_launch_schur(int R, const SchurArgs& S, cudaStream_t st);
 // pre-GEMM C[col * ldc + row] = sum_k X[row][k] B[col][k], col < c2 (BF16 hi / lo operands)
 cudaError_t oa_launch_pre_tc(const __nv_bfloat16* Xhi, const __nv_bfloat16* Xlo, int xrows,

@@ -36,7 +36,7 @@ struct LeanArgs {
     int items_cap;
     float* mean;          // [mb*r] column means if center, else imputation means (0 if the column had no NaN)
     int* has_nan;
-    float* D;             // [mb][r*r] X'X over all rows
+    double* D;            // [mb][r*r] X'X over all rows
     float* Dset;          // [nsets][mb][r*r] X'X over each row set
     __nv_bfloat16* Xhi;   // [mb*r][n_pad] (tensor-core form) or null
     __nv_bfloat16* Xlo;
@@ -45,15 +45,16 @@ struct LeanArgs {
     int center;           // take each column relative to its mean (valid when XL holds an intercept)
     int* err;
     // all-rows covariate projection A = Q'(x - shift) of every column, summed here (short FP32
-    // partial sums, FP64 across warps) instead of taken from the pre-GEMM, or null: with two or
-    // more columns per SNP the all-rows Schur complement D - A'A (var_x) and the pattern systems
-    // cancel a large part of D, and the pre-GEMM's long FP32 / BF16-split sums of A are then the
-    // largest error of the statistics (the qx kernels, at most LEAN_QX_L covariates)
+    // partial sums, FP64 across warps) instead of taken from the pre-GEMM, or null: where the
+    // all-rows Schur complement D - A'A (var_x) and the pattern systems cancel a large part of D
+    // (two or more columns per SNP; a SNP column near a covariate), the pre-GEMM's sums of A are
+    // the largest error of the statistics (the qx kernels, l <= ql)
     const float4* Qb;     // [n_pad / 4][l] the orthonormal covariate basis (FP32) by blocks of four
                           // rows: Qb[k4 * l + q] = rows 4 k4 .. 4 k4 + 3 of covariate q (0 past n)
-    int l;
+    int l, ql;            // covariates, and the slots for them: 4, 8 or 16
+    int f64;              // the qx kernels' sums are FP64 from the thread's partial sum on
     const double* qsum;   // [l] column sums of the basis (FP64)
-    double* Afull;        // [mb*R][LEAN_QX_L]: A of column c, covariate q at Afull[c * LEAN_QX_L + q]
+    double* Afull;        // [mb*R][ql]: A of column c, covariate q at Afull[c * ql + q]
 };
 
 // Threads per CTA (the template's NT): 256; groups of one SNP may also run 512 (launched where
@@ -63,15 +64,14 @@ constexpr int LEAN_MAX_THREADS = 512;
 constexpr int LEAN_MAX_WARPS = LEAN_MAX_THREADS / 32;
 constexpr int LEAN_BLOCK_ROWS = 256;    // rows of a set per index block (one 16-byte load of eight rows per lane)
 constexpr int LEAN_STAGE_U = 8;         // elements per thread and step of the element-wise staging
-constexpr int LEAN_QX_L = 8;            // covariates of the in-kernel projection (l <= 8)
-constexpr int LEAN_QX_NC = 4;           // columns per group of the qx kernels
+constexpr int LEAN_QX_SUMS = 32;        // slots of the in-kernel projection: columns per group x 4, 8 or 16 covariates
 constexpr int LEAN_COL_PAD = 8;         // floats after a staged column: its offset (0..3) and the pad row
 
 // Shared memory of k_snp_lean: the group's columns (stride n_pad + LEAN_COL_PAD floats) | per-item
 // partial sums | reduction scratch.
-__host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int items_cap, bool qx = false) {
+__host__ __device__ inline size_t lean_smem_bytes(int R, int n_pad, int spb, int items_cap, int ql = 0) {
     const int NC = spb * R, NU = spb * R * (R + 1) / 2;
-    const int NQ = NC + NU + (qx ? NC * LEAN_QX_L : 0);   // NU >= NC: also the NaN path's 2 NC sums
+    const int NQ = NC + NU + NC * ql;   // NU >= NC: also the NaN path's 2 NC sums
     return (size_t)NC * (n_pad + LEAN_COL_PAD) * 4 + (size_t)items_cap * NU * 4 +
            (size_t)(LEAN_MAX_WARPS + 1) * NQ * 8 + 64;
 }
@@ -94,11 +94,11 @@ inline int lean_threads_for(int R, int n_pad) {
 // n = 1,000 0.29 / 0.18 / 0.16 / 0.19 ms, n = 2,000 0.33 / 0.21 / 0.20 / 0.26, n = 3,500 0.39 / 0.27 / 0.29 /
 // 0.34, n = 7,000 0.65 / 0.62 / - / -, n = 10,000 1.37 / 1.46 / - / -);
 // with two, the covariate basis read once per group is worth two CTAs (20,000 SNPs, n = 6,000 1.27 / 1.23).
-inline int lean_auto_spb(int R, int n_pad, bool qx, int snps, int sms) {
+inline int lean_auto_spb(int R, int n_pad, int ql, int snps, int sms) {
     int s = 1;
     for (;;) {
         const size_t bytes = (R > 1 ? 100 : (s == 1 ? 60 : 40)) * 1024;
-        if (s * 2 * R > 4 || lean_smem_bytes(R, n_pad, s * 2, 0, qx) > bytes || snps / (s * 2) < 2 * sms) break;
+        if (s * 2 * R > 4 || lean_smem_bytes(R, n_pad, s * 2, 0, ql) > bytes || snps / (s * 2) < 2 * sms) break;
         s *= 2;
     }
     return s;
@@ -185,13 +185,43 @@ __device__ __forceinline__ void warp_sums(const float (&v)[NV], Store&& store) {
     }
 }
 
-// Block-wide sum of NV floats per thread over NW warps: FP32 within a warp, FP64 across
+// The same in FP64, eight values at a time (18 shuffles where one butterfly per value takes 80).
+template <int NV, class Store>
+__device__ __forceinline__ void warp_sums_f64(const float (&v)[NV], Store&& store) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int base = 0; base < NV; base += 8) {
+        double x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = base + i < NV ? (double)v[base + i < NV ? base + i : 0] : 0.0;
+        int idx = 0;
+#pragma unroll
+        for (int m = 4, o = 16; m > 0; m /= 2, o /= 2) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < m) {
+                    const double keep = up ? x[i + m] : x[i], send = up ? x[i] : x[i + m];
+                    x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            idx += up ? m : 0;
+        }
+        x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+        x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+        if ((lane & 3) == 0 && base + idx < NV) store(base + idx, x[0]);
+    }
+}
+
+// Block-wide sum of NV floats per thread over NW warps: FP32 (F64: FP64) within a warp, FP64 across
 // warps (in warp order; the values are spread over the warps); the first NB sums are copied to out[] on
 // every thread, all NV stay at red + LEAN_MAX_WARPS * NV until red is reused.
-template <int NW, int NV, int NB = NV>
+template <int NW, int NV, int NB = NV, bool F64 = false>
 __device__ __forceinline__ void block_sum_fd(float (&v)[NV], double (&out)[NB], double* red /* [warps + 1][NV] */) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    warp_sums<NV>(v, [&](int q, float sum) { red[w * NV + q] = (double)sum; });
+    if constexpr (F64)
+        warp_sums_f64<NV>(v, [&](int q, double sum) { red[w * NV + q] = sum; });
+    else
+        warp_sums<NV>(v, [&](int q, float sum) { red[w * NV + q] = (double)sum; });
     __syncthreads();
     double* bc = red + LEAN_MAX_WARPS * NV;
     for (int q = w; q < NV; q += NW) {
@@ -222,7 +252,7 @@ __device__ __forceinline__ bool lean_narrow(float raw, float mean, int n) {
 // Q'x with l covariates, Qb); offs: two bits of offset per column.  A constant column becomes exact zeros,
 // whatever its mean was rounded to.  Called by the whole block, out of line: rare, and its code and
 // registers stay out of the usual case's.
-template <int R, int NC, bool QX>
+template <int R, int NC, int QL>
 __device__ __noinline__ void lean_recentre(float* cols, int cs, unsigned offs, int n, int ncol, double* red, double* bc,
                                            float* moved, const float4* Qb, int l) {
     constexpr int NP = R * (R + 1) / 2, NU = NC / R * NP;
@@ -276,13 +306,13 @@ __device__ __noinline__ void lean_recentre(float* cols, int cs, unsigned offs, i
                 if (b == a) block_total(sum, bc + i + a);
                 block_total(prod, bc + NC + i / R * NP + lean_pair<R>(a, b));
             }
-            if (QX && (narrow >> a & 1))
+            if (QL && (narrow >> a & 1))
 #pragma unroll 1
                 for (int q = 0; q < l; ++q) {
                     double dot = 0.0;
                     for (int k = threadIdx.x; k < n; k += blockDim.x)
                         dot += (double)reinterpret_cast<const float*>(Qb + (size_t)(k / 4) * l + q)[k % 4] * (double)xa[k];
-                    block_total(dot, bc + NC + NU + (i + a) * LEAN_QX_L + q);
+                    block_total(dot, bc + NC + NU + (i + a) * QL + q);
                 }
         }
     }
@@ -291,7 +321,9 @@ __device__ __noinline__ void lean_recentre(float* cols, int cs, unsigned offs, i
 // Resident CTAs the register allocation leaves room for: 64 registers a thread for groups of one or two
 // columns or of four SNPs, 48 for two SNPs and 40 for a gathered one (where shared memory holds five and
 // six CTAs of 256 threads), else 128.
-constexpr int lean_min_ctas(int R, int SPB, bool gather, int NT) {
+// The projection's partial sums take their own registers.
+constexpr int lean_min_ctas(int R, int SPB, bool gather, int NT, int QL) {
+    if (R == 1 && QL > 0) return SPB * QL <= 16 && QL < 16 ? 1024 / NT : 512 / NT;
     if (R == 1 && SPB == 2) return 5;
     if (R == 1 && SPB == 1 && gather) return 1536 / NT;
     return R * SPB <= 2 || (R == 1 && SPB == 4) ? 1024 / NT : 512 / NT;
@@ -327,8 +359,9 @@ constexpr int lean_min_ctas(int R, int SPB, bool gather, int NT) {
 // where the row sets are few (n = 12,347: 5.9 TB/s of columns read and split written, 0.90 of a copy's
 // rate); with 20 sets of 500 rows the set pass takes the shared-memory pipe to 0.6 and it runs at
 // 4.8 TB/s (n = 10,000).  Unaligned columns: 0.86 ms where 4-byte copies took 1.27 (n = 12,347).
-template <int R, int SPB, bool GATHER, bool QX = false, int NT = 256>
-__global__ void __launch_bounds__(NT, lean_min_ctas(R, SPB, GATHER, NT))
+// QL: covariate slots of the in-kernel projection (0: none); F64: LeanArgs.f64.
+template <int R, int SPB, bool GATHER, int QL = 0, int NT = 256, bool F64 = false>
+__global__ void __launch_bounds__(NT, lean_min_ctas(R, SPB, GATHER, NT, QL))
 k_snp_lean(LeanArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int NC = SPB * R;                 // columns per group
@@ -491,10 +524,10 @@ k_snp_lean(LeanArgs A) {
         float sh[NC];                          // subtracted from every value (centring), 0 without
         float hs[NC];                          // scale of the FP16 split
         {
-            constexpr int NQX = QX ? NC * LEAN_QX_L : 0;
+            constexpr int NQX = NC * QL;
             constexpr int NV = NC + NU + NQX;  // [column sums | cross products | Q'x of the raw columns]
             constexpr int NB = NC + NU;        // sums every thread keeps (Q'x stays in shared memory)
-            static_assert(!QX || NC <= LEAN_QX_NC, "columns of the qx kernels");
+            static_assert(NQX <= LEAN_QX_SUMS, "slots of the qx kernels");
             double tot[NB];
             const double* qxs = red + LEAN_MAX_WARPS * NV + NB;   // the block's Q'x sums after the last sweep
             bool cnan[NC];
@@ -514,15 +547,15 @@ k_snp_lean(LeanArgs A) {
                             v[c] = c < ncol ? ld4(O, c, k4) : make_float4(0.f, 0.f, 0.f, 0.f);
                             acc[c] += (v[c].x + v[c].y) + (v[c].z + v[c].w);
                         }
-                        if constexpr (QX) {
+                        if constexpr (QL > 0) {
                             // rows 4 k4 .. 4 k4 + 3 of each covariate: one 16-byte load per covariate
 #pragma unroll
-                            for (int qq = 0; qq < LEAN_QX_L; ++qq) {
+                            for (int qq = 0; qq < QL; ++qq) {
                                 if (qq < A.l) {
                                     const float4 q4 = __ldg(A.Qb + (size_t)k4 * A.l + qq);
 #pragma unroll
                                     for (int c = 0; c < NC; ++c) {
-                                        float& a = acc[NC + NU + c * LEAN_QX_L + qq];
+                                        float& a = acc[NC + NU + c * QL + qq];
                                         a = fmaf(q4.x, v[c].x, a);
                                         a = fmaf(q4.y, v[c].y, a);
                                         a = fmaf(q4.z, v[c].z, a);
@@ -546,7 +579,7 @@ k_snp_lean(LeanArgs A) {
                                 }
                     }
                 });
-                block_sum_fd<NWARP, NV, NB>(acc, tot, red);
+                block_sum_fd<NWARP, NV, NB, F64>(acc, tot, red);
                 if (round == 1) break;
                 bool any_nan = false;
 #pragma unroll
@@ -595,7 +628,7 @@ k_snp_lean(LeanArgs A) {
 #pragma unroll
                     for (int c = 0; c < NC; ++c) offs |= (unsigned)off[c] << (2 * c);
                     double* bc = red + LEAN_MAX_WARPS * NV;
-                    lean_recentre<R, NC, QX>(cols, cs, offs, n, ncol, red, bc, moved, A.Qb, A.l);
+                    lean_recentre<R, NC, QL>(cols, cs, offs, n, ncol, red, bc, moved, A.Qb, A.l);
 #pragma unroll
                     for (int u = 0; u < NB; ++u) tot[u] = bc[u];
 #pragma unroll
@@ -620,15 +653,15 @@ k_snp_lean(LeanArgs A) {
                     if (threadIdx.x == 0 && c < ncol) A.xscale[i0 * R + c] = inv;
                 }
             }
-            if constexpr (QX) {
+            if constexpr (QL > 0) {
                 // A = Q'(x - shift) = Q'x - shift * (column sums of Q), in FP64; thread u writes entry u
                 // (compile-time register indices)
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
-                    if ((int)threadIdx.x / LEAN_QX_L == c && c < ncol) {
-                        const int qq = threadIdx.x % LEAN_QX_L;
-                        A.Afull[(size_t)(i0 * R + c) * LEAN_QX_L + qq] =
-                            qq < A.l ? qxs[c * LEAN_QX_L + qq] - (double)sh[c] * A.qsum[qq] : 0.0;
+                    if ((int)threadIdx.x / QL == c && c < ncol) {
+                        const int qq = threadIdx.x % QL;
+                        A.Afull[(size_t)(i0 * R + c) * QL + qq] =
+                            qq < A.l ? qxs[c * QL + qq] - (double)sh[c] * A.qsum[qq] : 0.0;
                     }
             }
             if (threadIdx.x == 0) {
@@ -651,7 +684,7 @@ k_snp_lean(LeanArgs A) {
                         const int ca = s2 * R + a, cb = s2 * R + bb, u = s2 * NP + lean_pair<R>(a, bb);
                         if (lane == 0 && w == u % NWARP && s2 < nsnp) {
                             const double sa = sh[ca], sb = sh[cb];
-                            const float d = (float)(tot[NC + u] - sa * tot[cb] - sb * tot[ca] + (double)n * sa * sb);
+                            const double d = tot[NC + u] - sa * tot[cb] - sb * tot[ca] + (double)n * sa * sb;
                             A.D[(size_t)(i0 + s2) * R * R + a * R + bb] = d;
                             A.D[(size_t)(i0 + s2) * R * R + bb * R + a] = d;
                         }
@@ -817,7 +850,7 @@ struct SchurArgs {
     int l, mb, G, Z, ldc;
     int rr;                  // the caller's columns per SNP; columns [rr, R) are zero padding
     const float* C2;         // pre-GEMM output, column c of SNP column x at C2[c * ldc + x]
-    const float* D;          // [mb][r*r]
+    const double* D;         // [mb][r*r]
     const float* Dset;       // [G+Z][mb][r*r]
     const double* W;         // [G][l][l]
     const uint8_t* pat_bad;  // [G]
@@ -832,9 +865,10 @@ struct SchurArgs {
     // the reference's r >= 2 downdate (quirk mode, raw uncentred columns), or null:
     float* qdel;             // [G][mb][l][r] the quirk's change of Q_obs'X
     double* qK;              // [G][mb][r][r] Gram matrix term of the quirk's RSS
-    // all-rows projection A of each SNP column from k_snp_lean ([mb*r][LEAN_QX_L]), or null: A from
+    // all-rows projection A of each SNP column from k_snp_lean ([mb*r][ql]), or null: A from
     // the pre-GEMM's first l columns
     const double* Afull_lean;
+    int ql;
 };
 
 // The system of (pattern g, SNP i) as the reference's r >= 2 downdate builds
@@ -940,11 +974,11 @@ __device__ __forceinline__ void schur_slots(const SchurArgs& S, int i, int slot0
 #pragma unroll
         for (int a = 0; a < R; ++a)
             a_full[qq * R + a] = qq >= l ? 0.0
-                                 : S.Afull_lean ? S.Afull_lean[((size_t)i * R + a) * LEAN_QX_L + qq]
+                                 : S.Afull_lean ? S.Afull_lean[((size_t)i * R + a) * S.ql + qq]
                                                 : (double)S.C2[(size_t)qq * S.ldc + i * R + a];
     double Dm[R * R];
 #pragma unroll
-    for (int u = 0; u < R * R; ++u) Dm[u] = (double)S.D[(size_t)i * R * R + u];
+    for (int u = 0; u < R * R; ++u) Dm[u] = S.D[(size_t)i * R * R + u];
     // all-rows Schur complement D - A'A (Q orthonormal): var_x of the SNP terms (src/Algorithm.cpp:665-670)
     double Sf[R * R];
 #pragma unroll

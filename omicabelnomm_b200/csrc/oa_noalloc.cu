@@ -491,12 +491,14 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         return OA_OK;
     };
     // Tensor-core form: column statistics, one product with [Y~ | B2] per chunk of SNPs and the tests from
-    // it, as the engine's plain form.  Taken with an intercept as the first covariate (the columns are then
-    // centred; uncentred ones cancel more than the tensor-core sums keep) where its buffers fit the array
+    // it, as the engine's wide blocks.  Taken with an intercept as the first covariate (the columns are then
+    // centred; uncentred ones cancel more than the tensor-core sums keep) where the statistics kernel sums
+    // the all-rows projection itself and the buffers fit the array
     // with chunks of 256 SNPs or the whole block.  At n = 2,000 with 200 traits and 4,000 SNPs the FP32
     // form's row gathers and SIMT product took 1.10 of 1.35 ms.
-    const bool qx = r >= 2 && l <= LEAN_QX_L;
-    if (hinfo[6] && (r == 1 || qx) && n_pad < 65536) {
+    // slots of the covariates that the column statistics project on themselves
+    const int ql = r == 1 ? (l <= 4 ? 4 : (l <= 8 ? 8 : 16)) : (l <= 8 ? 8 : 0);
+    if (hinfo[6] && ql && n_pad < 65536) {
         const int nblk = hinfo[7], c2 = l * (1 + nsets), cols = t + c2;
         int* rows = tc.take<int>((size_t)(nrows > 0 ? nrows : 1));
         uint16_t* item_rows = tc.take<uint16_t>((size_t)(nblk > 0 ? nblk : 1) * LEAN_BLOCK_ROWS);
@@ -506,10 +508,10 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         float* cscale = tc.take<float>(cols);
         const bool need_aobs = Z > 0;
         const size_t per_snp = (size_t)r * n_pad * 4 + (size_t)r * cols * 4 + (size_t)r * 12 +
-                               (size_t)r * r * (4 + 4 * (size_t)nsets + 8 * (size_t)t) + t + (qx ? r * LEAN_QX_L * 8 : 0) +
+                               (size_t)r * r * (8 + 4 * (size_t)nsets + 8 * (size_t)t) + t + (size_t)r * ql * 8 +
                                (need_aobs ? 4 * ((size_t)t * l * r + (size_t)Z * (l * r + r * r)) : 0);
         // alignment of the pieces below, and the basis blocks
-        const size_t slack = 16 * 256 + (qx ? (size_t)n_pad * l * 4 + (size_t)l * 8 : 0);
+        const size_t slack = 16 * 256 + (size_t)n_pad * l * 4 + (size_t)l * 8;
         const long long room = (long long)OA_NOALLOC_SCRATCH_BYTES - (long long)tc.used - (long long)slack;
         long long fit = room > 0 ? room / (long long)per_snp : 0;
         if (fit < mb) fit = fit / 256 * 256;
@@ -518,29 +520,25 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
         const int threads = lean_threads_for(r, n_pad);
         int sms = 148;
         NA_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const int spb = threads == 256 ? lean_auto_spb(r, n_pad, qx, chunk, sms) : 1;
-        const size_t smem = lean_smem_bytes(r, n_pad, spb, nblk > 0 ? nblk : 1, qx);
+        const int spb = threads == 256 && ql <= 8 ? lean_auto_spb(r, n_pad, ql, chunk, sms) : 1;
+        const size_t smem = lean_smem_bytes(r, n_pad, spb, nblk > 0 ? nblk : 1, ql);
         if (chunk > 0 && smem <= 227 * 1024 - 1024) {
             float* mean_c = tc.take<float>((size_t)chunk * r);
             float* varx_c = tc.take<float>((size_t)chunk * r);
             float* xscale = tc.take<float>((size_t)chunk * r);
-            float* D = tc.take<float>((size_t)chunk * r * r);
+            double* D = tc.take<double>((size_t)chunk * r * r);
             float* Dset = tc.take<float>((size_t)nsets * chunk * r * r);
             __nv_bfloat16* xhi = tc.take<__nv_bfloat16>((size_t)chunk * r * n_pad);
             __nv_bfloat16* xlo = tc.take<__nv_bfloat16>((size_t)chunk * r * n_pad);
             float* C = tc.take<float>((size_t)cols * chunk * r);
             double* sinv_c = tc.take<double>((size_t)t * chunk * r * r);
             uint8_t* sing_c = tc.take<uint8_t>((size_t)t * chunk);
-            double* afull = qx ? tc.take<double>((size_t)chunk * r * LEAN_QX_L) : nullptr;
+            double* afull = tc.take<double>((size_t)chunk * r * ql);
             float* aobs_c = need_aobs ? tc.take<float>((size_t)t * chunk * l * r) : nullptr;
             float* zA_c = need_aobs ? tc.take<float>((size_t)Z * chunk * l * r) : nullptr;
             float* zD_c = need_aobs ? tc.take<float>((size_t)Z * chunk * r * r) : nullptr;
-            float* qb = nullptr;
-            double* qsum = nullptr;
-            if (qx) {
-                qb = tc.take<float>((size_t)n_pad * l);
-                qsum = tc.take<double>(l);
-            }
+            float* qb = tc.take<float>((size_t)n_pad * l);
+            double* qsum = tc.take<double>(l);
             if (tc.used <= OA_NOALLOC_SCRATCH_BYTES) {
                 k_set_rows<<<nsets, SET_THREADS, 0, st>>>(y, (size_t)n, n, set_rep, set_kind, set_off, rows);
                 k_set_gram<<<nsets, OA_NTHREADS, 0, st>>>(Q64, n, l, set_kind, set_off, rows, W, zQ, set_slot, pat_bad);
@@ -553,7 +551,7 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
                 k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, st>>>(Qr, LP, n, n_pad, l, c2, 1, bhi + ny, blo + ny);
                 k_b2_scatter<<<nsets, 256, 0, st>>>(Qr, LP, n_pad, l, set_off, rows, 1, bhi + ny, blo + ny);
                 k_fill<<<(c2 + 255) / 256, 256, 0, st>>>(cscale + t, c2, 1.f / HALF_SCALE_Q);
-                if (qx) k_na_qblocks<<<l, 256, 0, st>>>(Qr, LP, n, n_pad, l, qb, qsum);
+                k_na_qblocks<<<l, 256, 0, st>>>(Qr, LP, n, n_pad, l, qb, qsum);
                 NA_CU(cudaGetLastError());
                 int* err = reinterpret_cast<int*>(counters + 3);
                 LeanArgs A{};
@@ -577,12 +575,12 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
                 A.xscale = xscale;
                 A.center = 1;
                 A.err = err;
-                if (qx) {
-                    A.Qb = reinterpret_cast<const float4*>(qb);
-                    A.l = l;
-                    A.qsum = qsum;
-                    A.Afull = afull;
-                }
+                A.Qb = reinterpret_cast<const float4*>(qb);
+                A.l = l;
+                A.ql = ql;
+                A.f64 = 1;
+                A.qsum = qsum;
+                A.Afull = afull;
                 SchurArgs S{};
                 S.l = l;
                 S.G = t;
@@ -601,6 +599,7 @@ extern "C" oa_status oa_scan_dense_noalloc(const float* xl, const float* y, cons
                 S.zD = zD_c;
                 S.rr = r;
                 S.Afull_lean = afull;
+                S.ql = ql;
                 const int per_sm = (int)(227 * 1024 / (smem + 2048));
                 for (int c0 = 0; c0 < mb; c0 += chunk) {
                     const int mc = mb - c0 < chunk ? mb - c0 : chunk;

@@ -54,7 +54,7 @@ cudaError_t oa_launch_snp_stats(int R, int LP, const StatsArgs& A, int grid, siz
     }
 }
 
-template <int R, int SPB, bool QX, int NT = 256>
+template <int R, int SPB, int QL, int NT, bool F64>
 static cudaError_t go_lean(const LeanArgs& A, int grid, size_t smem, cudaStream_t st) {
     static int set_bulk[64], set_gather[64];
     int dev = 0;
@@ -62,26 +62,26 @@ static cudaError_t go_lean(const LeanArgs& A, int grid, size_t smem, cudaStream_
     const int d = dev & 63;
     int* done = A.xrows ? set_gather : set_bulk;
     if (done[d] < (int)smem) {
-        cudaError_t e = A.xrows ? cudaFuncSetAttribute(k_snp_lean<R, SPB, true, QX, NT>,
+        cudaError_t e = A.xrows ? cudaFuncSetAttribute(k_snp_lean<R, SPB, true, QL, NT, F64>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024)
-                                : cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QX, NT>,
+                                : cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QL, NT, F64>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
         if (e != cudaSuccess) return e;
         done[d] = 227 * 1024 - 1024;
     }
     if (A.xrows)
-        k_snp_lean<R, SPB, true, QX, NT><<<grid, NT, smem, st>>>(A);
+        k_snp_lean<R, SPB, true, QL, NT, F64><<<grid, NT, smem, st>>>(A);
     else
-        k_snp_lean<R, SPB, false, QX, NT><<<grid, NT, smem, st>>>(A);
+        k_snp_lean<R, SPB, false, QL, NT, F64><<<grid, NT, smem, st>>>(A);
     return cudaGetLastError();
 }
 
-template <int R, int SPB, bool QX, int NT = 256>
+template <int R, int SPB, int QL, int NT, bool F64>
 static int lean_occ(size_t smem) {
     int nb = 0;
-    if (cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QX, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_snp_lean<R, SPB, false, QL, NT, F64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              227 * 1024 - 1024) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_snp_lean<R, SPB, false, QX, NT>, NT, smem) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_snp_lean<R, SPB, false, QL, NT, F64>, NT, smem) !=
             cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -89,52 +89,89 @@ static int lean_occ(size_t smem) {
     return nb;
 }
 
-// The qx kernels (all-rows covariate projection summed in the kernel) exist for groups of at most
-// LEAN_QX_NC columns with two or more columns per SNP.
-bool oa_lean_has_qx(int R, int spb) { return R >= 2 && R * spb <= LEAN_QX_NC; }
+// The instantiated forms: groups of R columns x SPB SNPs, QL covariate slots of the in-kernel projection
+// (0: none), threads, FP64 sums.  f(R, SPB, QL, NT, F64) as integral constants; false if there is no such form.
+template <class F>
+static bool lean_form(int R, int spb, int ql, int threads, bool f64, F&& f) {
+    const int key = (((R * 16 + spb) * 32 + ql) * 4 + threads / 256) * 2 + (f64 ? 1 : 0);
+    bool found = false;
+    auto form = [&](auto r, auto s, auto q, auto nt, auto p) {
+        constexpr int k = (((decltype(r)::value * 16 + decltype(s)::value) * 32 + decltype(q)::value) * 4 +
+                           decltype(nt)::value / 256) * 2 + (decltype(p)::value ? 1 : 0);
+        if (key == k) {
+            f(r, s, q, nt, p);
+            found = true;
+        }
+    };
+    using std::integral_constant;
+    constexpr std::false_type f32{};
+    constexpr std::true_type dbl{};
+    constexpr integral_constant<int, 0> n0{};
+    constexpr integral_constant<int, 1> n1{};
+    constexpr integral_constant<int, 2> n2{};
+    constexpr integral_constant<int, 4> n4{};
+    constexpr integral_constant<int, 8> n8{};
+    constexpr integral_constant<int, 16> n16{};
+    constexpr integral_constant<int, 256> t256{};
+    constexpr integral_constant<int, LEAN_MAX_THREADS> t512{};
+    form(n1, n1, n0, t256, f32);
+    form(n1, n2, n0, t256, f32);
+    form(n1, n4, n0, t256, f32);
+    form(n1, n8, n0, t256, f32);
+    form(n2, n1, n0, t256, f32);
+    form(n2, n2, n0, t256, f32);
+    form(n2, n4, n0, t256, f32);
+    form(n4, n1, n0, t256, f32);
+    form(n4, n2, n0, t256, f32);
+    form(n8, n1, n0, t256, f32);
+    form(n1, n1, n0, t512, f32);
+    form(n2, n1, n0, t512, f32);
+    form(n4, n1, n0, t512, f32);
+    form(n2, n1, n8, t256, f32);
+    form(n2, n2, n8, t256, f32);
+    form(n4, n1, n8, t256, f32);
+    form(n2, n1, n8, t512, f32);
+    form(n4, n1, n8, t512, f32);
+    // wide blocks
+    form(n1, n1, n4, t256, dbl);
+    form(n1, n2, n4, t256, dbl);
+    form(n1, n4, n4, t256, dbl);
+    form(n1, n1, n4, t512, dbl);
+    form(n1, n1, n8, t256, dbl);
+    form(n1, n2, n8, t256, dbl);
+    form(n1, n4, n8, t256, dbl);
+    form(n1, n1, n8, t512, dbl);
+    form(n1, n1, n16, t256, dbl);
+    form(n1, n1, n16, t512, dbl);
+    form(n2, n1, n8, t256, dbl);
+    form(n2, n2, n8, t256, dbl);
+    form(n4, n1, n8, t256, dbl);
+    form(n2, n1, n8, t512, dbl);
+    form(n4, n1, n8, t512, dbl);
+    return found;
+}
 
-int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads) {
-    // cached per (device, R, spb, qx, smem, threads): no runtime calls while a stream is captured
-    static std::map<std::tuple<int, int, int, bool, size_t, int>, int> cache;
+bool oa_lean_has_qx(int R, int spb, int ql, bool f64) {
+    return ql > 0 && lean_form(R, spb, ql, 256, f64, [](auto...) {});
+}
+
+int oa_lean_ctas_per_sm(int R, int spb, size_t smem, int ql, int threads, bool f64) {
+    // cached per (device, R, spb, ql, smem, threads, f64): no runtime calls while a stream is captured
+    static std::map<std::tuple<int, int, int, int, size_t, int, bool>, int> cache;
     static std::mutex mu;
     int dev = 0;
     cudaGetDevice(&dev);
-    const auto key = std::make_tuple(dev, R, spb, qx, smem, threads);
+    const auto key = std::make_tuple(dev, R, spb, ql, smem, threads, f64);
     {
         std::lock_guard<std::mutex> g(mu);
         auto it = cache.find(key);
         if (it != cache.end()) return it->second;
     }
     int v = 0;
-    if (threads == LEAN_MAX_THREADS) {
-        switch (R * 100 + spb) {
-            case 101: v = qx ? 0 : lean_occ<1, 1, false, LEAN_MAX_THREADS>(smem); break;
-            case 201: v = qx ? lean_occ<2, 1, true, LEAN_MAX_THREADS>(smem) : lean_occ<2, 1, false, LEAN_MAX_THREADS>(smem); break;
-            case 401: v = qx ? lean_occ<4, 1, true, LEAN_MAX_THREADS>(smem) : lean_occ<4, 1, false, LEAN_MAX_THREADS>(smem); break;
-            default: v = 0;
-        }
-    } else if (qx) {
-        switch (R * 100 + spb) {
-            case 201: v = lean_occ<2, 1, true>(smem); break;
-            case 202: v = lean_occ<2, 2, true>(smem); break;
-            case 401: v = lean_occ<4, 1, true>(smem); break;
-            default: v = 0;
-        }
-    } else {
-        switch (R * 100 + spb) {
-            case 101: v = lean_occ<1, 1, false>(smem); break;
-            case 102: v = lean_occ<1, 2, false>(smem); break;
-            case 104: v = lean_occ<1, 4, false>(smem); break;
-            case 108: v = lean_occ<1, 8, false>(smem); break;
-            case 201: v = lean_occ<2, 1, false>(smem); break;
-            case 202: v = lean_occ<2, 2, false>(smem); break;
-            case 204: v = lean_occ<2, 4, false>(smem); break;
-            case 401: v = lean_occ<4, 1, false>(smem); break;
-            case 402: v = lean_occ<4, 2, false>(smem); break;
-            case 801: v = lean_occ<8, 1, false>(smem); break;
-            default: v = 0;
-        }
-    }
+    lean_form(R, spb, ql, threads, f64, [&](auto r, auto s, auto q, auto nt, auto p) {
+        v = lean_occ<decltype(r)::value, decltype(s)::value, decltype(q)::value, decltype(nt)::value,
+                     decltype(p)::value>(smem);
+    });
     std::lock_guard<std::mutex> g(mu);
     cache[key] = v;
     return v;
@@ -142,38 +179,12 @@ int oa_lean_ctas_per_sm(int R, int spb, size_t smem, bool qx, int threads) {
 
 cudaError_t oa_launch_snp_lean(int R, int spb, const LeanArgs& A, int grid, int threads, size_t smem,
                                cudaStream_t st) {
-    if (threads == LEAN_MAX_THREADS) {
-        switch (R * 100 + spb) {
-            case 101: return A.Afull ? cudaErrorInvalidValue : go_lean<1, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
-            case 201: return A.Afull ? go_lean<2, 1, true, LEAN_MAX_THREADS>(A, grid, smem, st)
-                                     : go_lean<2, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
-            case 401: return A.Afull ? go_lean<4, 1, true, LEAN_MAX_THREADS>(A, grid, smem, st)
-                                     : go_lean<4, 1, false, LEAN_MAX_THREADS>(A, grid, smem, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    if (threads != 256) return cudaErrorInvalidValue;
-    if (A.Afull) {
-        switch (R * 100 + spb) {
-            case 201: return go_lean<2, 1, true>(A, grid, smem, st);
-            case 202: return go_lean<2, 2, true>(A, grid, smem, st);
-            case 401: return go_lean<4, 1, true>(A, grid, smem, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (R * 100 + spb) {
-        case 101: return go_lean<1, 1, false>(A, grid, smem, st);
-        case 102: return go_lean<1, 2, false>(A, grid, smem, st);
-        case 104: return go_lean<1, 4, false>(A, grid, smem, st);
-        case 108: return go_lean<1, 8, false>(A, grid, smem, st);
-        case 201: return go_lean<2, 1, false>(A, grid, smem, st);
-        case 202: return go_lean<2, 2, false>(A, grid, smem, st);
-        case 204: return go_lean<2, 4, false>(A, grid, smem, st);
-        case 401: return go_lean<4, 1, false>(A, grid, smem, st);
-        case 402: return go_lean<4, 2, false>(A, grid, smem, st);
-        case 801: return go_lean<8, 1, false>(A, grid, smem, st);
-        default: return cudaErrorInvalidValue;
-    }
+    cudaError_t e = cudaErrorInvalidValue;
+    lean_form(R, spb, A.Afull ? A.ql : 0, threads, A.Afull && A.f64, [&](auto r, auto s, auto q, auto nt, auto p) {
+        e = go_lean<decltype(r)::value, decltype(s)::value, decltype(q)::value, decltype(nt)::value,
+                    decltype(p)::value>(A, grid, smem, st);
+    });
+    return e;
 }
 
 cudaError_t oa_set_wait_limit_stats(unsigned long long ns) {
