@@ -303,7 +303,7 @@ struct oa_engine {
     bool fused_last = false;  // the last enqueued chunk took the fused form
     // traits
     int t = 0;
-    DBuf<float> Yraw, Yt;
+    DBuf<float> Yraw;
     // 16-bit hi / lo of the GEMMs' column operand, n_pad values per column: the traits' residuals Y~
     // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  BF16; with `half` FP16
     // of scaled columns, with cscale = 1 / scale of each column
@@ -434,7 +434,7 @@ int live_engines(int device, int delta) {
 template <class F>
 void for_each_buf(oa_engine* e, F&& f) {
     f(e->Q64); f(e->Rinv); f(e->Qr); f(e->Qb); f(e->qsum); f(e->Afull_lean);
-    f(e->Yraw); f(e->Yt); f(e->Yhi); f(e->Ylo); f(e->cscale);
+    f(e->Yraw); f(e->Yhi); f(e->Ylo); f(e->cscale);
     f(e->tsums); f(e->rss0); f(e->b0); f(e->W); f(e->zQ);
     f(e->tcounts); f(e->pat); f(e->zset); f(e->nobs); f(e->set_off); f(e->set_rows); f(e->set_rep);
     f(e->set_kind); f(e->set_slot); f(e->tperm); f(e->tinv);
@@ -879,7 +879,6 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     e->c2 = l * (1 + e->nsets);
     e->b2_ready = false;
     e->lp = oa_engine::LeanPlan{};
-    OA_CHECK(e->Yt.ensure((size_t)t * e->n_pad));
     e->half = half_block(e);
     const size_t ycols = (size_t)t + (use_pre_for(e) ? e->c2 : 0);   // B2 follows Y~
     OA_CHECK(e->Yhi.ensure(ycols * e->n_pad));
@@ -893,7 +892,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     OA_CHECK(e->inv_ncorr.ensure(t));
     OA_CHECK(e->vf.ensure(t));
     k_trait_resid<<<t, TRAIT_THREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
-                                               e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, e->Yt.p, e->Yhi.p,
+                                               e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, nullptr, e->Yhi.p,
                                                e->Ylo.p, e->rss0.p, e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p,
                                                e->inv_ncorr.p, e->vf.p, e->half ? e->cscale.p : nullptr);
     ++e->launches;
@@ -2433,7 +2432,6 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         OA_CHECK(e->tcounts.ensure(t * 2));
         OA_CHECK(e->thash.ensure(t * 4));
         for (auto* b : {&e->pat, &e->zset, &e->tperm, &e->tinv}) OA_CHECK(b->ensure(t));
-        OA_CHECK(e->Yt.ensure(t * e->n_pad));
         OA_CHECK(e->Yhi.ensure(t * e->n_pad));
         OA_CHECK(e->Ylo.ensure(t * e->n_pad));
         OA_CHECK(e->rss0.ensure(t));

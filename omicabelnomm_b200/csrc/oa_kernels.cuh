@@ -270,12 +270,12 @@ k_set_gram(const double* __restrict__ Q64, int n, int l, const int* __restrict__
 
 // y~ = y - Q b0 on observed rows (0 on missing rows), b0 = W Q'y.
 // Block jj builds internal trait jj = original trait tperm[jj] (traits are
-// kept sorted by missingness pattern inside the engine).  Writes Y~ (FP32,
-// and BF16 hi/lo for the tensor-core form), RSS0, SST and the constants the
+// kept sorted by missingness pattern inside the engine).  Writes Y~ (FP32 to
+// Yt, if not null; BF16 hi/lo to Yhi, Ylo, if not null), RSS0, SST and the constants the
 // epilogue folds: a_r2 = (n-1)/((n_corr-1) SST), 1/n_corr, (n-miss)/n.
 // With yscale (the FP32-accurate tensor-core form) the split is FP16 of the
-// scaled residuals, written once RSS0 is known, and yscale[jj] = 1 / scale;
-// Yt may be null there (the residuals are then formed twice).
+// scaled residuals and yscale[jj] = 1 / scale: the scale follows from RSS0, so
+// the pass that sums it leaves the residuals' FP32 bits in the two halves.
 static __global__ void __launch_bounds__(TRAIT_THREADS)
 k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, int p,
               const double* __restrict__ Q64, const double* __restrict__ sums,
@@ -315,7 +315,11 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
         rss += d * d;
         const float e = (float)d;
         if (out) out[k] = e;
-        if (Yhi && !yscale) {
+        if (yscale) {
+            const unsigned bits = __float_as_uint(e);
+            reinterpret_cast<unsigned short*>(Yhi)[(size_t)jj * n_pad + k] = (unsigned short)(bits >> 16);
+            reinterpret_cast<unsigned short*>(Ylo)[(size_t)jj * n_pad + k] = (unsigned short)bits;
+        } else if (Yhi) {
             const __nv_bfloat16 hi = __float2bfloat16_rn(e);
             Yhi[(size_t)jj * n_pad + k] = hi;
             Ylo[(size_t)jj * n_pad + k] = __float2bfloat16_rn(e - __bfloat162float(hi));
@@ -348,8 +352,10 @@ k_trait_resid(const float* __restrict__ Y, size_t ldy, int n, int n_pad, int l, 
         const float sc = half_s;
         __half* yh = reinterpret_cast<__half*>(Yhi) + (size_t)jj * n_pad;
         __half* yl = reinterpret_cast<__half*>(Ylo) + (size_t)jj * n_pad;
-        for (int k = threadIdx.x; k < n_pad; k += blockDim.x)
-            split_half((out ? out[k] : (float)resid(k)) * sc, yh[k], yl[k]);   // out: own writes
+        for (int k = threadIdx.x; k < n_pad; k += blockDim.x) {   // own writes
+            const unsigned bits = (unsigned)__half_as_ushort(yh[k]) << 16 | __half_as_ushort(yl[k]);
+            split_half(__uint_as_float(bits) * sc, yh[k], yl[k]);
+        }
     }
 }
 
