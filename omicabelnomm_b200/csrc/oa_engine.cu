@@ -342,6 +342,8 @@ struct oa_engine {
     bool stored_z = false;
     // SNP chunk buffers
     int chunk = 0;
+    int chunk_limit = 0;     // SNPs per chunk the device memory took for this trait block (0: no limit met)
+    bool pre_off = false;    // the pre-GEMM's columns of this wide block did not fit: row gathers
     DBuf<float> Xstage[2];
     // column model (dosage models): each SNP arrives as in_cols file columns and its r columns are
     // formed on the device; in_cols = 0: the input already holds r columns per SNP
@@ -677,7 +679,9 @@ int wave_chunk(const oa_engine* e, int t) {
 
 // SNPs per device chunk of the current trait block.
 int chunk_for(const oa_engine* e) {
-    return std::min(e->cfg.max_snps, e->req.chunk_snps > 0 ? e->req.chunk_snps : wave_chunk(e, e->t));
+    if (e->req.chunk_snps > 0) return std::min(e->cfg.max_snps, e->req.chunk_snps);
+    const int chunk = std::min(e->cfg.max_snps, wave_chunk(e, e->t));
+    return e->chunk_limit > 0 ? std::min(chunk, e->chunk_limit) : chunk;
 }
 
 // Blocks with more pre-GEMM columns than traits (and than one 256-column tile) whose per-SNP covariate sums the
@@ -713,13 +717,49 @@ bool half_block(const oa_engine* e) {
 //     columns of 8 +- 2: 6.0e-7 / 3.9e-6 and 5.4e-5 / 1.2e-3);
 //   * of two or four columns per SNP with more than eight covariates (no lean_ql);
 //   * whose column matrix and products would take more than PRE_BYTES (thousands of row sets with many
-//     covariates).
+//     covariates), or do not fit the device memory (pre_off).
 constexpr size_t PRE_BYTES = 4ull << 30;
 bool use_pre_for(const oa_engine* e) {
     if (quirk_on(e) || padded(e) || e->r > 4 || e->req.stats_path == 1) return true;
-    if (e->req.stats_path == 2) return false;
+    if (e->req.stats_path == 2 || e->pre_off) return false;
     return !wide_block(e) ||
            (e->center && lean_ql(e) > 0 && (size_t)e->c2 * 4 * ((size_t)e->n_pad + (size_t)chunk_for(e) * e->r) <= PRE_BYTES);
+}
+
+void drop_graph(oa_engine* e);
+
+// Gives back the buffers of a chunk (the next block allocates them again) and the graph that holds their addresses.
+void release_chunk(oa_engine* e) {
+    drop_graph(e);
+    e->warm_key = oa_engine::GraphKey{};
+    auto give = [](auto&... b) { (b.release(), ...); };
+    give(e->mean, e->varx, e->sinv, e->sing, e->zA, e->zD, e->aobs, e->qdel, e->qK, e->afull, e->sfinv, e->Xhi, e->Xlo,
+         e->xscale, e->D, e->Dset, e->C2T, e->Afull_lean, e->Xmodel, e->Xstage[0], e->Xstage[1]);
+}
+
+// After a failed allocation for a block: half the SNPs per chunk, where the chunk is chosen here, then the row
+// gathers in place of a wide block's pre-GEMM.  False when nothing is left to give up.  (The plain form's 16-bit
+// split of the chunk and the stored products are 4 n_pad bytes per SNP column and up to 4 (8,192 + c2): 3.8 GB
+// and more at n = 50,000, which a caller near its memory's end need not have.)
+constexpr int CHUNK_LEAST = 256;
+bool less_memory(oa_engine* e) {
+    if (e->req.chunk_snps == 0 && e->chunk > CHUNK_LEAST)
+        e->chunk_limit = std::max(CHUNK_LEAST, e->chunk / 2);
+    else if (e->use_pre && !e->pre_off && e->req.stats_path == 0 && wide_block(e))
+        e->pre_off = true;
+    else
+        return false;
+    release_chunk(e);
+    return true;
+}
+
+// f(), and once more without the chunk's buffers if it found no device memory.
+template <class F>
+oa_status with_room(oa_engine* e, F&& f) {
+    const oa_status s = f();
+    if (s != OA_ERR_NOMEM) return s;
+    release_chunk(e);
+    return f();
 }
 
 oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_ptr) {
@@ -880,10 +920,20 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     e->b2_ready = false;
     e->lp = oa_engine::LeanPlan{};
     e->half = half_block(e);
-    const size_t ycols = (size_t)t + (use_pre_for(e) ? e->c2 : 0);   // B2 follows Y~
-    OA_CHECK(e->Yhi.ensure(ycols * e->n_pad));
-    OA_CHECK(e->Ylo.ensure(ycols * e->n_pad));
-    OA_CHECK(e->cscale.ensure(ycols));
+    e->chunk_limit = 0;
+    e->pre_off = false;
+    auto columns = [&]() -> oa_status {
+        const size_t cols = (size_t)t + (use_pre_for(e) ? e->c2 : 0);   // B2 follows Y~
+        OA_CHECK(e->Yhi.ensure(cols * e->n_pad));
+        OA_CHECK(e->Ylo.ensure(cols * e->n_pad));
+        return e->cscale.ensure(cols);
+    };
+    oa_status fits = with_room(e, columns);
+    if (fits == OA_ERR_NOMEM && use_pre_for(e) && wide_block(e) && e->req.stats_path == 0) {
+        e->pre_off = true;
+        fits = columns();
+    }
+    OA_CHECK(fits);
     OA_CHECK(e->rss0.ensure(t));
     OA_CHECK(e->sst.ensure(t));
     OA_CHECK(e->nobs.ensure(t));
@@ -1145,7 +1195,6 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     const bool f64 = wide_block(e);
     const int ql = oa_lean_has_qx(R, spb, lean_ql(e), f64) ? lean_ql(e) : 0;
     if (ql) {
-        OA_CHECK(e->Afull_lean.ensure((size_t)e->chunk * R * ql));
         A.Qb = reinterpret_cast<const float4*>(e->Qb.p);
         A.l = e->l;
         A.ql = ql;
@@ -1377,6 +1426,7 @@ oa_status ensure_chunk_buffers(oa_engine* e) {
     OA_CHECK(e->Xlo.ensure(mb * r * e->n_pad));
     if (e->half) OA_CHECK(e->xscale.ensure(mb * r));
     if (e->use_pre) {
+        if (lean_ql(e)) OA_CHECK(e->Afull_lean.ensure(mb * r * lean_ql(e)));
         OA_CHECK(e->D.ensure(mb * r * r));
         OA_CHECK(e->Dset.ensure((size_t)std::max(e->nsets, 1) * mb * r * r));
     }
@@ -1567,7 +1617,7 @@ oa_status run_block(oa_engine* e, const float* xr, int mb, bool host_input) {
             drop_graph(e);
             continue;
         }
-        e->timed_chunks = nch;   // their events are read when a time is asked for (block_times)
+        e->timed_chunks = nch;   // their events are read when a time is asked for (chunk_ms, oa_last_block_ms)
         e->block_timed = true;
         e->last_name = e->stored_z                                      ? stored_name(e)
                        : e->fused_last                                  ? (e->t > 128 ? "k_gemm_tc2f" : "k_gemm_tcf")
@@ -1645,10 +1695,11 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
                 e->ru);
         return OA_ERR_STATE;
     }
-    OA_CHECK(prepare_tuning(e));
-    OA_CHECK(ensure_chunk_buffers(e));
+    if (e->subset && host_input) {
+        set_err("a row subset applies to device SNP blocks only (oa_run_snps_device)");
+        return OA_ERR_STATE;
+    }
     const long long tests = (long long)mb * e->t;
-    OA_CHECK(ensure_cap(e, slots_needed(e, mb, e->t, e->chunk)));
     if (e->dense_on || e->cfg.disp_cov) {
         const size_t nd = (size_t)e->t * mb;
         OA_CHECK(e->d_beta.ensure(nd * e->r));
@@ -1662,25 +1713,28 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
     e->timed_chunks = 0;
     e->block_timed = false;
     e->last_mb = mb;
-    if (e->subset) {
-        if (host_input) {
-            set_err("a row subset applies to device SNP blocks only (oa_run_snps_device)");
-            return OA_ERR_STATE;
-        }
-        if (!lean_gathers(e)) OA_CHECK(e->Xstage[0].ensure((size_t)e->chunk * e->r * e->n));
-    }
-    if (column_pass(e)) OA_CHECK(e->Xmodel.ensure((size_t)e->chunk * e->r * model_ld(e)));
-    if (host_input) {
-        if (!e->cp) OA_CU(cudaStreamCreateWithFlags(&e->cp, cudaStreamNonBlocking));
-        for (int b = 0; b < 2; ++b) {
-            OA_CHECK(e->Xstage[b].ensure((size_t)e->chunk * input_cols(e) * e->n));
-            OA_CU(cudaEventRecord(e->ev_used[b], e->st));   // the copy stream starts after the allocation
-        }
-    }
-    if (e->cfg.disp_cov) OA_CHECK(e->marks.ensure((mb + e->chunk - 1) / e->chunk));
-    {
+    if (host_input && !e->cp) OA_CU(cudaStreamCreateWithFlags(&e->cp, cudaStreamNonBlocking));
+    auto chunk_memory = [&]() -> oa_status {
+        OA_CHECK(prepare_tuning(e));
+        OA_CHECK(ensure_chunk_buffers(e));
+        OA_CHECK(ensure_cap(e, slots_needed(e, mb, e->t, e->chunk)));
+        if (e->subset && !lean_gathers(e)) OA_CHECK(e->Xstage[0].ensure((size_t)e->chunk * e->r * e->n));
+        if (column_pass(e)) OA_CHECK(e->Xmodel.ensure((size_t)e->chunk * e->r * model_ld(e)));
+        if (host_input)
+            for (int b = 0; b < 2; ++b) {
+                OA_CHECK(e->Xstage[b].ensure((size_t)e->chunk * input_cols(e) * e->n));
+                OA_CU(cudaEventRecord(e->ev_used[b], e->st));   // the copy stream starts after the allocation
+            }
+        if (e->cfg.disp_cov) OA_CHECK(e->marks.ensure((mb + e->chunk - 1) / e->chunk));
+        return OA_OK;
+    };
+    for (;;) {
         OA_TRACE("SNP block on the device");
-        OA_CHECK(run_block<R>(e, xr, mb, host_input));
+        oa_status s = chunk_memory();
+        if (s == OA_OK) s = run_block<R>(e, xr, mb, host_input);
+        if (s == OA_ERR_NOMEM && less_memory(e)) continue;
+        OA_CHECK(s);
+        break;
     }
     OA_TRACE("stored rows: sort, copy back, convert");
     unsigned long long cnt[5];   // read back by run_block
@@ -1706,8 +1760,8 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
         OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, final_slots(e, (size_t)N), e->retired_pinned));
         const FinalRows hf = final_rows(e->h_rec, N, p);
         if (N > 0) {
-            OA_CHECK(sort_rows<R>(e, NS, mb));
-            OA_CHECK(e->rec2.ensure(final_slots(e, (size_t)N)));
+            OA_CHECK(with_room(e, [&] { return sort_rows<R>(e, NS, mb); }));
+            OA_CHECK(with_room(e, [&] { return e->rec2.ensure(final_slots(e, (size_t)N)); }));
             k_rec_final<R><<<(unsigned)((N * p + 255) / 256), 256, 0, e->st>>>(
                 reinterpret_cast<const RecOf<R>*>(e->rec.p), e->perm2.p, N, l, e->ru, e->nobs.p,
                 e->cfg.disp_cov ? e->cov.p : nullptr, e->cfg.min_t_store, e->cfg.store_all != 0,
@@ -1731,9 +1785,9 @@ oa_status run_snps_impl(oa_engine* e, const float* xr, int32_t mb, bool host_inp
     OA_CHECK(ensure_pinned(e->h_rec, e->h_rec_cap, (size_t)N * rec_slots(R), e->retired_pinned));
     if (e->cfg.disp_cov) OA_CHECK(ensure_pinned(e->h_cov, e->h_cov_cap, (size_t)N * l * 3, e->retired_pinned));
     {
-        OA_CHECK(sort_rows<R>(e, NS, mb));
-        OA_CHECK(e->rec2.ensure((size_t)N * rec_slots(R)));
-        if (e->cfg.disp_cov) OA_CHECK(e->cov2.ensure((size_t)N * l * 3));
+        OA_CHECK(with_room(e, [&] { return sort_rows<R>(e, NS, mb); }));
+        OA_CHECK(with_room(e, [&] { return e->rec2.ensure((size_t)N * rec_slots(R)); }));
+        if (e->cfg.disp_cov) OA_CHECK(with_room(e, [&] { return e->cov2.ensure((size_t)N * l * 3); }));
         const RowsSoA dsoa = rows_soa(e->rec2.p, N, R);   // the record buffer holds the packed fields
         k_rec_gather<R><<<(unsigned)((N + 255) / 256), 256, 0, e->st>>>(reinterpret_cast<const RecOf<R>*>(e->rec.p),
                                                                         e->perm2.p, N, dsoa,
