@@ -189,8 +189,10 @@ int64_t oa_device_bytes(const oa_engine* e);
 /* Allocates now what a trait block of up to `traits` traits and an SNP
  * block of up to `snps` SNPs need at the engine's store thresholds
  * (trait-sized device buffers, the stored-row buffers and their sort space
- * on the device, the pinned host buffer the rows come back in), so that
- * later calls within those sizes seldom allocate.  Pinned host allocations
+ * on the device, the pinned host buffer the rows come back in).  Later
+ * calls within those sizes allocate what depends on the traits' row sets
+ * (stream-ordered, from the device's pool): the first trait block and the
+ * first SNP block after it.  Pinned host allocations
  * are slow while other engines keep the GPU busy: a server reserves its
  * engines' buffers when it creates them.  No counterpart in the reference
  * (one scan per process). */

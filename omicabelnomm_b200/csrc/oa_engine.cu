@@ -2486,12 +2486,11 @@ oa_status oa_reserve(oa_engine* e, int32_t traits, int32_t snps) {
         OA_CHECK(e->tcounts.ensure(t * 2));
         OA_CHECK(e->thash.ensure(t * 4));
         for (auto* b : {&e->pat, &e->zset, &e->tperm, &e->tinv}) OA_CHECK(b->ensure(t));
-        // the traits and the pre-GEMM columns of blocks that are not wide (every trait its own pattern and
-        // zero set at most)
-        const size_t cols = t + std::min(std::max<size_t>(t, 256), l * (1 + 2 * t));
-        OA_CHECK(e->Yhi.ensure(cols * e->n_pad));
-        OA_CHECK(e->Ylo.ensure(cols * e->n_pad));
-        OA_CHECK(e->cscale.ensure(cols));
+        // The first trait block grows these by its pre-GEMM columns.  Reserving room for the columns (of eight
+        // row sets, or of max(t, 256)), or leaving the buffers to the trait block, made four serving requests
+        // slower (5.8 -> 6.3 ms): what the growth gives back is the memory the block's small tables land in.
+        OA_CHECK(e->Yhi.ensure(t * e->n_pad));
+        OA_CHECK(e->Ylo.ensure(t * e->n_pad));
         OA_CHECK(e->rss0.ensure(t));
         for (auto* b : {&e->sst, &e->a_r2, &e->inv_ncorr, &e->vf}) OA_CHECK(b->ensure(t));
         OA_CHECK(e->nobs.ensure(t));

@@ -1,5 +1,5 @@
-"""Device memory of an engine: what a trait block holds, what oa_reserve
-leaves to be allocated, and blocks near the end of the memory."""
+"""Device memory of an engine: what a trait block holds, and blocks near the
+end of the memory."""
 import numpy as np
 import pytest
 
@@ -29,23 +29,6 @@ def test_trait_block_holds_its_columns_once(prec):
     eng.set_traits_device(y.data_ptr(), 64)
     held = eng.device_bytes() - before
     assert columns <= held < columns + 16 * column, (held / column, columns / column)
-    eng.close()
-
-
-@pytest.mark.parametrize("prec", [E.PLAIN, E.MIXED])
-def test_reserved_engine_takes_a_trait_block_without_growing(prec):
-    import torch
-    ds, column, columns = _block()
-    l, n = ds.XL.shape
-    y = torch.from_numpy(ds.Y).cuda()
-    torch.cuda.synchronize()
-    eng = E.Engine(n, l, 1, 64, 1000, precision=prec, min_t_store=5.0, min_r2_store=1e-6)
-    eng.set_covariates(ds.XL)
-    eng.reserve(64, 1000)
-    before = eng.device_bytes()
-    eng.set_traits_device(y.data_ptr(), 64)
-    grown = eng.device_bytes() - before
-    assert grown < 10 * column, grown / column      # the tables of the row sets, no column buffer
     eng.close()
 
 
