@@ -54,8 +54,7 @@ typedef enum oa_status {
 
 typedef enum oa_precision {
     OA_PLAIN_FP32 = 0,   /* FP32 data, tcgen05 products of FP16 hi/lo splits summed in FP32, FP64 small systems */
-    OA_MIXED_BF16X3 = 1  /* XR'Y on tcgen05 tensor cores, BF16 hi/lo 3-product, FP32 accumulate (centred blocks of
-                            many missingness patterns: the plain form's products) */
+    OA_MIXED_BF16X3 = 1  /* XR'Y on tcgen05 tensor cores, BF16 hi/lo 3-product, FP32 accumulate */
 } oa_precision;
 
 /* ---------------------------------------------------------------------------

@@ -305,9 +305,8 @@ struct oa_engine {
     int t = 0;
     DBuf<float> Yraw;
     // 16-bit hi / lo of the GEMMs' column operand, n_pad values per column: the traits' residuals Y~
-    // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  BF16; with `half` FP16
-    // of scaled columns, with cscale = 1 / scale of each column
-    bool half = false;   // the trait block's products are FP16 hi / lo summed in FP32 (half_block)
+    // [0, t), then (pre-GEMM statistics) the column matrix B2 [t, t + c2).  FP16 of scaled columns in the
+    // plain form, with cscale = 1 / scale of each column; else BF16, but for the B2 of wide blocks (half_pre)
     DBuf<__nv_bfloat16> Yhi, Ylo;
     DBuf<float> cscale;
     DBuf<double> tsums, rss0, b0, W, zQ;
@@ -338,7 +337,7 @@ struct oa_engine {
     long long tune_gen = 0;
     std::vector<int> h_nobs;
     // the chunk's GEMM stores z = X'Y~ (and the pre-GEMM's columns beside it, from one read of X) and
-    // k_test_stats evaluates it: FP16 products, and narrow mixed blocks (combined_columns)
+    // k_test_stats evaluates it: the plain form, and narrow mixed blocks (combined_columns)
     bool stored_z = false;
     // SNP chunk buffers
     int chunk = 0;
@@ -355,10 +354,11 @@ struct oa_engine {
     DBuf<float> inter;
     int n_inter = 0, inter_keep = 0;
     DBuf<__nv_bfloat16> Xhi, Xlo;
+    DBuf<__nv_bfloat16> Phi, Plo;   // mixed wide blocks: the FP16 split beside it, for the pre-GEMM (half_pre)
     DBuf<float> mean, varx, aobs, afull, zA, zD;
     DBuf<double> D;             // X'X
     DBuf<float> Dset, C2T;      // per-set X'X; stored products (pre-GEMM columns and / or z)
-    DBuf<float> xscale;         // FP16 products: 1 / scale of each SNP column's FP16 split
+    DBuf<float> xscale;         // FP16 splits: 1 / scale of each SNP column's FP16 split
     DBuf<int> has_nan;
     DBuf<double> sinv, sfinv;
     DBuf<float> qdel;           // quirk mode: per (pattern, SNP) terms of the reference's r >= 2 downdate
@@ -441,7 +441,7 @@ void for_each_buf(oa_engine* e, F&& f) {
     f(e->tcounts); f(e->pat); f(e->zset); f(e->nobs); f(e->set_off); f(e->set_rows); f(e->set_rep);
     f(e->set_kind); f(e->set_slot); f(e->tperm); f(e->tinv);
     f(e->a_r2); f(e->inv_ncorr); f(e->vf); f(e->thash); f(e->tcheck); f(e->sst); f(e->qrows); f(e->pat_bad);
-    f(e->Xstage[0]); f(e->Xstage[1]); f(e->Xmodel); f(e->inter); f(e->Xhi); f(e->Xlo);
+    f(e->Xstage[0]); f(e->Xstage[1]); f(e->Xmodel); f(e->inter); f(e->Xhi); f(e->Xlo); f(e->Phi); f(e->Plo);
     f(e->mean); f(e->varx); f(e->aobs); f(e->afull); f(e->zA); f(e->zD); f(e->D); f(e->Dset); f(e->C2T);
     f(e->xscale);
     f(e->has_nan); f(e->sinv); f(e->sfinv); f(e->sing); f(e->qdel); f(e->qK);
@@ -702,11 +702,11 @@ int lean_ql(const oa_engine* e) {
     return wide_block(e) && e->center ? (e->l <= 4 ? 4 : (e->l <= 8 ? 8 : 16)) : 0;
 }
 
-// The block's products are FP16 hi / lo splits summed in FP32: the plain form, and the mixed form's wide
-// blocks that leave the row gathers (for their covariate sums' sake; z comes with them).
-bool half_block(const oa_engine* e) {
-    return e->cfg.precision == OA_PLAIN_FP32 || (wide_block(e) && e->center && lean_ql(e) > 0);
-}
+bool is_plain(const oa_engine* e) { return e->cfg.precision == OA_PLAIN_FP32; }
+
+// The pre-GEMM's products are FP16 hi / lo splits summed in FP32: the plain form, and the wide blocks that leave
+// the row gathers in the mixed form (whose main product stays BF16: two splits of the columns).
+bool half_pre(const oa_engine* e) { return is_plain(e) || (wide_block(e) && e->center && lean_ql(e) > 0); }
 
 // The per-SNP covariate sums of the current trait block come from the pre-GEMM, else from row gathers.  The
 // pre-GEMM is the faster one whatever the row sets (statistics stage, gathers / pre-GEMM: 100 patterns of
@@ -733,7 +733,7 @@ void release_chunk(oa_engine* e) {
     drop_graph(e);
     e->warm_key = oa_engine::GraphKey{};
     auto give = [](auto&... b) { (b.release(), ...); };
-    give(e->mean, e->varx, e->sinv, e->sing, e->zA, e->zD, e->aobs, e->qdel, e->qK, e->afull, e->sfinv, e->Xhi, e->Xlo,
+    give(e->mean, e->varx, e->sinv, e->sing, e->zA, e->zD, e->aobs, e->qdel, e->qK, e->afull, e->sfinv, e->Xhi, e->Xlo, e->Phi, e->Plo,
          e->xscale, e->D, e->Dset, e->C2T, e->Afull_lean, e->Xmodel, e->Xstage[0], e->Xstage[1]);
 }
 
@@ -919,7 +919,6 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     e->c2 = l * (1 + e->nsets);
     e->b2_ready = false;
     e->lp = oa_engine::LeanPlan{};
-    e->half = half_block(e);
     e->chunk_limit = 0;
     e->pre_off = false;
     auto columns = [&]() -> oa_status {
@@ -944,7 +943,7 @@ oa_status set_traits_impl(oa_engine* e, const float* y, int32_t t, bool device_p
     k_trait_resid<<<t, TRAIT_THREADS, 0, e->st>>>(Y, (size_t)n, n, e->n_pad, l, e->p, e->Q64.p, e->tsums.p,
                                                e->tcounts.p, e->pat.p, e->W.p, e->tperm.p, nullptr, e->Yhi.p,
                                                e->Ylo.p, e->rss0.p, e->sst.p, e->nobs.p, e->b0.p, e->a_r2.p,
-                                               e->inv_ncorr.p, e->vf.p, e->half ? e->cscale.p : nullptr);
+                                               e->inv_ncorr.p, e->vf.p, is_plain(e) ? e->cscale.p : nullptr);
     ++e->launches;
     OA_CU(cudaGetLastError());
     OA_CU(cudaStreamSynchronize(e->st));
@@ -976,7 +975,7 @@ oa_status grow_keep(oa_engine* e, DBuf<T>& b, size_t keep, size_t want) {
 // Mixed blocks whose traits and pre-GEMM columns fit one 256-column tile: both products come from one
 // launch that reads the split columns once (reading them is what bounds such a block).
 bool combined_columns(const oa_engine* e) {
-    return !e->half && e->use_pre && !e->fuse_split && e->t + e->c2 <= 256;
+    return !is_plain(e) && e->use_pre && !e->fuse_split && e->t + e->c2 <= 256;
 }
 
 oa_status prepare_tuning(oa_engine* e) {
@@ -993,22 +992,22 @@ oa_status prepare_tuning(oa_engine* e) {
         OA_CHECK(grow_keep(e, e->Yhi, ny, ny + nb2));   // the tuning may have changed since the traits were set
         OA_CHECK(grow_keep(e, e->Ylo, ny, ny + nb2));
         OA_CHECK(grow_keep(e, e->cscale, e->t, (size_t)e->t + e->c2));
-        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, e->half,
+        k_b2_init<<<(unsigned)((nb2 + 255) / 256), 256, 0, e->st>>>(e->Qr.p, e->LP, n, e->n_pad, l, e->c2, half_pre(e),
                                                                    e->Yhi.p + ny, e->Ylo.p + ny);
         ++e->launches;
         if (e->nsets > 0) {
             k_b2_scatter<<<e->nsets, 256, 0, e->st>>>(e->Qr.p, e->LP, e->n_pad, l, e->set_off.p, e->set_rows.p,
-                                                      e->half,                                                      e->Yhi.p + ny, e->Ylo.p + ny);
+                                                      half_pre(e), e->Yhi.p + ny, e->Ylo.p + ny);
             ++e->launches;
         }
-        if (e->half) {
+        if (half_pre(e)) {
             k_fill<<<(e->c2 + 255) / 256, 256, 0, e->st>>>(e->cscale.p + e->t, e->c2, 1.f / HALF_SCALE_Q);
             ++e->launches;
         }
         OA_CU(cudaGetLastError());
         e->b2_ready = true;
     }
-    e->stored_z = e->half || combined_columns(e);
+    e->stored_z = is_plain(e) || combined_columns(e);
     if (e->use_pre) OA_CHECK(lean_plan(e));
     return OA_OK;
 }
@@ -1045,7 +1044,7 @@ StatsArgs stats_args(oa_engine* e, const float* X, int mbc, int LP, int spb, int
     A.zA = e->zA.p;
     A.zD = e->zD.p;
     A.write_split = 1;
-    A.xscale = e->half ? e->xscale.p : nullptr;
+    A.xscale = is_plain(e) ? e->xscale.p : nullptr;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
@@ -1155,7 +1154,7 @@ oa_status lean_plan(oa_engine* e) {
 // floats, and a GEMM shape that has a fused form (OA_FUSED_SPLIT at engine
 // creation: 1 takes the fused forms, 0 keeps the split copy).
 bool fused_chunk(const oa_engine* e, const float* X, size_t ldx, const int* xrows) {
-    return e->fuse_split && !e->half && e->use_pre && e->c2 <= 128 && !xrows &&
+    return e->fuse_split && !is_plain(e) && e->use_pre && e->c2 <= 128 && !xrows &&
            ldx == (size_t)e->n && e->n % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 &&
            oa_gemm_tc_fusable(e->variant, e->t);
 }
@@ -1187,13 +1186,24 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     A.D = e->D.p;
     A.Dset = e->Dset.p;
     A.write_split = fused ? 0 : 1;
-    A.xscale = e->half ? e->xscale.p : nullptr;
+    A.xscale = half_pre(e) ? e->xscale.p : nullptr;
     A.center = e->center ? 1 : 0;
     A.Xhi = e->Xhi.p;
     A.Xlo = e->Xlo.p;
     A.err = reinterpret_cast<int*>(e->counters.p + 3);
     const bool f64 = wide_block(e);
     const int ql = oa_lean_has_qx(R, spb, lean_ql(e), f64) ? lean_ql(e) : 0;
+    const bool two_splits = half_pre(e) && !is_plain(e);
+    if (two_splits) {
+        if (!ql || !f64) {   // lean_group picks groups that have the kernel
+            set_err("no column-statistics kernel writes both splits for r = %d, %d SNPs per group", R, spb);
+            return OA_ERR_UNSUPPORTED;
+        }
+        A.Xhi = e->Phi.p;
+        A.Xlo = e->Plo.p;
+        A.Bhi = e->Xhi.p;
+        A.Blo = e->Xlo.p;
+    }
     if (ql) {
         A.Qb = reinterpret_cast<const float4*>(e->Qb.p);
         A.l = e->l;
@@ -1215,6 +1225,9 @@ oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, 
     if (fused)
         OA_CU(oa_launch_pre_tcf(X, ldx, e->n, mbc * R, e->mean.p, e->has_nan.p, e->center ? 1 : 0, e->Yhi.p + ny,
                                 e->Ylo.p + ny, e->c2, e->n_pad, e->C2T.p, ldc, err, e->st));
+    else if (two_splits)
+        OA_CU(oa_launch_gemm_tcp(e->Phi.p, e->Plo.p, mbc * R, e->Yhi.p + ny, e->Ylo.p + ny, e->c2, e->n_pad,
+                                 e->xscale.p, e->cscale.p + e->t, e->C2T.p, ldc, err, e->st));
     else
         OA_CU(oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, e->Yhi.p + ny, e->Ylo.p + ny, e->c2, e->n_pad, e->C2T.p,
                                ldc, err, e->st));
@@ -1344,7 +1357,7 @@ constexpr int Z_TRAITS = 8192;   // traits per stored product
 
 // Name of the kernel that forms the stored product.
 const char* stored_name(const oa_engine* e) {
-    if (!e->half) return "k_gemm_tc";
+    if (!is_plain(e)) return "k_gemm_tc";
     return std::min(e->t, Z_TRAITS) + (e->use_pre && e->t <= Z_TRAITS ? e->c2 : 0) > 128 ? "k_gemm_tcp2"
                                                                                           : "k_gemm_tcp";
 }
@@ -1357,7 +1370,7 @@ oa_status gemm_dispatch(oa_engine* e, const float* X, int mbc, int snp_base, boo
         int* err = reinterpret_cast<int*>(e->counters.p + 3);
         auto product = [&](int col0, int cols) -> oa_status {   // columns [col0, col0 + cols) of [Y~ | B2] to C2T
             const __nv_bfloat16 *bh = e->Yhi.p + (size_t)col0 * e->n_pad, *bl = e->Ylo.p + (size_t)col0 * e->n_pad;
-            OA_CU(e->half ? oa_launch_gemm_tcp(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->xscale.p,
+            OA_CU(is_plain(e) ? oa_launch_gemm_tcp(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->xscale.p,
                                              e->cscale.p + col0, e->C2T.p, ldc, err, e->st)
                         : oa_launch_pre_tc(e->Xhi.p, e->Xlo.p, mbc * R, bh, bl, cols, e->n_pad, e->C2T.p, ldc, err,
                                            e->st));
@@ -1424,7 +1437,11 @@ oa_status ensure_chunk_buffers(oa_engine* e) {
     }
     OA_CHECK(e->Xhi.ensure(mb * r * e->n_pad));
     OA_CHECK(e->Xlo.ensure(mb * r * e->n_pad));
-    if (e->half) OA_CHECK(e->xscale.ensure(mb * r));
+    if (half_pre(e)) OA_CHECK(e->xscale.ensure(mb * r));
+    if (half_pre(e) && !is_plain(e) && e->use_pre) {
+        OA_CHECK(e->Phi.ensure(mb * r * e->n_pad));
+        OA_CHECK(e->Plo.ensure(mb * r * e->n_pad));
+    }
     if (e->use_pre) {
         if (lean_ql(e)) OA_CHECK(e->Afull_lean.ensure(mb * r * lean_ql(e)));
         OA_CHECK(e->D.ensure(mb * r * r));

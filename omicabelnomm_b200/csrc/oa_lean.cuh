@@ -42,6 +42,8 @@ struct LeanArgs {
     __nv_bfloat16* Xlo;
     int write_split;
     float* xscale;        // FP16 split of the columns times a power of two, 1 / scale here ([mb*r]); null: BF16 split
+    __nv_bfloat16* Bhi;   // with xscale and the f64 kernels: a BF16 split as well (the mixed form's main product), or null
+    __nv_bfloat16* Blo;
     int center;           // take each column relative to its mean (valid when XL holds an intercept)
     int* err;
     // all-rows covariate projection A = Q'(x - shift) of every column, summed here (short FP32
@@ -704,6 +706,12 @@ k_snp_lean(LeanArgs A) {
                     split4(p, h, o);
                 reinterpret_cast<uint2*>(A.Xhi + (size_t)(i0 * R + c) * A.n_pad)[k4] = h;
                 reinterpret_cast<uint2*>(A.Xlo + (size_t)(i0 * R + c) * A.n_pad)[k4] = o;
+                if constexpr (F64)
+                    if (A.Bhi) {
+                        split4(p, h, o);
+                        reinterpret_cast<uint2*>(A.Bhi + (size_t)(i0 * R + c) * A.n_pad)[k4] = h;
+                        reinterpret_cast<uint2*>(A.Blo + (size_t)(i0 * R + c) * A.n_pad)[k4] = o;
+                    }
             };
             by_offset([&](auto O) {
 #pragma unroll 2
