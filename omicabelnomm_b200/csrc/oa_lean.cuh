@@ -226,9 +226,13 @@ __device__ __forceinline__ void block_sum_fd(float (&v)[NV], double (&out)[NB], 
         warp_sums<NV>(v, [&](int q, float sum) { red[w * NV + q] = (double)sum; });
     __syncthreads();
     double* bc = red + LEAN_MAX_WARPS * NV;
-    for (int q = w; q < NV; q += NW) {
-        const double s = warp_sum(lane < NW ? red[lane * NV + q] : 0.0);
-        if (lane == 0) bc[q] = s;
+    constexpr int PER = 32 / NW;   // values a warp adds up at once, NW lanes each
+    for (int q0 = w * PER; q0 < NV; q0 += NW * PER) {
+        const int q = q0 + lane / NW;
+        double s = q < NV ? red[lane % NW * NV + q] : 0.0;
+#pragma unroll
+        for (int o = NW / 2; o > 0; o /= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane % NW == 0 && q < NV) bc[q] = s;
     }
     __syncthreads();
 #pragma unroll
