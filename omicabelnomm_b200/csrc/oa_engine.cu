@@ -1086,9 +1086,6 @@ oa_status stats_gather(oa_engine* e, const float* X, int mbc) {
     return pick(std::integral_constant<int, 16>{});
 }
 
-// Lean path: k_snp_lean (imputation, 16-bit split, X'X over all rows and over
-// each row set) -> pre-GEMM C2 = [Q | Q o m_1 | ...]'X -> k_schur.
-
 // Threads per k_snp_lean CTA (OA_LEAN_THREADS asks for 256 or 512 where long columns run 512).
 int lean_threads(const oa_engine* e) {
     const int t = lean_threads_for(e->r, e->n_pad);
@@ -1162,6 +1159,8 @@ bool fused_chunk(const oa_engine* e, const float* X, size_t ldx, const int* xrow
 template <int R>
 oa_status schur(oa_engine* e, const float* C2, int mbc);
 
+// Lean path: k_snp_lean (imputation, 16-bit split, X'X over all rows and over
+// each row set) -> pre-GEMM C2 = [Q | Q o m_1 | ...]'X -> k_schur.
 template <int R>
 oa_status stats_pre(oa_engine* e, const float* X, size_t ldx, const int* xrows, int mbc, bool fused) {
     const int spb = e->lp.spb;
